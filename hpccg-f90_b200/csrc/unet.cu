@@ -255,10 +255,10 @@ static int weight_grad(hpccg_unet *u, int layer, int level, const __nv_bfloat16 
   a.x_f32 = xf;
   a.dy = dy;
   a.partial = u->partial;
-  const int blocks = (int)std::min<int64_t>(u->partial_blocks, (u->L[level].nvox + 63) / 64);
-  k_dW<<<blocks, 256, 0, u->stream>>>(a);
+  int blocks = 0;
+  UNET_TRY(launch_dW(a, u->partial_blocks, u->d_err, u->num_sms, u->stream, &blocks));
   const int n = (27 * d.cin + 1) * 16;
-  k_reduce_partials<<<(n + 255) / 256, 256, 0, u->stream>>>(u->partial, blocks, n, u->grads + u->off[layer], 1);
+  k_reduce_partials<<<(n + 31) / 32, 256, 0, u->stream>>>(u->partial, blocks, n, u->grads + u->off[layer], 1);
   HPCCG_CUDA(cudaGetLastError());
   return HPCCG_OK;
 }
@@ -277,7 +277,7 @@ static int backward(hpccg_unet *u, const float *in) {
   const int pb = (int)std::min<int64_t>(u->partial_blocks, (L[0].nvox + 255) / 256);
   k_proj_bwd<<<pb, 256, 0, s>>>(u->c1, u->params + u->off[kNumLayers], u->dout, u->pre[0], u->partial, L[0].nvox,
                                 L[0].nx);
-  k_reduce_partials<<<1, 32, 0, s>>>(u->partial, pb, 17, u->grads + u->off[kNumLayers], 1);
+  k_reduce_partials<<<1, 256, 0, s>>>(u->partial, pb, 17, u->grads + u->off[kNumLayers], 1);
   UNET_TRY(weight_grad(u, 12, 0, u->e1b, u->u1, nullptr, u->pre[0]));
   UNET_TRY(conv(u, 12, 0, u->pre[0], nullptr, nullptr, kEpiRawF32, u->gs[0], 0));  // d e1b (skip)
   UNET_TRY(conv(u, 12, 0, u->pre[0], nullptr, nullptr, kEpiRawF32, u->gt[0], 1));  // d u1

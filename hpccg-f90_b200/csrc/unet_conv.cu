@@ -28,66 +28,6 @@ __device__ __forceinline__ TileOrigin tile_origin(const ConvGeom &g, int t) {
   return o;
 }
 
-// One lane's share of a fetch: the span of `len` units of half h of grid row
-// (b, z, y) starting at voxel xs goes to dst.  Units outside the grid are
-// zeroed here (generic stores); the in-grid part is described for a later
-// bulk copy.
-struct Span {
-  const __nv_bfloat16 *src;
-  uint8_t *dst;
-  uint32_t bytes;
-  bool zeroed;  // this lane wrote zero fill with ordinary stores
-};
-
-__device__ __forceinline__ Span plan_span(const ConvGeom &g, const __nv_bfloat16 *base, int b, int z, int y, int h,
-                                          int xs, int len, uint8_t *dst) {
-  Span sp{nullptr, nullptr, 0, false};
-  const uint4 zero = make_uint4(0, 0, 0, 0);
-  if (z < 0 || z >= g.nz || y < 0 || y >= g.ny) {
-    for (int u = 0; u < len; ++u) reinterpret_cast<uint4 *>(dst)[u] = zero;
-    sp.zeroed = true;
-    return sp;
-  }
-  const int lo = max(xs, 0), hi = min(xs + len, g.nx);
-  for (int u = 0; u < lo - xs; ++u) reinterpret_cast<uint4 *>(dst)[u] = zero;
-  for (int u = hi - xs; u < len; ++u) reinterpret_cast<uint4 *>(dst)[u] = zero;
-  sp.zeroed = lo > xs || hi < xs + len;
-  if (hi <= lo) return sp;
-  const int64_t row = ((int64_t)b * g.nz + z) * g.ny + y;
-  sp.src = base + act_unit(row, h, lo, g.nx) * 8;
-  sp.dst = dst + (lo - xs) * 16;
-  sp.bytes = (uint32_t)(hi - lo) * 16;
-  return sp;
-}
-
-// Posts the stage: lanes that zero-filled fence their stores into the async
-// proxy, lane 0 arms the barrier with the warp's total bulk bytes, then every
-// lane issues its copies.
-__device__ __forceinline__ void post_spans(const Span *sp, int nsp, uint64_t *bar, int lane) {
-  uint32_t bytes = 0;
-  bool zeroed = false;
-  for (int i = 0; i < nsp; ++i) {
-    bytes += sp[i].bytes;
-    zeroed |= sp[i].zeroed;
-  }
-  if (zeroed) fence_proxy_async_smem();  // only lanes that stored zeros
-  const uint32_t total = __reduce_add_sync(0xffffffffu, bytes);
-  __syncwarp();
-  if (lane == 0) mbar_expect_tx(bar, total);
-  __syncwarp();
-  for (int i = 0; i < nsp; ++i)
-    if (sp[i].bytes) bulk_g2s(sp[i].dst, sp[i].src, sp[i].bytes, bar);
-}
-
-// Lane 0 waits, the result is shared with the warp.
-__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, int *err, int where, int lane) {
-  bool ok = true;
-  if (lane == 0) ok = mbar_wait(bar, parity, err, where);
-  ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-  __syncwarp();
-  return ok;
-}
-
 // Epilogue of one voxel: row m of tile t holds its 16 accumulated channels in v.
 template <int EPI>
 __device__ __forceinline__ void conv_store(const ConvArgs &a, int t, int m, const float *v, const float *bias,

@@ -1,0 +1,373 @@
+// unet_dw.cu -- weight and bias gradients of the U-Net's convolutions.
+//
+// dW[tap][ci][co] = sum_v X[v + off(tap)][ci] dY[v][co], dbias[co] = sum_v dY[v][co].
+// Layers with BF16 inputs run as a GEMM on tcgen05 (k_dW_tc); the 1-channel
+// input layer keeps its FP32 input and runs on the CUDA cores (k_dW_in1).
+// Both leave one partial per CTA, [block][27*cin + 1][16], which
+// k_reduce_partials sums in block order, so gradients are reproducible.
+#include <algorithm>
+
+#include "unet_ops.cuh"
+
+namespace hpccg {
+
+using namespace tc;
+
+// ---- BF16 inputs: tcgen05 ------------------------------------------------------------
+// The contraction runs over voxels.  Both operands are "MN-major": the
+// row-planar layout holds, for 8 channels, 8 consecutive voxels as 128
+// contiguous bytes, which is a no-swizzle core matrix of 8 channels x 8 voxels.
+// For one x row j of X (three z planes, all input groups) the A operand's M
+// index is (dz, input group, half, channel) -- planes of one slab at a uniform
+// stride -- and B's N index is (dY row j-1, j, j+1; co): one MMA of M = 128,
+// N = 48, K = 16 voxels forms the nine (dz, dy) taps of all channels, and the
+// three dx taps are the same A shifted by one voxel (16 bytes) into three
+// accumulators of 48 TMEM columns.  So 16 voxels cost 3 MMAs (an N = 48 MMA
+// takes the ~46 cycles of an N = 16 one) where a tap-by-tap GEMM needs 27.
+// A plane of ones behind each slab's planes gives the bias gradient in the same
+// MMAs.  BF16 products are exact in FP32, but the tensor core's accumulation
+// truncates: left in TMEM over a CTA's ~450 steps the sums were 5e-6 off at
+// 64^3, batch 4, ten times what the FP32 FMA chain of the CUDA cores is
+// (4.4e-7).  So the accumulators are drained after at most kDwChain steps and
+// added up in registers with rounded FP32 additions (1.6e-7); two accumulator
+// sets let the drain run under the next steps' MMAs.
+//
+// A unit is (batch, z, 8 rows of y, up to 128 voxels of x): its ten dY rows
+// (double-buffered) and a ring of X slabs arrive by bulk copies of row spans.
+// Rows outside the grid, the x halo and the padding of dY to whole 16-voxel
+// steps are zeros.  A's rows past the ones plane read whatever follows in
+// shared memory; they only reach accumulator rows that nobody stores.
+//
+// Against the CUDA-core kernel it replaces (one thread per (tap, ci), each
+// re-reading its input voxel from global memory): the 13 layers of a 64^3,
+// batch 4 training step 25.7 -> 0.62 ms (a 16-channel layer at 64^3, batch 4:
+// 6.24 -> 0.12 ms), of which the MMAs are about a third and start-up, drain and
+// the first copies of each unit the rest.
+constexpr int kDwThreads = 192;  // producer warp, MMA warp, four draining warps
+constexpr int kDwRows = 8;   // y rows per unit
+constexpr int kDwSlots = 4;  // X slabs in flight
+constexpr int kDwMaxX = 128;
+constexpr int kDwChain = 8;  // MMA steps between two drains
+
+struct DwTcArgs {
+  ConvGeom g;  // volume and batch only
+  const __nv_bfloat16 *x0, *x1, *dy;
+  float *partial;
+  int *err;
+  int kx;                    // voxels per unit row, a multiple of 16
+  int nxb, nyb, nunits;      // x and y blocks, units
+};
+
+__host__ __device__ constexpr int dw_plane_bytes(int kx) { return (kx + 2) * 16; }
+__host__ __device__ constexpr int dw_planes(int nin) { return 6 * nin + 1; }
+__host__ __device__ constexpr int dw_dy_bytes(int kx) { return (kDwRows + 2) * 2 * kx * 16; }
+// dY buffers, slabs, and the planes that the last slab's M = 128 rows read beyond it
+__host__ __device__ constexpr int dw_smem_bytes(int nin, int kx) {
+  return 2 * dw_dy_bytes(kx) + (kDwSlots * dw_planes(nin) + 16 - dw_planes(nin)) * dw_plane_bytes(kx);
+}
+
+// Instruction descriptor: as idesc_bf16, with A and B MN-major (bits 15, 16).
+__host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) {
+  return idesc_bf16(M, N) | (1u << 15) | (1u << 16);
+}
+
+template <int NIN>
+__global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(DwTcArgs a) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ uint64_t fullx[kDwSlots], emptyx[kDwSlots], fully[2], emptyy[2], acc_full[2], acc_empty[2], drain;
+  __shared__ uint32_t slot;
+  constexpr int P = dw_planes(NIN);
+  const ConvGeom &g = a.g;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int ps = dw_plane_bytes(a.kx), slab = P * ps, dyb = dw_dy_bytes(a.kx);
+  uint8_t *sY = smem, *sX = smem + 2 * dyb;
+  for (int s = 0; s < kDwSlots; ++s) {  // the ones planes: written once, no copy touches them
+    uint32_t *o = reinterpret_cast<uint32_t *>(sX + s * slab + (P - 1) * ps);
+    for (int i = threadIdx.x; i < ps / 4; i += kDwThreads) o[i] = 0x3f803f80u;
+  }
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kDwSlots; ++s) {
+      mbar_init(&fullx[s], 1);
+      mbar_init(&emptyx[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&fully[s], 1);
+      mbar_init(&emptyy[s], 1);
+      mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_empty[s], 4);
+    }
+    mbar_init(&drain, 1);
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&slot, 512);
+    tmem_relinquish();
+  }
+  fence_proxy_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = slot;
+  const int ksteps = a.kx / 16, chunk = max(1, kDwChain / ksteps);  // rows between two drains
+  auto unit = [&](int u, int &b, int &z, int &ya, int &yb, int &x0) {
+    x0 = (u % a.nxb) * kDwMaxX;
+    u /= a.nxb;
+    ya = (u % a.nyb) * kDwRows;
+    yb = min(g.ny, ya + kDwRows);
+    u /= a.nyb;
+    z = u % g.nz;
+    b = u / g.nz;
+  };
+  if (warp == 0) {
+    uint32_t sc = 0, uc = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x, ++uc) {
+      int b, z, ya, yb, x0;
+      unit(u, b, z, ya, yb, x0);
+      const int yp = uc & 1;
+      if (uc >= 2 && !(ok = warp_wait(&emptyy[yp], ((uc >> 1) - 1) & 1, a.err, 41, lane))) break;
+      Span sp[1];
+      int nsp = 0;
+      if (lane < 2 * (kDwRows + 2)) {
+        sp[0] = plan_span(g, a.dy, b, z, ya - 1 + (lane >> 1), lane & 1, x0, a.kx, sY + yp * dyb + lane * a.kx * 16);
+        nsp = 1;
+      }
+      post_spans(sp, nsp, &fully[yp], lane);
+      for (int y = ya; y < yb; ++y, ++sc) {
+        const int s = sc % kDwSlots;
+        const uint32_t n = sc / kDwSlots;
+        if (n > 0 && !(ok = warp_wait(&emptyx[s], (n - 1) & 1, a.err, 42, lane))) break;
+        nsp = 0;
+        if (lane < 6 * NIN) {  // plane (dz, input group, half) = lane
+          const int h = lane & 1, in = (lane >> 1) % NIN, dz = (lane >> 1) / NIN;
+          sp[0] = plan_span(g, in ? a.x1 : a.x0, b, z + dz - 1, y, h, x0 - 1, a.kx + 2, sX + s * slab + lane * ps);
+          nsp = 1;
+        }
+        post_spans(sp, nsp, &fullx[s], lane);
+      }
+    }
+    if (lane == 0) {  // every issued copy has landed before the CTA may exit
+      for (uint32_t j = sc > (uint32_t)kDwSlots ? sc - kDwSlots : 0; j < sc; ++j)
+        mbar_wait(&fullx[j % kDwSlots], (j / kDwSlots) & 1, a.err, 43);
+      for (uint32_t j = uc > 2u ? uc - 2 : 0; j < uc; ++j) mbar_wait(&fully[j & 1], (j >> 1) & 1, a.err, 44);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = idesc_bf16_mn(128, 48);
+      uint32_t sc = 0, uc = 0, cc = 0;  // rows, units, chunks of rows
+      int in_chunk = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x, ++uc) {
+        int b, z, ya, yb, x0;
+        unit(u, b, z, ya, yb, x0);
+        if (!(ok = mbar_wait(&fully[uc & 1], (uc >> 1) & 1, a.err, 45))) break;
+        for (int y = ya; y < yb; ++y, ++sc) {
+          const int s = sc % kDwSlots;
+          if (in_chunk == 0 && cc >= 2 && !(ok = mbar_wait(&acc_empty[cc & 1], ((cc >> 1) - 1) & 1, a.err, 48))) break;
+          if (!(ok = mbar_wait(&fullx[s], (sc / kDwSlots) & 1, a.err, 46))) break;
+          tc_fence_after();
+          const uint32_t d = tmem + 256 * (cc & 1);
+          // MN-major: lbo = distance of 8-voxel groups (K), sbo = of 8-channel groups
+          uint64_t ad = smem_desc(sX + s * slab, 128, ps);
+          uint64_t bd = smem_desc(sY + (uc & 1) * dyb + (y - ya) * 2 * a.kx * 16, 128, a.kx * 16);
+          for (int k = 0; k < ksteps; ++k, ad += 16, bd += 16)
+#pragma unroll
+            for (int dx = 0; dx < 3; ++dx)
+              mma_bf16(d + 48 * dx, ad + dx, bd, idesc, in_chunk > 0 || k > 0 ? 1u : 0u);
+          mma_commit(&emptyx[s]);
+          if (++in_chunk == chunk) {
+            mma_commit(&acc_full[cc & 1]);
+            in_chunk = 0;
+            ++cc;
+          }
+        }
+        if (!ok) break;
+        mma_commit(&emptyy[uc & 1]);
+      }
+      if (ok && in_chunk) mma_commit(&acc_full[cc & 1]);
+      mma_commit(&drain);
+      mbar_wait(&drain, 0, a.err, 47);
+    }
+  } else {
+    int rows = 0;
+    for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
+      int b, z, ya, yb, x0;
+      unit(u, b, z, ya, yb, x0);
+      rows += yb - ya;
+    }
+    const int q = warp & 3;  // the TMEM lane quarter this warp may read
+    const uint32_t base = tmem + ((uint32_t)(q * 32) << 16);
+    float acc[144];
+#pragma unroll
+    for (int i = 0; i < 144; ++i) acc[i] = 0.f;
+    const uint32_t chunks = (uint32_t)((rows + chunk - 1) / chunk);
+    for (uint32_t cc = 0; cc < chunks; ++cc) {
+      if (!mbar_wait(&acc_full[cc & 1], (cc >> 1) & 1, a.err, 49)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int j = 0; j < 9; ++j) {
+        float v[16];
+        tmem_ld16(base + 256 * (cc & 1) + 16 * j, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[16 * j + i] += v[i];
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[cc & 1]);
+    }
+    // accumulator row m = 8 * plane + channel; columns dx * 48 + ii * 16 + co, dY row j - 1 + ii
+    constexpr int cin = 16 * NIN;
+    const int m = q * 32 + lane, plane = m >> 3, c = m & 7;
+    const int dz = plane / (2 * NIN), ci = (plane / 2 % NIN) * 16 + (plane & 1) * 8 + c;
+    float *out = a.partial + (size_t)blockIdx.x * (27 * cin + 1) * 16;
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int ii = 0; ii < 3; ++ii) {
+        const float *v = acc + dx * 48 + ii * 16;
+        int row = -1;
+        if (plane < 6 * NIN) row = (dz * 9 + (2 - ii) * 3 + dx) * cin + ci;
+        else if (m == 48 * NIN && dx == 1 && ii == 1) row = 27 * cin;  // ones: the bias
+        if (row >= 0) {
+          float4 *o = reinterpret_cast<float4 *>(out + (size_t)row * 16);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) o[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        }
+      }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
+}
+
+// ---- the 1-channel FP32 input ----------------------------------------------------------
+// A block walks rows (b, z, y) in pieces of up to 128 voxels: the nine input
+// lines around the piece and its dY (as FP32) are staged in shared memory; a
+// thread owns one (dz, dy) line, four output channels and one of seven x
+// segments, and slides a three-voxel window along it: one input value and one
+// 16-byte dY quad feed 12 FMAs.  The seven segments' sums are added in order at
+// the end.  (A thread per tap
+// re-reading global memory 2.29 ms at 64^3, batch 4; this 0.12 ms, bound by the
+// shared-memory reads: 2 per 12 FMAs.)
+constexpr int kDwInThreads = 256;
+constexpr int kDwInX = 128, kDwInSeg = 7, kDwInPerSm = 6;
+constexpr int kDwInLine = kDwInX + 4;
+
+__global__ void __launch_bounds__(kDwInThreads) k_dW_in1(DwArgs a) {
+  __shared__ __align__(16) float sin[9 * kDwInLine];
+  __shared__ __align__(16) float sdy[kDwInX * 16];
+  __shared__ float red[28 * 16];
+  const int nx = a.nx, ny = a.ny, nz = a.nz;
+  const int nxb = (nx + kDwInX - 1) / kDwInX;
+  const int64_t nrow = (int64_t)ny * nz * a.nb, nunit = nrow * nxb;
+  const int t = threadIdx.x, seg = t / 36, line = (t % 36) / 4, q = t & 3;
+  float acc[3][4], bs[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) acc[0][c] = acc[1][c] = acc[2][c] = bs[c] = 0.f;
+  for (int64_t u = blockIdx.x; u < nunit; u += gridDim.x) {
+    const int64_t row = u / nxb;
+    const int x0 = (int)(u - row * nxb) * kDwInX, w = min(kDwInX, nx - x0);
+    const int y = (int)(row % ny), z = (int)(row / ny % nz);
+    __syncthreads();  // the previous piece has been read
+    for (int e = t; e < 9 * (kDwInX + 2); e += kDwInThreads) {
+      const int l = e / (kDwInX + 2), i = e - l * (kDwInX + 2), x = x0 + i - 1;
+      const int dz = l / 3 - 1, dy = l % 3 - 1;
+      const bool in = (unsigned)x < (unsigned)nx && (unsigned)(y + dy) < (unsigned)ny && (unsigned)(z + dz) < (unsigned)nz;
+      sin[l * kDwInLine + i] = in ? __ldg(a.x_f32 + (row + dz * ny + dy) * nx + x) : 0.f;
+    }
+    for (int e = t; e < 2 * w; e += kDwInThreads) {
+      const int h = e / w, x = e - h * w;
+      const uint4 p = *reinterpret_cast<const uint4 *>(a.dy + act_unit(row, h, x0 + x, nx) * 8);
+      const __nv_bfloat162 *p2 = reinterpret_cast<const __nv_bfloat162 *>(&p);
+      const float2 f0 = __bfloat1622float2(p2[0]), f1 = __bfloat1622float2(p2[1]);
+      const float2 f2 = __bfloat1622float2(p2[2]), f3 = __bfloat1622float2(p2[3]);
+      float4 *d = reinterpret_cast<float4 *>(sdy + x * 16 + 8 * h);
+      d[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
+      d[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+    }
+    __syncthreads();
+    if (seg < kDwInSeg) {
+      const int segx = (w + kDwInSeg - 1) / kDwInSeg, xa = seg * segx, xb = min(w, xa + segx);
+      if (xa < xb) {
+        const float *s = sin + line * kDwInLine;  // voxel x's taps: s[x], s[x + 1], s[x + 2]
+        float v0 = s[xa], v1 = s[xa + 1];
+        for (int x = xa; x < xb; ++x) {
+          const float v2 = s[x + 2];
+          const float4 d = *reinterpret_cast<const float4 *>(sdy + x * 16 + 4 * q);
+          const float dv[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            acc[0][c] = fmaf(v0, dv[c], acc[0][c]);
+            acc[1][c] = fmaf(v1, dv[c], acc[1][c]);
+            acc[2][c] = fmaf(v2, dv[c], acc[2][c]);
+            bs[c] += dv[c];
+          }
+          v0 = v1;
+          v1 = v2;
+        }
+      }
+    }
+  }
+  for (int s = 0; s < kDwInSeg; ++s) {  // the segments in order
+    __syncthreads();
+    if (seg == s) {
+#pragma unroll
+      for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float *r = red + (line * 3 + dx) * 16 + 4 * q + c;
+          *r = s ? *r + acc[dx][c] : acc[dx][c];
+        }
+      if (line == 4)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float *r = red + 27 * 16 + 4 * q + c;
+          *r = s ? *r + bs[c] : bs[c];
+        }
+    }
+  }
+  __syncthreads();
+  for (int e = t; e < 28 * 16; e += kDwInThreads) a.partial[(size_t)blockIdx.x * 28 * 16 + e] = red[e];
+}
+
+// Partials of one layer's gradient (a.partial holds max_blocks of them); *blocks: how many.
+int launch_dW(const DwArgs &a, int max_blocks, int *err, int num_sms, cudaStream_t s, int *blocks) {
+  if (a.x_f32) {
+    const int64_t units = (int64_t)a.ny * a.nz * a.nb * ((a.nx + kDwInX - 1) / kDwInX);
+    // its partials are 1/30 of a 32-channel layer's, which max_blocks counts
+    *blocks = (int)std::min<int64_t>(std::min(30 * max_blocks, kDwInPerSm * num_sms), units);
+    k_dW_in1<<<*blocks, kDwInThreads, 0, s>>>(a);
+    HPCCG_CUDA(cudaGetLastError());
+    return HPCCG_OK;
+  }
+  DwTcArgs t{};
+  t.g.nx = a.nx;
+  t.g.ny = a.ny;
+  t.g.nz = a.nz;
+  t.g.nb = a.nb;
+  t.x0 = a.x0;
+  t.x1 = a.x1;
+  t.dy = a.dy;
+  t.partial = a.partial;
+  t.err = err;
+  t.kx = std::min(kDwMaxX, (a.nx + 15) / 16 * 16);
+  t.nxb = (a.nx + kDwMaxX - 1) / kDwMaxX;
+  t.nyb = (a.ny + kDwRows - 1) / kDwRows;
+  const int64_t units = (int64_t)t.nxb * t.nyb * a.nz * a.nb;
+  if (units >= ((int64_t)1 << 31)) return HPCCG_ERR_TOO_LARGE;
+  t.nunits = (int)units;
+  *blocks = (int)std::min<int64_t>(std::min(max_blocks, num_sms), units);
+  static_assert(dw_smem_bytes(2, kDwMaxX) <= 226 * 1024, "shared memory of a CTA");
+  const int nin = a.cin / 16, smem = dw_smem_bytes(nin, t.kx);
+  auto kern = nin == 2 ? k_dW_tc<2> : k_dW_tc<1>;
+  // the attribute is per device: set every time, to the most any width needs
+  HPCCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_smem_bytes(nin, kDwMaxX)));
+  kern<<<*blocks, kDwThreads, smem, s>>>(t);
+  HPCCG_CUDA(cudaGetLastError());
+  return HPCCG_OK;
+}
+
+}  // namespace hpccg

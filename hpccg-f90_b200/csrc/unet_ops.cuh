@@ -38,7 +38,6 @@ __global__ void k_pool_bwd(const float *dc, float *df, int nx, int ny, int nz, i
 __global__ void k_up_bwd(const float *df, float *dc, int nx, int ny, int nz, int nb);
 __global__ void k_relu_mask(const float *d, const __nv_bfloat16 *act, __nv_bfloat16 *out, int64_t n);
 __global__ void k_add_f32(const float *src, float *dst, int64_t n);
-__global__ void k_dW(DwArgs a);
 __global__ void k_reduce_partials(const float *partial, int nblocks, int n, float *grad, int accumulate);
 __global__ void k_proj_fwd(const __nv_bfloat16 *act, const float *proj, float *out, int64_t nvox, int nx);
 __global__ void k_proj_bwd(const __nv_bfloat16 *act, const float *proj, const float *dout, __nv_bfloat16 *dact,
@@ -48,5 +47,9 @@ __global__ void k_energy(const float *out, const float *tgt, float *dout, float 
                          int nb);
 __global__ void k_adam(float *p, const float *g, float *m, float *v, int n, float lr, float b1, float b2, float eps,
                        float c1, float c2);
+
+// Weight and bias gradient partials of one layer (unet_dw.cu): at most max_blocks
+// of [27*cin + 1][16] in a.partial; *blocks receives their number.
+int launch_dW(const DwArgs &a, int max_blocks, int *err, int num_sms, cudaStream_t s, int *blocks);
 
 }  // namespace hpccg

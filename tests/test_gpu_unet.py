@@ -152,6 +152,26 @@ def test_gradients_match_oracle(env):
         assert err <= 6e-2, (l, err)
 
 
+@pytest.mark.parametrize("nx,ny,nz,nb", [(24, 16, 40, 2), (136, 16, 16, 1), (40, 24, 16, 1)])
+def test_gradients_ragged_shapes(env, nx, ny, nz, nb):
+    """Rows that are no multiple of 16 voxels, a second x block of 8 voxels, partial
+    blocks of y rows; the bar of the 16^3 test (BF16 activations set it, not the sums)."""
+    torch, hp = env
+    net, p = _net_and_params(hp, seed=11)
+    rng = np.random.default_rng(nx)
+    r = rng.normal(0, 1, (nb, nz, ny, nx))
+    t = rng.normal(0, 0.05, (nb, nz, ny, nx))
+    _, g_ref = uo.loss_grad(p, r, t)
+    din = torch.from_numpy(r.astype(np.float32)).cuda()
+    dt = torch.from_numpy(t.astype(np.float32)).cuda()
+    _, g = net.loss_grad(din, dt, nx, ny, nz, nb, want_grad=True)
+    off, n = uo.offsets()
+    for l in range(14):
+        a, b = off[l], (off[l + 1] if l < 13 else n)
+        err = np.linalg.norm(g[a:b] - g_ref[a:b]) / (np.linalg.norm(g_ref[a:b]) + 1e-30)
+        assert err <= 6e-2, (l, err)
+
+
 def test_trained_network_reduces_fcg_iterations(env):
     """What the trained network gains: FCG iterations to FP64 rel-res 1e-8 on
     held-out Gaussian-random-field right-hand sides, against plain CG through
