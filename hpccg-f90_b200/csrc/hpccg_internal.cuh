@@ -173,5 +173,8 @@ int launch_spmv(hpccg_ctx *c, const double *x, double *y, cudaStream_t s);
 int autotune_spmv(hpccg_ctx *c);
 int ensure_workspace(hpccg_ctx *c, int32_t hist_cap);
 void release_mixed(const hpccg_ctx *c);
+// cuTensorMapEncodeTiled without interleave or swizzle, zeros outside the tensor.
+int encode_tmap(CUtensorMap *map, CUtensorMapDataType type, int rank, const void *base, const cuuint64_t *dims,
+                const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapL2promotion l2);
 
 }  // namespace hpccg

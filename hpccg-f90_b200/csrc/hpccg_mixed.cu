@@ -488,10 +488,8 @@ __global__ void __launch_bounds__(kBlock) k_spmv_lp_tma(TmaTile t, const __grid_
 static PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 static std::mutex g_encode_mu;
 
-// A 3D tensor map over a grid vector of `esize`-byte elements, box box_x x box_y x 1;
-// out-of-grid elements of a box read as zeros.
-static int encode_grid_tmap(CUtensorMap *map, CUtensorMapDataType type, int esize, const void *base, int nx, int ny,
-                            int nz, int box_x, int box_y) {
+int encode_tmap(CUtensorMap *map, CUtensorMapDataType type, int rank, const void *base, const cuuint64_t *dims,
+                const cuuint64_t *strides, const cuuint32_t *box, CUtensorMapL2promotion l2) {
   {
     std::lock_guard<std::mutex> lk(g_encode_mu);
     if (!g_encode) {
@@ -504,17 +502,24 @@ static int encode_grid_tmap(CUtensorMap *map, CUtensorMapDataType type, int esiz
       g_encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
     }
   }
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  const CUresult r = g_encode(map, type, (cuuint32_t)rank, const_cast<void *>(base), dims, strides, box, estr,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, l2,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? HPCCG_OK : HPCCG_ERR_UNSUPPORTED;
+}
+
+// A 3D tensor map over a grid vector of `esize`-byte elements, box box_x x box_y x 1;
+// out-of-grid elements of a box read as zeros.
+static int encode_grid_tmap(CUtensorMap *map, CUtensorMapDataType type, int esize, const void *base, int nx, int ny,
+                            int nz, int box_x, int box_y) {
   // 16-byte base, row and plane strides; 16-byte inner box extent
   if ((reinterpret_cast<uintptr_t>(base) & 15) || ((int64_t)nx * esize) % 16 || ((int64_t)box_x * esize) % 16)
     return HPCCG_ERR_UNSUPPORTED;
   const cuuint64_t dims[3] = {(cuuint64_t)nx, (cuuint64_t)ny, (cuuint64_t)nz};
   const cuuint64_t strides[2] = {(cuuint64_t)nx * esize, (cuuint64_t)nx * ny * esize};
   const cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_y, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = g_encode(map, type, 3, const_cast<void *>(base), dims, strides, box, estr,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? HPCCG_OK : HPCCG_ERR_UNSUPPORTED;
+  return encode_tmap(map, type, 3, base, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
 }
 
 int make_stencil_tmap(CUtensorMap *map, const float *base, int nx, int ny, int nz, int box_y, int box_x) {

@@ -9,7 +9,7 @@
 //   decoder       : c3a = relu(conv(e3b ++ up(e4b))), c3b;  c2a(e2b ++ up(c3b)), c2b;
 //                   out = proj . relu(conv(e1b ++ up(c2b))) + b  (1 channel, FP32)
 // "++" is a virtual concatenation: the conv reads both 16-channel tensors.
-// 16-channel convs on volumes of >= 128 voxels run on tcgen05 (unet_conv.cu),
+// 16-channel convs on volumes of >= 128 voxels run on tcgen05 (unet_conv_win.cu),
 // the 1-channel input conv and smaller volumes on CUDA cores (unet_ops.cu).
 #include <stdlib.h>
 
@@ -166,7 +166,7 @@ static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, c
     a.proj = proj;
     a.out = out;
     a.err = u->d_err;
-    return launch_conv3_tc(nin, epi, a, u->num_sms, u->stream);
+    return launch_conv3_win(nin, epi, a, u->num_sms, u->stream);
   }
   if (in_f32 && (epi == kEpiBiasRelu || epi == kEpiBias)) {  // the 1-channel input layer
     if (Lv.nx % 128 == 0)  // tensor cores, 128-voxel row tiles
@@ -595,7 +595,7 @@ extern "C" int hpccg_unet_conv3_layer(int32_t nx, int32_t ny, int32_t nz, int32_
     a.proj = d_proj;
     a.out = d_out;
     a.err = d_err;
-    rc = launch_conv3_tc(nin, epi, a, sms, 0, path == 2);
+    rc = path == 2 ? launch_conv3_brick(nin, epi, a, sms, 0) : launch_conv3_win(nin, epi, a, sms, 0);
     if (cudaDeviceSynchronize() != cudaSuccess) rc = set_cuda_error(cudaGetLastError(), "conv3 tc", __FILE__, __LINE__);
     cudaFree(packed);
   } else {

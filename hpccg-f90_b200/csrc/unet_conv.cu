@@ -1,7 +1,8 @@
-// unet_conv.cu -- tcgen05 3x3x3 convolution kernels (layout and roles in
-// unet_conv.cuh).  Operand tiles arrive by 1D bulk copies of row-planar spans;
-// grid faces are zero-filled with ordinary stores, fenced into the async proxy
-// before the tensor cores read them.
+// unet_conv.cu -- the brick form of the tcgen05 3x3x3 convolutions and the
+// 1-channel input layer (layout in unet_conv.cuh; the network's 16- and
+// 32-channel layers run the kernels of unet_conv_win.cu).  Operand tiles arrive
+// by 1D bulk copies of row-planar spans; grid faces are zero-filled with ordinary
+// stores, fenced into the async proxy before the tensor cores read them.
 #include <stdlib.h>
 
 #include <algorithm>
@@ -88,39 +89,6 @@ __device__ __forceinline__ uint32_t conv_setup(const ConvArgs &a, uint8_t *sW, u
   }
   if (warp == 1) {
     tmem_alloc(slot, 32);
-    tmem_relinquish();
-  }
-  fence_proxy_async_smem();  // weights -> tensor-core proxy
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  return *slot;
-}
-
-// Set-up of the row kernel: weights, the barriers of each of the P pipelines
-// (pipeline p starts at rings + p*pipe_bytes; its 2R+5 barriers follow its ring
-// of ring_bytes), and
-// 32*P TMEM columns allocated by warp 1; the TMEM base lands in *slot.
-template <int NIN, int R, int P>
-__device__ __forceinline__ uint32_t conv_setup_row(const ConvArgs &a, uint8_t *sW, uint8_t *rings, int ring_bytes,
-                                                   int pipe_bytes, uint32_t *slot, int warp) {
-  constexpr int kWBytes = NIN * 27 * kWTapBytes;
-  for (int i = threadIdx.x; i < kWBytes / 16; i += blockDim.x)
-    reinterpret_cast<uint4 *>(sW)[i] = reinterpret_cast<const uint4 *>(a.wpack)[i];
-  if (threadIdx.x == 0) {
-    for (int p = 0; p < P; ++p) {
-      uint64_t *bars = reinterpret_cast<uint64_t *>(rings + p * pipe_bytes + ring_bytes);
-      for (int s = 0; s < 2 * R; ++s) mbar_init(&bars[s], 1);
-      mbar_init(&bars[2 * R + 0], 1);
-      mbar_init(&bars[2 * R + 1], 1);
-      mbar_init(&bars[2 * R + 2], 4);
-      mbar_init(&bars[2 * R + 3], 4);
-      mbar_init(&bars[2 * R + 4], 1);
-    }
-    fence_mbar_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(slot, 32 * P);
     tmem_relinquish();
   }
   fence_proxy_async_smem();  // weights -> tensor-core proxy
@@ -241,184 +209,6 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv3_brick(ConvArgs a) {
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem, 32);
-  }
-}
-
-// ---- row tiles: rolling window of slabs along y -------------------------------------------
-struct RowUnits {
-  int nxb, nchunks, nunits;
-};
-template <int RX>
-__host__ __device__ __forceinline__ RowUnits row_units(const ConvGeom &g) {
-  RowUnits r;
-  r.nxb = g.nx / RX;
-  r.nchunks = (g.ny + row_chunk(RX) - 1) / row_chunk(RX);
-  r.nunits = r.nxb * g.nz * g.nb * r.nchunks;
-  return r;
-}
-struct RowUnit {
-  int b, z, x0, ya, yb;
-};
-template <int RX>
-__device__ __forceinline__ RowUnit row_unit(const ConvGeom &g, const RowUnits &ru, int u) {
-  RowUnit w;
-  const int c = u % ru.nchunks;
-  int r = u / ru.nchunks;
-  w.x0 = (r % ru.nxb) * RX;
-  r /= ru.nxb;
-  w.z = r % g.nz;
-  w.b = r / g.nz;
-  w.ya = c * row_chunk(RX);
-  w.yb = min(g.ny, w.ya + row_chunk(RX));
-  return w;
-}
-// Tile index (as tile_origin decodes it, g.bx = RX) of row y of a unit.
-template <int RX>
-__device__ __forceinline__ int row_tile_index(const ConvGeom &g, const RowUnit &w, int y) {
-  return ((w.b * g.nz + w.z) * g.ny + y) * g.tx + w.x0 / RX;
-}
-
-// RX = 128: one TMEM lane per voxel.  RX = 64 (MMA M = 64): voxel row m of the
-// tile sits in TMEM lane (m / 16) * 32 + m % 16, i.e. lanes 0-15 of each
-// warp's quarter (checked on the GPU by dumping an M = 64 accumulator).
-template <int NIN, int EPI, int RX>
-__global__ void __launch_bounds__(kConvThreads * row_pipes(NIN, RX), 1) k_conv3_row(ConvArgs a) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int P = row_pipes(NIN, RX);
-  constexpr int kWBytes = NIN * 27 * kWTapBytes;
-  constexpr int kSlab = slab_bytes(NIN, RX);
-  constexpr int R = row_slots(NIN, RX, P);
-  constexpr int kRowVox = row_vox(RX), kSlabPlaneBytes = slab_plane_bytes(RX);
-  static_assert(RX == 128 || RX == 64, "MMA M is 128 or 64");
-  static_assert((2 * R + 5) * 8 + 4 <= bar_bytes(R), "barrier area");
-  static_assert(R >= 4, "the window needs the three slabs of a tile plus one in flight");
-  constexpr int kPipeBytes = row_pipe_bytes(NIN, RX);
-  static_assert(R * kSlab + bar_bytes(R) <= kPipeBytes && kPipeBytes % 128 == 0, "shared memory plan");
-  // pipeline `pipe` = warps 6*pipe .. 6*pipe+5 in the roles producer, MMA, 4 x epilogue;
-  // it owns units blockIdx.x + (k*P + pipe)*gridDim.x, its slab ring, its barriers
-  // and TMEM columns 32*pipe .. +31
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pipe = warp / 6, role = warp % 6;
-  uint8_t *sW = smem;
-  uint8_t *sA = smem + kWBytes + pipe * kPipeBytes;
-  uint64_t *full = reinterpret_cast<uint64_t *>(sA + R * kSlab);
-  uint64_t *empty = full + R;
-  uint64_t *acc_full = empty + R;
-  uint64_t *acc_empty = acc_full + 2;
-  uint64_t *drain = acc_empty + 2;
-  uint32_t *slot = reinterpret_cast<uint32_t *>(smem + kWBytes + R * kSlab + 2 * R * 8 + 5 * 8);  // pipeline 0's
-  const uint32_t tmem = conv_setup_row<NIN, R, P>(a, sW, smem + kWBytes, R * kSlab, kPipeBytes, slot, warp) + 32 * pipe;
-  const ConvGeom &g = a.g;
-  const RowUnits ru = row_units<RX>(g);
-  const int u0 = blockIdx.x + pipe * gridDim.x, ustep = P * gridDim.x;
-
-  if (role == 0) {
-    // fetch slabs ya-1 .. yb of every unit: NIN x 2 halves x 3 z-rows spans
-    uint32_t sc = 0;
-    bool ok = true;
-    for (int u = u0; u < ru.nunits && ok; u += ustep) {
-      const RowUnit w = row_unit<RX>(g, ru, u);
-      for (int ys = w.ya - 1; ys <= w.yb; ++ys, ++sc) {
-        const int s = sc % R;
-        const uint32_t n = sc / R;
-        if (n > 0 && !(ok = warp_wait(&empty[s], (n - 1) & 1, a.err, 11, lane))) break;
-        uint8_t *base = sA + s * kSlab;
-        Span sp[1];
-        int nsp = 0;
-        if (lane < 6 * NIN) {
-          const int r = lane % 3, h = (lane / 3) & 1, in = lane / 6;
-          sp[0] = plan_span(g, in ? a.in1 : a.in0, w.b, w.z + r - 1, ys, h, w.x0 - 1, kRowVox,
-                            base + (in * 2 + h) * kSlabPlaneBytes + r * kRowVox * 16);
-          nsp = 1;
-        }
-        post_spans(sp, nsp, &full[s], lane);
-      }
-    }
-    if (lane == 0) {
-      const uint32_t first = sc > (uint32_t)R ? sc - R : 0;
-      for (uint32_t j = first; j < sc; ++j) mbar_wait(&full[j % R], (j / R) & 1, a.err, 15);
-    }
-  } else if (role == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16(RX, 16);
-      const uint64_t wd = smem_desc(sW, 256, 128);
-      uint32_t sc0 = 0, tcount = 0;
-      bool ok = true;
-      for (int u = u0; u < ru.nunits && ok; u += ustep) {
-        const RowUnit w = row_unit<RX>(g, ru, u);
-        const int ntile = w.yb - w.ya;
-        uint32_t ready = sc0;  // slabs [sc0, ready) have been waited for
-        for (int i = 0; i < ntile; ++i, ++tcount) {
-          const int buf = tcount & 1;
-          const uint32_t use = tcount >> 1;
-          if (use > 0 && !(ok = mbar_wait(&acc_empty[buf], (use - 1) & 1, a.err, 12))) break;
-          for (; ready < sc0 + i + 3; ++ready)
-            if (!(ok = mbar_wait(&full[ready % R], (ready / R) & 1, a.err, 13))) break;
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t d = tmem + (uint32_t)(buf * 16);
-          // descriptors of the three slabs (y-1, y, y+1); a tap adds a constant
-          // offset (address field in 16-byte units, no carry: smem < 256 KB)
-          uint64_t sd[3];
-#pragma unroll
-          for (int j = 0; j < 3; ++j) sd[j] = smem_desc(sA + ((sc0 + i + j) % R) * kSlab, kSlabPlaneBytes, 128);
-          // taps in dy-major order: the nine of dy = -1 first, so slab y-1 (this
-          // tile is its last user) is released as soon as they complete and the
-          // producer refills its slot while the other 18 run
-#pragma unroll
-          for (int ks = 0; ks < 27 * NIN; ++ks) {
-            const int t = ks / NIN, in = ks % NIN;
-            const int dyp = t / 9, dzp = (t / 3) % 3, dxp = t % 3;  // offsets + 1
-            const int tap = dzp * 9 + dyp * 3 + dxp;
-            const uint64_t ad = sd[dyp] + (uint64_t)((in * 2 * kSlabPlaneBytes + (dzp * kRowVox + dxp) * 16) >> 4);
-            const uint64_t bd = wd + (uint64_t)(((in * 27 + tap) * kWTapBytes) >> 4);
-            mma_bf16(d, ad, bd, idesc, ks > 0 ? 1u : 0u);
-            if (ks == 9 * NIN - 1) mma_commit(&empty[(sc0 + i) % R]);  // slab y-1 is done for the unit
-          }
-          mma_commit(&acc_full[buf]);
-        }
-        if (!ok) break;
-        mma_commit(&empty[(sc0 + ntile) % R]);  // the unit's last two slabs
-        mma_commit(&empty[(sc0 + ntile + 1) % R]);
-        sc0 += ntile + 2;
-      }
-      mma_commit(drain);
-      mbar_wait(drain, 0, a.err, 16);
-    }
-  } else {
-    // epilogue: tiles in unit order
-    const int q = warp & 3;
-    uint32_t tcount = 0;
-    float bias[16], proj[17];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) bias[c] = (EPI == kEpiRawF32 || !a.bias) ? 0.f : a.bias[c];
-    if (EPI == kEpiProject)
-#pragma unroll
-      for (int c = 0; c < 17; ++c) proj[c] = a.proj[c];
-    bool ok = true;
-    for (int u = u0; u < ru.nunits && ok; u += ustep) {
-      const RowUnit w = row_unit<RX>(g, ru, u);
-      for (int y = w.ya; y < w.yb; ++y, ++tcount) {
-        const int buf = tcount & 1;
-        if (!(ok = mbar_wait(&acc_full[buf], (tcount >> 1) & 1, a.err, 14))) break;
-        tc_fence_after();
-        float v[16];
-        tmem_ld16(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 16), v);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[buf]);
-        if (RX == 128)
-          conv_store<EPI>(a, row_tile_index<RX>(g, w, y), q * 32 + lane, v, bias, proj);
-        else if (lane < 16)
-          conv_store<EPI>(a, row_tile_index<RX>(g, w, y), q * 16 + lane, v, bias, proj);
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem - 32 * pipe, 32 * P);
   }
 }
 
@@ -624,59 +414,34 @@ int launch_conv3_in1_tc(const float *in, const float *W, const float *bias, __nv
   return HPCCG_OK;
 }
 
-// RX = 0: brick tiles; 128 / 64: row tiles of that many voxels.
-template <int NIN, int EPI, int RX>
-static int launch_one(const ConvArgs &a, int num_sms, cudaStream_t s) {
-  constexpr bool ROW = RX != 0;
-  constexpr int smem = ROW ? row_smem_bytes(NIN, RX == 0 ? 128 : RX) : brick_smem_bytes(NIN);
+template <int NIN, int EPI>
+static int launch_brick(const ConvArgs &a, int num_sms, cudaStream_t s) {
+  constexpr int smem = brick_smem_bytes(NIN);
   static_assert(smem <= 227 * 1024, "conv CTA exceeds the shared-memory limit");
-  auto kern = ROW ? k_conv3_row<NIN, EPI, RX == 0 ? 128 : RX> : k_conv3_brick<NIN, EPI>;
-  static int per_sm = 0;
-  if (!per_sm) {
-    HPCCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    // resident CTAs per SM by shared memory (each CTA also reserves 1 KB)
-    per_sm = std::max(1, (227 * 1024) / (smem + 1024));
-  }
-  constexpr int pipes = ROW ? row_pipes(NIN, RX == 0 ? 128 : RX) : 1;
-  const int work = ROW ? row_units<RX == 0 ? 128 : RX>(a.g).nunits : a.g.ntiles;
-  const int grid = std::min((work + pipes - 1) / pipes, num_sms * per_sm);
-  kern<<<grid, kConvThreads * pipes, smem, s>>>(a);
+  auto kern = k_conv3_brick<NIN, EPI>;
+  // the attribute is per device: set every time
+  HPCCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  // resident CTAs per SM by shared memory (each CTA also reserves 1 KB)
+  constexpr int per_sm = (227 * 1024) / (smem + 1024);
+  kern<<<std::min(a.g.ntiles, num_sms * (per_sm > 1 ? per_sm : 1)), kConvThreads, smem, s>>>(a);
   HPCCG_CUDA(cudaGetLastError());
   return HPCCG_OK;
 }
 
-template <int NIN, int EPI>
-static int launch_mode(const ConvArgs &a, int num_sms, cudaStream_t s, int rx) {
-  if (rx == 128) return launch_one<NIN, EPI, 128>(a, num_sms, s);
-  if (rx == 64) return launch_one<NIN, EPI, 64>(a, num_sms, s);
-  return launch_one<NIN, EPI, 0>(a, num_sms, s);
-}
-
-int launch_conv3_tc(int nin, int epi, const ConvArgs &a_in, int num_sms, cudaStream_t s, bool force_brick) {
-  ConvArgs a = a_in;
-  int row = 0;
-  if (!force_brick) {
-    ConvGeom g64;
-    if (conv_row_ok(a.g)) {
-      row = 128;
-    } else if (conv_row64_geom(a.g, &g64)) {
-      a.g = g64;
-      row = 64;
-    }
-  }
+int launch_conv3_brick(int nin, int epi, const ConvArgs &a, int num_sms, cudaStream_t s) {
   if (nin == 1) {
     switch (epi) {
-      case kEpiBiasRelu: return launch_mode<1, kEpiBiasRelu>(a, num_sms, s, row);
-      case kEpiBias: return launch_mode<1, kEpiBias>(a, num_sms, s, row);
-      case kEpiProject: return launch_mode<1, kEpiProject>(a, num_sms, s, row);
-      default: return launch_mode<1, kEpiRawF32>(a, num_sms, s, row);
+      case kEpiBiasRelu: return launch_brick<1, kEpiBiasRelu>(a, num_sms, s);
+      case kEpiBias: return launch_brick<1, kEpiBias>(a, num_sms, s);
+      case kEpiProject: return launch_brick<1, kEpiProject>(a, num_sms, s);
+      default: return launch_brick<1, kEpiRawF32>(a, num_sms, s);
     }
   }
   switch (epi) {
-    case kEpiBiasRelu: return launch_mode<2, kEpiBiasRelu>(a, num_sms, s, row);
-    case kEpiBias: return launch_mode<2, kEpiBias>(a, num_sms, s, row);
-    case kEpiProject: return launch_mode<2, kEpiProject>(a, num_sms, s, row);
-    default: return launch_mode<2, kEpiRawF32>(a, num_sms, s, row);
+    case kEpiBiasRelu: return launch_brick<2, kEpiBiasRelu>(a, num_sms, s);
+    case kEpiBias: return launch_brick<2, kEpiBias>(a, num_sms, s);
+    case kEpiProject: return launch_brick<2, kEpiProject>(a, num_sms, s);
+    default: return launch_brick<2, kEpiRawF32>(a, num_sms, s);
   }
 }
 

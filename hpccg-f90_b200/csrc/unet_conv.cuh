@@ -9,19 +9,16 @@
 // are the two K chunks).  So every operand tile arrives by 1D bulk copies
 // (cp.async.bulk) of whole row spans, with zero fill at the grid faces.
 //
-// A conv is an implicit GEMM per tile of 128 (or 64) voxels: for each of the
-// 27 taps and each 16-channel input group, one tcgen05.mma (M=128 or 64,
-// N=16, K=16) accumulates into a 16-column FP32 TMEM accumulator.
-//  * row tiles (nx a multiple of 128, or nx = 64 with M = 64): a tile is one
-//    x-row; the 3x3 neighbouring rows with a 1-voxel x halo are three "slabs"
-//    shared with the neighbouring tiles in y, and the 27 taps read them through
-//    shifted descriptors (one new slab fetched per tile);
-//  * brick tiles (other narrow grids): a tile is a bx*by*bz brick of 128
-//    voxels and each tap's shifted brick is fetched separately.
-// Roles per pipeline (192 threads): warp 0 fetches (its lanes issue the row
-// spans in parallel), warp 1 allocates TMEM and lane 0 issues the MMAs, warps
-// 2-5 (one per TMEM lane quarter) run the epilogue.  Row kernels of 32-channel
-// layers run two such pipelines per CTA (384 threads) that share the weights.
+// A conv is an implicit GEMM on tcgen05 over the 27 taps and each 16-channel
+// input group, accumulated in FP32 in TMEM:
+//  * window tiles (unet_conv_win.cu): voxels are the MMA's N, eight output rows x
+//    16 channels its M;
+//  * brick tiles (unet_conv.cu): 128 voxels of a bx*by*bz brick are M, the 16
+//    channels N, each tap's shifted brick fetched on its own.  Kept as the
+//    independent form that hpccg_unet_conv3_layer offers beside the other two.
+// Roles (192 threads): warp 0 fetches (its lanes issue the row spans in
+// parallel), warp 1 allocates TMEM and lane 0 issues the MMAs, warps 2-5 (one per
+// TMEM lane quarter) run the epilogue.
 #pragma once
 #include "hpccg_internal.cuh"
 #include "unet_tc.cuh"
@@ -42,37 +39,10 @@ constexpr int kWTapBytes = 16 * 16 * 2;  // one tap of B: 16 x 16 BF16
 // Brick tiles: one stage per k-step (tap, input): 2 halves x 128 units.
 constexpr int kBrickStages = 24;
 constexpr int kBrickStageBytes = 2 * 128 * 16;
-// Row tiles of RX = 128 voxels (nx a multiple of 128; MMA M = 128) or RX = 64
-// (nx = 64; M = 64) walk y inside a work unit (b, z, RX-voxel x block, chunk of
-// up to row_chunk(RX) rows of y).  A "slab" is grid row y of the three z planes
-// z-1, z, z+1 with a 1-voxel x halo: 3 rows x (RX + 2) units per half.  Tile y
-// reads slabs y-1, y, y+1, so each tile fetches one new slab and a ring of
-// row_slots slabs keeps several fetches in flight.
-__host__ __device__ constexpr int row_vox(int rx) { return rx + 2; }
-__host__ __device__ constexpr int row_chunk(int rx) { return rx == 128 ? 32 : 8; }
-__host__ __device__ constexpr int slab_plane_bytes(int rx) { return ((3 * row_vox(rx) * 16 + 127) / 128) * 128; }
-__host__ __device__ constexpr int slab_bytes(int nin, int rx) { return nin * 2 * slab_plane_bytes(rx); }
-__host__ __device__ constexpr int row_slots(int nin, int rx, int pipes = 1) {
-  return pipes == 2 ? 4 : ((rx == 128 && nin == 1) ? 8 : 6);
-}
-// Row kernels may run two independent pipelines (producer, MMA issuer and
-// epilogue warps each, own slab ring and accumulators) in one CTA that shares
-// the weights: two MMA-issuing threads per SM where the shared memory of one
-// pipeline per CTA leaves room for only one CTA.
-__host__ __device__ constexpr int row_pipes(int nin, int rx) { return (nin == 2 && rx == 128) ? 2 : 1; }
 // mbarriers: full[S], empty[S], acc_full[2], acc_empty[2], drain, + TMEM slot.
 __host__ __device__ constexpr int bar_bytes(int stages) { return (2 * stages + 5) * 8 + 16; }
 __host__ __device__ constexpr int brick_smem_bytes(int nin) {
   return nin * 27 * kWTapBytes + kBrickStages * kBrickStageBytes + bar_bytes(kBrickStages);
-}
-// One pipeline's ring and barriers, rounded up so that the next ring starts on
-// a 128-byte boundary (bulk copies and MMA operands need 16-byte alignment).
-__host__ __device__ constexpr int row_pipe_bytes(int nin, int rx) {
-  return ((row_slots(nin, rx, row_pipes(nin, rx)) * slab_bytes(nin, rx) +
-           bar_bytes(row_slots(nin, rx, row_pipes(nin, rx))) + 127) / 128) * 128;
-}
-__host__ __device__ constexpr int row_smem_bytes(int nin, int rx) {
-  return nin * 27 * kWTapBytes + row_pipes(nin, rx) * row_pipe_bytes(nin, rx);
 }
 
 enum ConvEpi : int {
@@ -118,20 +88,6 @@ inline bool conv_geom(int nx, int ny, int nz, int nb, ConvGeom *g) {
   g->ty = ny / by;
   g->tz = nz / bz;
   g->ntiles = g->tx * g->ty * g->tz * nb;
-  return true;
-}
-inline bool conv_row_ok(const ConvGeom &g) { return g.bx == 128 && g.by == 1 && g.bz == 1; }
-// Geometry of 64-voxel row tiles for nx = 64 (tile = one grid row).
-inline bool conv_row64_geom(const ConvGeom &g, ConvGeom *r) {
-  if (g.nx != 64) return false;
-  *r = g;
-  r->bx = 64;
-  r->by = 1;
-  r->bz = 1;
-  r->tx = 1;
-  r->ty = g.ny;
-  r->tz = g.nz;
-  r->ntiles = g.ny * g.nz * g.nb;
   return true;
 }
 
@@ -195,8 +151,31 @@ __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, int *e
   return ok;
 }
 
-// Launches the tensor-core conv (row tiles when possible unless force_brick).
-int launch_conv3_tc(int nin, int epi, const ConvArgs &a, int num_sms, cudaStream_t s, bool force_brick = false);
+// Tensor maps of an activation tensor.  Elements are 8 bytes (half of a 16-byte
+// unit), so a box may be 128 units long in x; zeros outside the grid.  The box's
+// dimensions come in the given order, each with its extent in the box.
+enum ActDim : int { kDimH, kDimY, kDimZ };
+inline int act_tmap(CUtensorMap *map, const __nv_bfloat16 *base, const ConvGeom &g, int box_units, ActDim d1, int n1,
+                    ActDim d2, int n2, ActDim d3, int n3) {
+  const ActDim d[3] = {d1, d2, d3};
+  const int n[3] = {n1, n2, n3};
+  cuuint64_t dims[5] = {(cuuint64_t)2 * g.nx, 0, 0, 0, (cuuint64_t)g.nb}, strides[4];
+  cuuint32_t box[5] = {(cuuint32_t)(2 * box_units), 0, 0, 0, 1};
+  const cuuint64_t row = (cuuint64_t)g.nx * 32;  // bytes of a grid row, both halves
+  for (int i = 0; i < 3; ++i) {
+    dims[i + 1] = d[i] == kDimH ? 2 : (d[i] == kDimY ? g.ny : g.nz);
+    strides[i] = d[i] == kDimH ? row / 2 : (d[i] == kDimY ? row : row * g.ny);
+    box[i + 1] = (cuuint32_t)n[i];
+  }
+  strides[3] = row * g.ny * g.nz;
+  return encode_tmap(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, base, dims, strides, box,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+}
+
+// Launch the tensor-core conv: window tiles (any volume; reads nx, ny, nz, nb of
+// a.g only) and brick tiles (a.g from conv_geom).
+int launch_conv3_win(int nin, int epi, const ConvArgs &a, int num_sms, cudaStream_t s);
+int launch_conv3_brick(int nin, int epi, const ConvArgs &a, int num_sms, cudaStream_t s);
 // The 1-channel input layer (FP32 input [nb][nz][ny][nx], W [27][16], bias [16])
 // on the tensor cores, BF16 operands, FP32 accumulation; nx a multiple of 128,
 // else HPCCG_ERR_UNSUPPORTED.

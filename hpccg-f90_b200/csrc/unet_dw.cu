@@ -18,7 +18,7 @@ using namespace tc;
 // row-planar layout holds, for 8 channels, 8 consecutive voxels as 128
 // contiguous bytes, which is a no-swizzle core matrix of 8 channels x 8 voxels.
 // For one x row j of X (three z planes, all input groups) the A operand's M
-// index is (dz, input group, half, channel) -- planes of one slab at a uniform
+// index is (input group, half, dz, channel) -- planes of one slab at a uniform
 // stride -- and B's N index is (dY row j-1, j, j+1; co): one MMA of M = 128,
 // N = 48, K = 16 voxels forms the nine (dz, dy) taps of all channels, and the
 // three dx taps are the same A shifted by one voxel (16 bytes) into three
@@ -32,8 +32,8 @@ using namespace tc;
 // added up in registers with rounded FP32 additions (1.6e-7); two accumulator
 // sets let the drain run under the next steps' MMAs.
 //
-// A unit is (batch, z, 8 rows of y, up to 128 voxels of x): its ten dY rows
-// (double-buffered) and a ring of X slabs arrive by bulk copies of row spans.
+// A unit is (batch, z, 8 rows of y, up to 112 voxels of x): its ten dY rows
+// (double-buffered) and the X slabs (a ring) arrive by TMA, one box per tensor.
 // Rows outside the grid, the x halo and the padding of dY to whole 16-voxel
 // steps are zeros.  A's rows past the ones plane read whatever follows in
 // shared memory; they only reach accumulator rows that nobody stores.
@@ -46,19 +46,20 @@ using namespace tc;
 constexpr int kDwThreads = 192;  // producer warp, MMA warp, four draining warps
 constexpr int kDwRows = 8;   // y rows per unit
 constexpr int kDwSlots = 4;  // X slabs in flight
-constexpr int kDwMaxX = 128;
+constexpr int kDwMaxX = 112;  // with the pitch's 8 more units a box of at most 128
 constexpr int kDwChain = 8;  // MMA steps between two drains
 
 struct DwTcArgs {
   ConvGeom g;  // volume and batch only
-  const __nv_bfloat16 *x0, *x1, *dy;
+  CUtensorMap xmap[2], ymap;  // boxes: pitch units x 3 z x 2 halves; kx units x 2 halves x 10 y
   float *partial;
   int *err;
   int kx;                    // voxels per unit row, a multiple of 16
   int nxb, nyb, nunits;      // x and y blocks, units
 };
 
-__host__ __device__ constexpr int dw_plane_bytes(int kx) { return (kx + 2) * 16; }
+// a plane's pitch: one-voxel halos, rounded so that every box starts on 128 bytes
+__host__ __device__ constexpr int dw_plane_bytes(int kx) { return (kx + 8) * 16; }
 __host__ __device__ constexpr int dw_planes(int nin) { return 6 * nin + 1; }
 __host__ __device__ constexpr int dw_dy_bytes(int kx) { return (kDwRows + 2) * 2 * kx * 16; }
 // dY buffers, slabs, and the planes that the last slab's M = 128 rows read beyond it
@@ -72,7 +73,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) {
 }
 
 template <int NIN>
-__global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(DwTcArgs a) {
+__global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__ DwTcArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t fullx[kDwSlots], emptyx[kDwSlots], fully[2], emptyy[2], acc_full[2], acc_empty[2], drain;
   __shared__ uint32_t slot;
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(DwTcArgs a) {
   const uint32_t tmem = slot;
   const int ksteps = a.kx / 16, chunk = max(1, kDwChain / ksteps);  // rows between two drains
   auto unit = [&](int u, int &b, int &z, int &ya, int &yb, int &x0) {
-    x0 = (u % a.nxb) * kDwMaxX;
+    x0 = (u % a.nxb) * a.kx;
     u /= a.nxb;
     ya = (u % a.nyb) * kDwRows;
     yb = min(g.ny, ya + kDwRows);
@@ -119,34 +120,27 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(DwTcArgs a) {
     b = u / g.nz;
   };
   if (warp == 0) {
-    uint32_t sc = 0, uc = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x, ++uc) {
-      int b, z, ya, yb, x0;
-      unit(u, b, z, ya, yb, x0);
-      const int yp = uc & 1;
-      if (uc >= 2 && !(ok = warp_wait(&emptyy[yp], ((uc >> 1) - 1) & 1, a.err, 41, lane))) break;
-      Span sp[1];
-      int nsp = 0;
-      if (lane < 2 * (kDwRows + 2)) {
-        sp[0] = plan_span(g, a.dy, b, z, ya - 1 + (lane >> 1), lane & 1, x0, a.kx, sY + yp * dyb + lane * a.kx * 16);
-        nsp = 1;
-      }
-      post_spans(sp, nsp, &fully[yp], lane);
-      for (int y = ya; y < yb; ++y, ++sc) {
-        const int s = sc % kDwSlots;
-        const uint32_t n = sc / kDwSlots;
-        if (n > 0 && !(ok = warp_wait(&emptyx[s], (n - 1) & 1, a.err, 42, lane))) break;
-        nsp = 0;
-        if (lane < 6 * NIN) {  // plane (dz, input group, half) = lane
-          const int h = lane & 1, in = (lane >> 1) % NIN, dz = (lane >> 1) / NIN;
-          sp[0] = plan_span(g, in ? a.x1 : a.x0, b, z + dz - 1, y, h, x0 - 1, a.kx + 2, sX + s * slab + lane * ps);
-          nsp = 1;
+    if (lane == 0) {
+      uint32_t sc = 0, uc = 0;
+      bool ok = true;
+      for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x, ++uc) {
+        int b, z, ya, yb, x0;
+        unit(u, b, z, ya, yb, x0);
+        const int yp = uc & 1;
+        if (uc >= 2 && !(ok = mbar_wait(&emptyy[yp], ((uc >> 1) - 1) & 1, a.err, 41))) break;
+        mbar_expect_tx(&fully[yp], dyb);
+        tma_g2s_5d(sY + yp * dyb, &a.ymap, 2 * x0, 0, ya - 1, z, b, &fully[yp]);
+        for (int y = ya; y < yb; ++y, ++sc) {
+          const int s = sc % kDwSlots;
+          const uint32_t n = sc / kDwSlots;
+          if (n > 0 && !(ok = mbar_wait(&emptyx[s], (n - 1) & 1, a.err, 42))) break;
+          mbar_expect_tx(&fullx[s], 6 * NIN * ps);
+#pragma unroll
+          for (int in = 0; in < NIN; ++in)
+            tma_g2s_5d(sX + s * slab + in * 6 * ps, &a.xmap[in], 2 * (x0 - 1), z - 1, 0, y, b, &fullx[s]);
         }
-        post_spans(sp, nsp, &fullx[s], lane);
       }
-    }
-    if (lane == 0) {  // every issued copy has landed before the CTA may exit
+      // every issued copy has landed before the CTA may exit
       for (uint32_t j = sc > (uint32_t)kDwSlots ? sc - kDwSlots : 0; j < sc; ++j)
         mbar_wait(&fullx[j % kDwSlots], (j / kDwSlots) & 1, a.err, 43);
       for (uint32_t j = uc > 2u ? uc - 2 : 0; j < uc; ++j) mbar_wait(&fully[j & 1], (j >> 1) & 1, a.err, 44);
@@ -218,7 +212,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(DwTcArgs a) {
     // accumulator row m = 8 * plane + channel; columns dx * 48 + ii * 16 + co, dY row j - 1 + ii
     constexpr int cin = 16 * NIN;
     const int m = q * 32 + lane, plane = m >> 3, c = m & 7;
-    const int dz = plane / (2 * NIN), ci = (plane / 2 % NIN) * 16 + (plane & 1) * 8 + c;
+    const int dz = plane % 3, ci = plane / 3 * 8 + c;  // plane = (input group * 2 + half) * 3 + dz
     float *out = a.partial + (size_t)blockIdx.x * (27 * cin + 1) * 16;
 #pragma unroll
     for (int dx = 0; dx < 3; ++dx)
@@ -348,19 +342,21 @@ int launch_dW(const DwArgs &a, int max_blocks, int *err, int num_sms, cudaStream
   t.g.ny = a.ny;
   t.g.nz = a.nz;
   t.g.nb = a.nb;
-  t.x0 = a.x0;
-  t.x1 = a.x1;
-  t.dy = a.dy;
   t.partial = a.partial;
   t.err = err;
-  t.kx = std::min(kDwMaxX, (a.nx + 15) / 16 * 16);
   t.nxb = (a.nx + kDwMaxX - 1) / kDwMaxX;
+  t.kx = ((a.nx + t.nxb - 1) / t.nxb + 15) / 16 * 16;
+  t.nxb = (a.nx + t.kx - 1) / t.kx;
   t.nyb = (a.ny + kDwRows - 1) / kDwRows;
   const int64_t units = (int64_t)t.nxb * t.nyb * a.nz * a.nb;
   if (units >= ((int64_t)1 << 31)) return HPCCG_ERR_TOO_LARGE;
   t.nunits = (int)units;
   *blocks = (int)std::min<int64_t>(std::min(max_blocks, num_sms), units);
   static_assert(dw_smem_bytes(2, kDwMaxX) <= 226 * 1024, "shared memory of a CTA");
+  int rc = act_tmap(&t.ymap, a.dy, t.g, t.kx, kDimH, 2, kDimY, kDwRows + 2, kDimZ, 1);
+  if (!rc) rc = act_tmap(&t.xmap[0], a.x0, t.g, t.kx + 8, kDimZ, 3, kDimH, 2, kDimY, 1);
+  if (!rc && a.cin == 32) rc = act_tmap(&t.xmap[1], a.x1, t.g, t.kx + 8, kDimZ, 3, kDimH, 2, kDimY, 1);
+  if (rc) return rc;
   const int nin = a.cin / 16, smem = dw_smem_bytes(nin, t.kx);
   auto kern = nin == 2 ? k_dW_tc<2> : k_dW_tc<1>;
   // the attribute is per device: set every time, to the most any width needs

@@ -275,7 +275,7 @@ int hpccg_unet_time_forward(hpccg_unet *unet, int32_t nx, int32_t ny, int32_t nz
  * channels; 16-channel outputs use the same layout), weights FP32 [27][16*nin][16],
  * epi 0 = bias+ReLU (BF16 out), 1 = bias (BF16), 2 = bias+ReLU then the 16->1
  * projection d_proj (FP32 out), 3 = raw FP32 16-channel out; path 0 =
- * tcgen05 (row tiles when nx is a multiple of 128), 1 = CUDA cores,
+ * tcgen05 as the network runs it (window tiles), 1 = CUDA cores,
  * 2 = tcgen05 with brick tiles (per-tap fetches).  nin = 0 is the network's
  * 1-channel input layer: d_in0 an FP32 grid [b][z][y][x], weights FP32 [27][16],
  * epi 0 or 1; path 0 = tcgen05 (nx a multiple of 128, else

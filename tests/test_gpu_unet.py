@@ -108,6 +108,43 @@ def test_input_layer_tc_and_cc(env, nx, ny, nz, nb, epi):
         assert np.all(np.abs(got - want) <= tol), (path, np.abs(got - want).max(), scale)
 
 
+@pytest.mark.parametrize("nx,ny,nz,nb", [(128, 9, 1, 1), (128, 1, 3, 1), (384, 10, 2, 1), (64, 18, 5, 1), (32, 12, 9, 2),
+                                         (16, 8, 17, 1), (8, 16, 9, 2)])
+@pytest.mark.parametrize("nin", [1, 2])
+@pytest.mark.parametrize("epi", [0, 2, 3])
+def test_conv_layer_window_edges(env, nx, ny, nz, nb, nin, epi):
+    """Partial tiles of rows and planes, several x blocks: the bars of
+    test_conv_layer_tc_and_cc, and on narrow grids (the same order of terms)
+    the bits of the brick form."""
+    torch, hp = env
+    rng = np.random.default_rng(nx + 3 * ny + nin)
+    xs = [uo.bf16_round(rng.normal(0, 1, (nb, nz, ny, nx, 16))) for _ in range(nin)]
+    W = rng.normal(0, 0.1, (27, 16 * nin, 16)).astype(np.float32)
+    b = rng.normal(0, 0.1, 16).astype(np.float32)
+    proj = rng.normal(0, 0.3, 17).astype(np.float32)
+    dW, db, dp = (torch.from_numpy(v).cuda() for v in (W, b, proj))
+    din = [_bf16_tensor(torch, to_planar(v)) for v in xs] + [None]
+    n = nx * ny * nz * nb
+    dtype, size = {0: (torch.bfloat16, 16 * n), 2: (torch.float32, n), 3: (torch.float32, 16 * n)}[epi]
+    outs = []
+    for path in (0, 2):
+        out = torch.full((size,), float("nan"), dtype=dtype, device="cuda")
+        hp.conv3_layer(din[0], din[1], dW, db, dp, epi, path, out, nx, ny, nz, nb)
+        outs.append(out)
+    pre = uo.conv3(np.concatenate(xs, -1).astype(np.float64), uo.bf16_round(W).astype(np.float64))
+    if epi == 2:
+        want = np.maximum(pre + b, 0) @ proj[:16].astype(np.float64) + proj[16]
+        got = outs[0].cpu().numpy().reshape(nb, nz, ny, nx)
+    else:
+        want = pre if epi == 3 else np.maximum(pre + b, 0)
+        got = from_planar(outs[0].float().cpu().numpy().reshape(nb, nz, ny, 2, nx, 8))
+    scale = np.abs(want).max()
+    bar = 1e-3 * scale + (np.abs(want) * 2.0 ** -8 if epi == 0 else 0)
+    assert (np.abs(got - want) <= bar).all(), np.abs(got - want).max() / scale
+    if nx < 64:
+        assert torch.equal(outs[0], outs[1])
+
+
 def _net_and_params(hp, seed=3):
     net = hp.Unet(seed)
     p = net.get_params().astype(np.float64)
