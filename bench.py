@@ -400,7 +400,8 @@ def run_ours(args):
             return {"outer": info.outer_iters, "inner": info.inner_iters, "device_relres": info.relres}, launches
         return run
 
-    ELL, STENCIL = hp.SPMV_AUTO, hp.SPMV_STENCIL
+    # the baselines stream the stored ELL (12 bytes a slot), whatever form HPCCG_SPMV_AUTO would pick
+    ELL, STENCIL = hp.SPMV_ELL, hp.SPMV_STENCIL
     methods = [("fp64_cg", "plain FP64 CG (reference operation order), one CUDA graph", fp64_cg, ELL),
                ("fp32_ir", "FP64 iterative refinement, FP32 inner CG", mixed(hp.PREC_FP32), ELL),
                ("bf16_ir", "FP64 iterative refinement, inner CG on BF16 values / FP32 vectors", mixed(hp.PREC_BF16),

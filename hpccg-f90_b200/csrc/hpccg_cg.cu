@@ -428,7 +428,7 @@ extern "C" int hpccg_gpu_set_spmv(hpccg_ctx *c, int32_t kind, int32_t param) {
 extern "C" int hpccg_gpu_get_spmv(const hpccg_ctx *c, int32_t *kind, int32_t *param) {
   if (!c) return HPCCG_ERR_INVALID_ARG;
   const SpmvArgs a = spmv_args(c);
-  if (kind) *kind = a.kind;
+  if (kind) *kind = a.kind == kSpmvPattern ? HPCCG_SPMV_ELL : a.kind;  // the ELL in its pattern form
   if (param) *param = a.param;
   return HPCCG_OK;
 }
@@ -451,6 +451,20 @@ namespace hpccg {
 int autotune_spmv(hpccg_ctx *c) {
   if (c->spmv_tuned) return HPCCG_OK;
   c->spmv_tuned = true;
+  // Row patterns where the matrix has at most kPatLocal: a block then holds the
+  // table (432 bytes a pattern) in shared memory and a row costs 2 bytes of matrix
+  // instead of 324; any matrix with more falls back to the ELL.  Bit-identical,
+  // and found for less than the ELL candidates take to time.
+  if (c->d_ell_col && c->ell_width == kPatW && !c->pat_tried) {
+    c->pat_tried = true;
+    const int rc = row_patterns(c->d_ell_col, c->d_ell_val, c->npad, c->nrow, kPatLocal, c->num_sms, c->stream, &c->pat);
+    if (rc) return rc;
+  }
+  if (c->pat.count) {
+    c->spmv_kind = kSpmvPattern;
+    c->spmv_param = 4;
+    return HPCCG_OK;
+  }
   if (!c->d_ell_col || c->ell_width != 27) {
     c->spmv_kind = c->d_ell_col ? HPCCG_SPMV_ELL : HPCCG_SPMV_CSR_VECTOR;
     c->spmv_param = c->d_ell_col ? 4 : 32;

@@ -37,6 +37,24 @@ struct CgState {
   int pad[2];
 };
 
+// Row patterns of a stored matrix (hpccg_pattern.cuh): table entries and the table.
+struct __align__(16) PatEntry64 {
+  double v;
+  int32_t off, pad;  // column - row
+};
+struct __align__(8) PatEntry32 {
+  int32_t off;
+  float v;
+};
+struct RowPatterns {
+  int count = 0;             // 0: none (too many patterns, or not looked for)
+  uint16_t *code = nullptr;  // [npad] pattern of each row
+  PatEntry64 *t64 = nullptr; // [count][27]
+  PatEntry32 *t32 = nullptr, *t16 = nullptr;  // the same with values rounded to FP32 / BF16
+};
+// An SpMV kind that HPCCG_SPMV_AUTO resolves to (not offered by hpccg_gpu_set_spmv).
+constexpr int kSpmvPattern = 100;
+
 struct Reduction {
   double *partials;   // [kMaxPartials]
   unsigned *counter;  // arrival counter, reset by the last block
@@ -87,6 +105,9 @@ struct hpccg_ctx {
   // tensor maps of d_p and d_x for the FP64 TMA walk (tmaps_ok false: plain loads)
   CUtensorMap tmaps[2];
   bool tmaps_ok = false;
+  // row patterns of the ELL (looked for once, by HPCCG_SPMV_AUTO)
+  hpccg::RowPatterns pat;
+  bool pat_tried = false;
   // SpMV selection
   int spmv_kind = HPCCG_SPMV_AUTO;
   int spmv_param = 0;

@@ -43,7 +43,8 @@ struct MixedArgs {
   double *x, *r64;
   float *r, *p, *Ap, *d;
   const int32_t *ell_col;
-  const void *val_lp;
+  const void *val_lp;     // values, or the pattern table of the precision
+  const uint16_t *code;   // row patterns
   MixedState *st;
   Reduction red;
   StencilGeom geom;  // matrix-free inner SpMV when the context uses the stencil
@@ -301,7 +302,8 @@ template <class S, typename VT>
 __global__ void __launch_bounds__(kBlock, S::kMinBlocks) k_mp_spmv_dot(MixedArgs g) {
   __shared__ double smem[32];
   EpiDot32 epi{g.p, g.Ap};
-  const double part = S::rows(g.n, g.npad, g.ell_col, reinterpret_cast<const VT *>(g.val_lp), g.p, epi, g.geom, g.pm);
+  const double part = S::rows(g.n, g.npad, g.ell_col, reinterpret_cast<const VT *>(g.val_lp), g.p, epi, g.geom, g.pm,
+                              g.code);
   const double tot = block_sum<kBlock>(part, smem);
   if (arrive_last(g.red, tot)) {
     const double pAp = finish_sum<kBlock>(g.red, smem);
@@ -474,9 +476,10 @@ struct EpiStore32 {
 template <class S, typename VT>
 __global__ void __launch_bounds__(kBlock, S::kMinBlocks) k_spmv_lp(int n, int npad, const int32_t *col,
                                                                    const VT *val, const float *x, float *y,
-                                                                   StencilGeom geom, PlaneMap pm) {
+                                                                   StencilGeom geom, PlaneMap pm,
+                                                                   const uint16_t *code) {
   EpiStore32 epi{y};
-  S::rows(n, npad, col, val, x, epi, geom, pm);
+  S::rows(n, npad, col, val, x, epi, geom, pm, code);
 }
 
 __global__ void __launch_bounds__(kBlock) k_spmv_lp_tma(TmaTile t, const __grid_constant__ CUtensorMap map, float *y,
@@ -592,10 +595,11 @@ __global__ void k_to_lp(const double *src, float *f32, __nv_bfloat16 *b16, size_
 }
 
 // Low-precision strategy dispatch: the matrix-free stencil when the context
-// uses it, else value type by precision, RPT and MINB by param.
+// uses it, row patterns likewise, else value type by precision, RPT and MINB by param.
 template <class F>
-inline int dispatch_lp(bool stencil, int precision, int rpt, F &&f) {
-  if (stencil) return f(StratLpStencil{}, (float *)nullptr);
+inline int dispatch_lp(int kind, int precision, int rpt, F &&f) {
+  if (kind == HPCCG_SPMV_STENCIL) return f(StratLpStencil{}, (float *)nullptr);
+  if (kind == kSpmvPattern) return f(StratLpPattern{}, (PatEntry32 *)nullptr);
   if (precision == 1) {
     switch (rpt) {
       case 1: return f(StratLp<float, 1, 4>{}, (float *)nullptr);
@@ -623,7 +627,7 @@ struct MixedRes {
   MixedState *st = nullptr;
   cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
   int exec_rpt[3] = {0, 0, 0};
-  bool exec_stencil[3] = {false, false, false};
+  int exec_kind[3] = {0, 0, 0};
   int rpt[3] = {0, 2, 4};  // rows per thread per precision (index 1 = FP32, 2 = BF16)
   // matrix-free SpMV on p by TMA (when the context uses the stencil and nx % 4 == 0)
   CUtensorMap pmap;
@@ -672,12 +676,19 @@ __global__ void k_pad_vals27(const double *src, int W, int npad, double *dst) {
     for (int k = 0; k < 27; ++k) dst[(size_t)k * npad + i] = k < W ? src[(size_t)k * npad + i] : 0.0;
 }
 
+static bool uses_patterns(const hpccg_ctx *c) { return spmv_args(c).kind == kSpmvPattern; }
+// The low-precision values of the context's row kernel.
+static const void *lp_values(const hpccg_ctx *c, const MixedRes *m, int precision) {
+  if (uses_patterns(c)) return precision == 1 ? c->pat.t32 : c->pat.t16;
+  return precision == 1 ? (const void *)m->val32 : (const void *)m->val16;
+}
 static bool uses_stencil(const hpccg_ctx *c) { return spmv_args(c).kind == HPCCG_SPMV_STENCIL; }
 
 // Row map of the low-precision matrix-free SpMV: four columns per thread in one
 // wave of resident threads (StratLpStencil: 256 threads x 4 blocks per SM) when
 // nx allows it, else the context's plane map.
 static PlaneMap lp_map(const hpccg_ctx *c) {
+  if (uses_patterns(c)) return spmv_args(c).pm;  // rows of one walk share table reads
   // the FP32 one-column walk takes one line a thread
   const PlaneMap pm = c->gx ? plane_map(c->gx, c->gy, c->gz, kMaxPartials) : spmv_args(c).pm;
   if (!uses_stencil(c) || pm.plane <= 0) return pm;
@@ -703,7 +714,7 @@ static int mixed_res(hpccg_ctx *c, int precision, MixedRes **out) {
   const size_t slots = (size_t)27 * c->npad;
   const double *src = c->d_ell_val;
   double *tmp = nullptr;
-  if (!stencil &&
+  if (!stencil && !uses_patterns(c) &&
       ((precision == 1 && !m->val32) || (precision == 2 && !m->val16) || (!m->col27 && c->ell_width != 27))) {
     if (c->ell_width != 27) {
       HPCCG_CUDA(cudaMalloc(&tmp, sizeof(double) * slots));
@@ -780,7 +791,9 @@ static MixedArgs mixed_args(hpccg_ctx *c, MixedRes *m, int precision) {
   g.Ap = m->Ap;
   g.d = m->d;
   g.ell_col = m->col27 ? m->col27 : c->d_ell_col;
-  g.val_lp = precision == 1 ? (const void *)m->val32 : (const void *)m->val16;
+  g.val_lp = lp_values(c, m, precision);
+  g.code = c->pat.code;
+  if (uses_patterns(c)) g.npad = c->pat.count;
   g.st = m->st;
   g.red = reduction_of(c);
   g.geom = StencilGeom{c->gx, c->gy, c->gz};
@@ -808,7 +821,7 @@ static int launch_inner_body(hpccg_ctx *c, MixedRes *m, int precision, const Mix
     k_mp_update_r<<<c->grid, kBlock, 0, s>>>(g);
     return (int)cudaGetLastError();
   }
-  int rc = dispatch_lp(uses_stencil(c), precision, m->rpt[precision], [&](auto strat, auto *vt) {
+  int rc = dispatch_lp(spmv_args(c).kind, precision, m->rpt[precision], [&](auto strat, auto *vt) {
     using St = decltype(strat);
     using VT = std::remove_pointer_t<decltype(vt)>;
     k_mp_spmv_dot<St, VT><<<St::grid(g.pm, g.geom, c->grid), kBlock, 0, s>>>(g);
@@ -955,7 +968,7 @@ static int build_mixed_graph(hpccg_ctx *c, MixedRes *m, int precision) {
     return set_cuda_error(e, "build mixed graph", __FILE__, __LINE__);
   }
   m->exec_rpt[precision] = m->rpt[precision];
-  m->exec_stencil[precision] = uses_stencil(c);
+  m->exec_kind[precision] = spmv_args(c).kind;
   m->exec_fused[precision] = use_iter(c, m);
   return HPCCG_OK;
 }
@@ -1009,9 +1022,9 @@ extern "C" int hpccg_gpu_set_mixed_rows_per_thread(hpccg_ctx *c, int32_t precisi
 static int solve_mixed_common(hpccg_ctx *c, int precision, double rel_tol, int32_t max_outer,
                               int32_t max_inner, double inner_rtol, hpccg_mixed_info *info) {
   MixedRes *m = nullptr;
-  int rc = mixed_res(c, precision, &m);
+  int rc = autotune_spmv(c);  // settles the row kernel, and with it which values are copied
   if (rc) return rc;
-  if ((rc = autotune_spmv(c))) return rc;
+  if ((rc = mixed_res(c, precision, &m))) return rc;
   MixedState h0 = {};
   h0.rel_tol = rel_tol;
   h0.max_outer = max_outer;
@@ -1025,7 +1038,7 @@ static int solve_mixed_common(hpccg_ctx *c, int precision, double rel_tol, int32
     if ((rc = run_mixed_eager(c, m, precision))) return rc;
   } else {
     if (!m->exec[precision] || m->exec_rpt[precision] != m->rpt[precision] ||
-        m->exec_stencil[precision] != uses_stencil(c) || m->exec_fused[precision] != use_iter(c, m))
+        m->exec_kind[precision] != spmv_args(c).kind || m->exec_fused[precision] != use_iter(c, m))
       if ((rc = build_mixed_graph(c, m, precision))) return rc;
     HPCCG_CUDA(cudaGraphLaunch(m->exec[precision], c->stream));
   }
@@ -1096,13 +1109,14 @@ extern "C" int hpccg_gpu_spmv_lowp(hpccg_ctx *c, int32_t precision, const float 
     }
   }
   const int32_t *col = m->col27 ? m->col27 : c->d_ell_col;
-  const void *val = precision == 1 ? (const void *)m->val32 : (const void *)m->val16;
-  rc = dispatch_lp(uses_stencil(c), precision, m->rpt[precision], [&](auto strat, auto *vt) {
+  const void *val = lp_values(c, m, precision);
+  rc = dispatch_lp(spmv_args(c).kind, precision, m->rpt[precision], [&](auto strat, auto *vt) {
     using St = decltype(strat);
     using VT = std::remove_pointer_t<decltype(vt)>;
     const PlaneMap pm = lp_map(c);
-    k_spmv_lp<St, VT><<<St::grid(pm, StencilGeom{c->gx, c->gy, c->gz}, c->grid), kBlock, 0, c->stream>>>(c->nrow, c->npad, col, (const VT *)val, d_x,
-                                                                        d_y, StencilGeom{c->gx, c->gy, c->gz}, pm);
+    k_spmv_lp<St, VT><<<St::grid(pm, StencilGeom{c->gx, c->gy, c->gz}, c->grid), kBlock, 0, c->stream>>>(c->nrow, uses_patterns(c) ? c->pat.count : c->npad, col, (const VT *)val, d_x,
+                                                                        d_y, StencilGeom{c->gx, c->gy, c->gz}, pm,
+                                                                        c->pat.code);
     return (int)cudaGetLastError();
   });
   if (rc) return set_cuda_error((cudaError_t)rc, "spmv_lowp", __FILE__, __LINE__);
@@ -1167,7 +1181,7 @@ extern "C" int hpccg_gpu_time_mixed_kernels(hpccg_ctx *c, int32_t precision, int
       } else if (which == 1 && use_tma(c, m)) {
         k_mp_spmv_dot_tma<<<tma_tile_grid(m->tile), kBlock, kTmaRingBytes, c->stream>>>(g, m->tile, m->pmap);
       } else if (which == 1) {
-        dispatch_lp(uses_stencil(c), precision, m->rpt[precision], [&](auto strat, auto *vt) {
+        dispatch_lp(spmv_args(c).kind, precision, m->rpt[precision], [&](auto strat, auto *vt) {
           using St = decltype(strat);
           using VT = std::remove_pointer_t<decltype(vt)>;
           k_mp_spmv_dot<St, VT><<<St::grid(g.pm, g.geom, c->grid), kBlock, 0, c->stream>>>(g);

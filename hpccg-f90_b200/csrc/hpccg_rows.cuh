@@ -14,11 +14,14 @@
 //    keeps x.
 //  * csr_vector_rows<LPR>: LPR lanes per CSR row (LPR = 32 is warp-per-row),
 //    lane-strided loads, butterfly shuffle reduction.  Reassociates the sum.
+//  * StratPatternWalk / Stride (hpccg_pattern.cuh): the ELL as row patterns, for a matrix that
+//    has few; the ELL kernel's rows, terms and order, so bit-identical to it.
 //  * stencil_rows (hpccg_stencil.cuh): matrix-free, for a context whose CSR
 //    was checked equal to generate_matrix(nx,ny,nz); bit-identical to ELL
 //    (both follow the same plane map of rows to threads).
 #pragma once
 #include "hpccg_internal.cuh"
+#include "hpccg_pattern.cuh"
 #include "hpccg_stencil.cuh"
 #include "hpccg_stencil_tma64.cuh"
 
@@ -195,11 +198,14 @@ struct EpiResidual {  // r = 1*b + (-1)*(A x), contribution r_i^2
 
 // Arguments every row strategy may need.
 struct SpmvArgs {
-  int kind;   // HPCCG_SPMV_ELL / ELL2 / CSR_VECTOR / STENCIL
+  int kind;   // HPCCG_SPMV_ELL / ELL2 / CSR_VECTOR / STENCIL, or kSpmvPattern
   int param;  // lanes per row for CSR_VECTOR
   int n, npad, W;
   const int32_t *rowptr, *col, *ell_col;
   const double *val, *ell_val;
+  const uint16_t *pat_code;   // row patterns
+  const PatEntry64 *pat;
+  int pat_count;
   StencilGeom geom;  // grid of generate_matrix (STENCIL only)
   PlaneMap pm;       // row map of ELL (one row per thread) and STENCIL when the grid is known
   // STENCIL under the tile map: tensor maps of the two vectors tma_vec[0..1],
@@ -230,6 +236,35 @@ struct StratEll1 {
   template <class Epi>
   static __device__ __forceinline__ double rows(const SpmvArgs &a, const double *x, Epi &e) {
     return ell_rows<27, 1, 27>(a.n, a.npad, a.ell_col, a.ell_val, x, e, a.pm);
+  }
+};
+// Row patterns: 2 bytes per row instead of 12 per slot, so the x gathers bound it
+// (a misaligned 256-byte L1 read costs 4 to 5 cycles, 27 of them per 32 rows) and
+// not HBM.  FP64 SpMV + dot: on a known grid, walking it with four rows to a table
+// read, 117 -> 38 us at 128^3 (four rows from global memory 41, two 46, one
+// table read per row 67; more or fewer blocks per SM slower); without a grid one
+// row at a time at full occupancy, 26.7 -> 14.7 us at 97 x 75 x 61 (two rows and
+// half the occupancy: 17.1).
+struct StratPatternWalk {  // the grid is known
+  static constexpr int kMinBlocks = 4;
+  static int grid(const SpmvArgs &a, int) { return plane_grid(a.pm); }
+  template <class Epi>
+  static __device__ __forceinline__ double rows(const SpmvArgs &a, const double *x, Epi &e) {
+    double part = 0.0;
+    pattern_walk(a.n, a.pm, a.pat_code, a.pat, a.pat_count, x,
+                 [&](int i, double s) { part = __dadd_rn(part, e(i, s)); });
+    return part;
+  }
+};
+struct StratPatternStride {
+  static constexpr int kMinBlocks = 8;
+  static int grid(const SpmvArgs &, int dflt) { return dflt; }
+  template <class Epi>
+  static __device__ __forceinline__ double rows(const SpmvArgs &a, const double *x, Epi &e) {
+    double part = 0.0;
+    pattern_stride(a.n, a.pat_code, a.pat, a.pat_count, x,
+                   [&](int i, double s) { part = __dadd_rn(part, e(i, s)); });
+    return part;
   }
 };
 template <int MINB>
@@ -301,6 +336,7 @@ inline int dispatch_strategy(const SpmvArgs &a, F &&f, const double *x = nullptr
     if (x && a.tma_ok && a.pm.tiles_x > 0 && (x == a.tma_vec[0] || x == a.tma_vec[1])) return f(StratStencilTma{});
     return f(StratStencil{});
   }
+  if (a.kind == kSpmvPattern) return a.pm.plane > 0 ? f(StratPatternWalk{}) : f(StratPatternStride{});
   if (a.kind == HPCCG_SPMV_CSR_VECTOR) {
     switch (a.param) {
       case 4: return f(StratCsr<4>{});
@@ -345,6 +381,7 @@ inline SpmvArgs spmv_args(const hpccg_ctx *c) {
   a.kind = c->spmv_kind == HPCCG_SPMV_AUTO ? HPCCG_SPMV_ELL : c->spmv_kind;
   a.param = c->spmv_kind == HPCCG_SPMV_AUTO ? 4 : c->spmv_param;
   if (a.kind == HPCCG_SPMV_STENCIL && !c->gx) a.kind = HPCCG_SPMV_ELL;
+  if (a.kind == kSpmvPattern && !c->pat.count) a.kind = HPCCG_SPMV_ELL;
   if (!c->d_ell_col && a.kind != HPCCG_SPMV_CSR_VECTOR && a.kind != HPCCG_SPMV_STENCIL) {
     a.kind = HPCCG_SPMV_CSR_VECTOR;
     a.param = 32;
@@ -357,6 +394,9 @@ inline SpmvArgs spmv_args(const hpccg_ctx *c) {
   a.val = c->d_val;
   a.ell_col = c->d_ell_col;
   a.ell_val = c->d_ell_val;
+  a.pat_code = c->pat.code;
+  a.pat = c->pat.t64;
+  a.pat_count = c->pat.count;
   a.geom = StencilGeom{c->gx, c->gy, c->gz};
   a.pm = c->gx ? fp64_map(c->gx, c->gy, c->gz, c->num_sms) : PlaneMap{0, 0, 0, 1, 1, 0};
   a.tma_ok = a.pm.tiles_x > 0 && c->tmaps_ok;

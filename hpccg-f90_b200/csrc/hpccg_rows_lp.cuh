@@ -5,6 +5,7 @@
 // 32*RPT*sizeof(value) load plus a 32*RPT*4-byte column-index load.
 #pragma once
 #include "hpccg_internal.cuh"
+#include "hpccg_pattern.cuh"
 #include "hpccg_stencil.cuh"
 
 namespace hpccg {
@@ -114,7 +115,8 @@ struct StratLp {
   static int grid(const PlaneMap &, const StencilGeom &, int dflt) { return dflt; }
   template <class Epi>
   static __device__ __forceinline__ double rows(int n, int npad, const int32_t *col, const VT *val,
-                                                const float *x, Epi &e, const StencilGeom &, const PlaneMap &) {
+                                                const float *x, Epi &e, const StencilGeom &, const PlaneMap &,
+                                                const uint16_t *) {
     return ell_rows_lp<VT, RPT, 27>(n, npad, col, val, x, e);
   }
 };
@@ -129,9 +131,26 @@ struct StratLpStencil {
   static int grid(const PlaneMap &m, const StencilGeom &, int dflt) { return m.plane > 0 ? plane_grid(m) : dflt; }
   template <class Epi>
   static __device__ __forceinline__ double rows(int n, int, const int32_t *, const float *, const float *x,
-                                                Epi &e, const StencilGeom &g, const PlaneMap &m) {
+                                                Epi &e, const StencilGeom &g, const PlaneMap &m, const uint16_t *) {
     if (m.cols == 4) return stencil_rows_boxw<4>(g, m, x, e);
     return m.plane > 0 ? stencil_rows_box(g, m, x, e) : stencil_rows<float>(n, g, m, x, e);
+  }
+};
+
+// Row patterns (hpccg_pattern.cuh), `table` the table of the wanted precision: one
+// row per thread, so that a warp's gathers are contiguous, at full occupancy.
+// BF16 values at 150 x 131 x 97: 58.7 -> 25.8 us (walking the grid: 29.1).
+struct StratLpPattern {
+  static constexpr int kMinBlocks = 8;
+  static int grid(const PlaneMap &, const StencilGeom &, int dflt) { return dflt; }
+  // npad: the number of patterns
+  template <class Epi>
+  static __device__ __forceinline__ double rows(int n, int npad, const int32_t *, const PatEntry32 *table,
+                                                const float *x, Epi &e, const StencilGeom &, const PlaneMap &,
+                                                const uint16_t *code) {
+    double part = 0.0;
+    pattern_stride(n, code, table, npad, x, [&](int r, float s) { part += e(r, s); });
+    return part;
   }
 };
 

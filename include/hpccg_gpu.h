@@ -78,8 +78,10 @@ int hpccg_gpu_download_csr(const hpccg_ctx *ctx, int32_t *rowindex, int32_t *col
                            double *values);
 
 /* SpMV kernel selection.  HPCCG_SPMV_AUTO picks the fastest bit-exact FP64
- * ELL kernel on first use (never the matrix-free stencil, which is opt-in);
- * the others force one kernel. */
+ * kernel on the stored matrix on first use (never the matrix-free stencil,
+ * which is opt-in): the ELL as row patterns where the matrix has few distinct
+ * rows (get_spmv then reports HPCCG_SPMV_ELL), else an ELL kernel; the others
+ * force one kernel. */
 #define HPCCG_SPMV_AUTO 0
 #define HPCCG_SPMV_ELL 1        /* thread per row, column-major ELL (param: resident blocks/SM hint 2,3,4,8) */
 #define HPCCG_SPMV_ELL2 2       /* two rows per thread, 16-byte loads (same param)  */

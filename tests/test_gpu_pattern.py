@@ -1,0 +1,79 @@
+"""Row patterns of a stored matrix (HPCCG_SPMV_AUTO) against the ELL kernels.
+
+The pattern form adds the same terms in the same order, so FP64 products, fused
+dots and CG runs, and the low-precision products, must equal the explicit ELL
+kernel's bit for bit (the low-precision ELL kernel sums in the same order too).
+"""
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def env():
+    import torch
+
+    import hpccg_b200 as hp
+    return torch, hp
+
+
+def _products(torch, hp, M, kind, x):
+    """FP64 and low-precision products and a CG run with one row kernel."""
+    M.set_spmv(kind)
+    n = M.nrow
+    dx = torch.from_numpy(x).cuda()
+    y = torch.full((n,), 7.0, dtype=torch.float64, device="cuda")
+    M.spmv(dx, y)
+    out = [y.cpu().numpy()]
+    xf = dx.float()
+    for prec in (hp.PREC_FP32, hp.PREC_BF16):
+        yf = torch.full((n,), 7.0, dtype=torch.float32, device="cuda")
+        M.spmv_lowp(prec, xf, yf)
+        out.append(yf.cpu().numpy())
+    return out
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(3, 3, 3), (5, 4, 7), (32, 16, 9), (33, 17, 5), (34, 6, 33), (64, 18, 20), (97, 3, 40)])
+@pytest.mark.parametrize("known_grid", [False, True])
+def test_patterns_equal_ell_on_grids(env, nx, ny, nz, known_grid):
+    torch, hp = env
+    A, x0, b, _ = oracle.generate_matrix(nx, ny, nz)
+    M = hp.Matrix.generated(nx, ny, nz) if known_grid else hp.Matrix.from_csr(A.rowindex, A.colindex, A.values)
+    x = np.random.default_rng(nx).uniform(-1, 1, A.nrow)
+    got, want = _products(torch, hp, M, hp.SPMV_AUTO, x), _products(torch, hp, M, hp.SPMV_ELL, x)
+    assert np.array_equal(want[0], oracle.spmv(A, x))
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
+
+
+def _mixed_rows(rng, n, npat):
+    """A CSR of n rows with npat patterns of up to 27 entries (one of them full)."""
+    pats = []
+    for k in range(npat):
+        w = 27 if k < 3 else int(rng.integers(0, 28))
+        lo, hi = ((0, 41) if k == 0 else (-40, 1) if k == 1 else (-40, 41))
+        off = np.sort(rng.choice(np.arange(lo, hi), w, replace=False))
+        val = rng.choice([0.0, -0.0, 1.5, -2.0, 1e300, 5e-324, 0.1], w) + 0.0 * off
+        pats.append((off, val))
+    which = rng.integers(0, npat, n)
+    which[:40], which[-40:] = 0, 1  # columns stay inside
+    cols = [pats[p][0] + i + 1 for i, p in enumerate(which)]
+    rowindex = np.concatenate([[1], 1 + np.cumsum([len(c) for c in cols])]).astype(np.int32)
+    return rowindex, np.concatenate(cols).astype(np.int32), np.concatenate([pats[p][1] for p in which])
+
+
+@pytest.mark.parametrize("n,npat", [(100, 3), (1000, 32), (5001, 31), (5001, 33), (20000, 400)])
+def test_patterns_of_other_matrices(env, n, npat):
+    """Matrices that are no stencil, up to and beyond the number of patterns kept
+    (more: the ELL kernels run); infinities reach the same rows as in the ELL."""
+    torch, hp = env
+    rng = np.random.default_rng(n + npat)
+    M = hp.Matrix.from_csr(*_mixed_rows(rng, n, npat))
+    x = rng.uniform(-1, 1, n)
+    x[n // 2] = np.inf
+    got, want = _products(torch, hp, M, hp.SPMV_AUTO, x), _products(torch, hp, M, hp.SPMV_ELL, x)
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w, equal_nan=True)
