@@ -15,6 +15,7 @@
 
 #include <algorithm>
 
+#include "hpccg_persist.cuh"
 #include "hpccg_rows.cuh"
 
 namespace hpccg {
@@ -354,6 +355,10 @@ static int cg_common(hpccg_ctx *c, int32_t max_iter, double tolerance, int32_t *
   if (eager) {
     HPCCG_CUDA(cudaEventRecord(c->solve0, c->stream));
     if ((rc = run_cg_eager(c))) return rc;
+    HPCCG_CUDA(cudaEventRecord(c->solve1, c->stream));
+  } else if (cg_persist_fits(c)) {
+    HPCCG_CUDA(cudaEventRecord(c->solve0, c->stream));
+    if ((rc = cg_persist(c))) return rc;
     HPCCG_CUDA(cudaEventRecord(c->solve1, c->stream));
   } else {
     const SpmvArgs a = spmv_args(c);

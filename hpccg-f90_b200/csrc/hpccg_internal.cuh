@@ -93,6 +93,9 @@ struct hpccg_ctx {
   double *d_ell_val = nullptr;
   // CG work vectors and staging
   double *d_r = nullptr, *d_p = nullptr, *d_Ap = nullptr, *d_x = nullptr, *d_b = nullptr;
+  // second p and the barrier slots of the one-kernel CG (allocated on its first solve)
+  double *d_p2 = nullptr;
+  void *d_slots = nullptr;
   // scratch
   double *d_partials = nullptr;
   unsigned *d_counter = nullptr;

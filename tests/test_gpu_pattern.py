@@ -1,5 +1,8 @@
 """Row patterns of a stored matrix (HPCCG_SPMV_AUTO) against the ELL kernels.
 
+The CG of small systems in one kernel is compared with the graph of the explicit
+ELL kernel: the rows are the same, the dot products associated differently.
+
 The pattern form adds the same terms in the same order, so FP64 products, fused
 dots and CG runs, and the low-precision products, must equal the explicit ELL
 kernel's bit for bit (the low-precision ELL kernel sums in the same order too).
@@ -77,3 +80,31 @@ def test_patterns_of_other_matrices(env, n, npat):
     got, want = _products(torch, hp, M, hp.SPMV_AUTO, x), _products(torch, hp, M, hp.SPMV_ELL, x)
     for g, w in zip(got, want):
         assert np.array_equal(g, w, equal_nan=True)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(3, 3, 3), (4, 4, 16), (16, 16, 17), (37, 32, 32), (19, 31, 65), (37, 64, 32),
+                                      (43, 43, 41), (101, 101, 102), (102, 102, 101)])
+def test_one_kernel_cg(env, nx, ny, nz):
+    """Row counts around one row a thread in blocks of 256 and 512, several rows a
+    thread, and the largest system of the one-kernel form (and one beyond it).
+    FP64 dots of n terms differ by n 2^-53 of their terms at most; the bars are the
+    history bars of the CG tests (1e-12 of the residual, of the first one once it
+    has fallen by 1e8) and 1e-10 for x."""
+    torch, hp = env
+    M = hp.Matrix.generated(nx, ny, nz)
+    n = M.nrow
+    xs = torch.from_numpy(np.random.default_rng(n).uniform(-1, 1, n)).cuda()
+    b = torch.empty_like(xs)
+    M.spmv(xs, b)
+    for max_iter, tol in ((0, 0.0), (1, 0.0), (12, 0.0), (200, 1e-9)):
+        runs = []
+        for kind in (hp.SPMV_AUTO, hp.SPMV_ELL):
+            M.set_spmv(kind)
+            x = torch.full_like(b, 0.25)
+            it, normr, hist, st = M.cg_device(b, x, max_iter, tol * float(torch.linalg.vector_norm(b)))
+            runs.append((it, normr, hist, st, x.cpu().numpy()))
+        (i0, n0, h0, s0, x0), (i1, n1, h1, s1, x1) = runs
+        assert (i0, s0) == (i1, s1)
+        band = np.where(h1 >= 1e-8 * h1[0], h1, h1[0]) * 1e-12
+        assert (np.abs(h0 - h1) <= band).all() and abs(n0 - n1) <= band[-1]
+        assert np.abs(x0 - x1).max() <= 1e-10
