@@ -186,3 +186,29 @@ def test_batch_stencil_bit_identical_to_ell(hp, torch):
     with pytest.raises(hp.HpccgError) as e:
         Bc.set_spmv(hp.SPMV_STENCIL)
     assert e.value.code == hp.HPCCG_ERR_UNSUPPORTED
+
+
+EDGES = [(33, 17, 5), (32, 16, 16), (31, 15, 17), (64, 18, 33), (5, 3, 2), (96, 1, 4), (1, 40, 9), (34, 33, 1), (8, 8, 40)]
+
+
+@pytest.mark.parametrize("sizes", [EDGES, EDGES + SIZES + EDGES[::-1], [(1, 1, 300), (2, 1, 50)], [(40, 40, 40)]])
+@pytest.mark.parametrize("prec", [FP32, FP64])
+def test_batch_matrix_free_shapes(hp, torch, sizes, prec):
+    """Partial tiles, pieces and z chunks; few systems and many (they decide in
+    different places); shapes the tiles do not suit.  Every system meets the
+    target by the oracle's FP64 true residual, from a start that is not 0."""
+    B = hp.Batch.generated(np.array(sizes))
+    B.set_spmv(hp.SPMV_STENCIL)
+    rng = np.random.default_rng(len(sizes))
+    bs = [rng.uniform(-1, 1, nx * ny * nz) for nx, ny, nz in sizes]
+    x0 = [rng.uniform(-1, 1, b.size) for b in bs]
+    db = torch.from_numpy(B.stack(bs)).cuda()
+    dx = torch.from_numpy(B.stack(x0)).cuda()
+    iters, relres, outer, status = B.solve(db, dx, prec, 1e-9, 500)
+    assert status == hp.HPCCG_OK
+    for (nx, ny, nz), b, x, rr in zip(sizes, bs, B.unstack(dx.cpu().numpy()), relres):
+        true = oracle.grid_true_relres(nx, ny, nz, b, x)
+        assert true <= 1e-9 * (1 + 1e-6) and rr == pytest.approx(true, rel=1e-6)
+    again = torch.from_numpy(B.stack(x0)).cuda()
+    B.solve(db, again, prec, 1e-9, 500)
+    assert torch.equal(again, dx)
