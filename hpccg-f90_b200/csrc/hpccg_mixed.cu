@@ -51,13 +51,16 @@ struct MixedArgs {
   PlaneMap pm;
   cudaGraphConditionalHandle cond_outer, cond_inner;
   int use_cond;
-  int skip_done;  // fused pass: return at once when the inner solve has ended
+  int skip_done;  // inner-loop kernels: return at once when the inner solve has ended
 };
 
 __device__ __forceinline__ void set_outer(const MixedArgs &g, int v) {
   g.st->cont_outer = v;
   if (g.use_cond) cudaGraphSetConditional(g.cond_outer, (unsigned)v);
 }
+// Whether a kernel of an unrolled loop body comes after the inner solve's end
+// (cont_inner is cleared by the last block of a pass only, after every block has read it).
+__device__ __forceinline__ bool inner_done(const MixedArgs &g) { return g.skip_done && !g.st->cont_inner; }
 __device__ __forceinline__ void set_inner(const MixedArgs &g, int v) {
   g.st->cont_inner = v;
   if (g.use_cond) cudaGraphSetConditional(g.cond_inner, (unsigned)v);
@@ -240,6 +243,7 @@ __global__ void __launch_bounds__(kBlock) k_mp_start_inner(MixedArgs g) {
 
 // p = r (first) or d += alpha p (deferred), p = r + beta p.
 __global__ void __launch_bounds__(kBlock) k_mp_update_p(MixedArgs g) {
+  if (inner_done(g)) return;
   const MixedState *st = g.st;
   const int n4 = g.n >> 2;
   const int stride = gridDim.x * blockDim.x;
@@ -301,6 +305,7 @@ struct EpiDot32 {
 template <class S, typename VT>
 __global__ void __launch_bounds__(kBlock, S::kMinBlocks) k_mp_spmv_dot(MixedArgs g) {
   __shared__ double smem[32];
+  if (inner_done(g)) return;
   EpiDot32 epi{g.p, g.Ap};
   const double part = S::rows(g.n, g.npad, g.ell_col, reinterpret_cast<const VT *>(g.val_lp), g.p, epi, g.geom, g.pm,
                               g.code);
@@ -325,6 +330,7 @@ __global__ void __launch_bounds__(kBlock, S::kMinBlocks) k_mp_spmv_dot(MixedArgs
 __global__ void __launch_bounds__(kBlock) k_mp_spmv_dot_tma(MixedArgs g, TmaTile t,
                                                             const __grid_constant__ CUtensorMap map) {
   __shared__ double smem[32];
+  if (inner_done(g)) return;
   EpiDot32 epi{g.p, g.Ap};
   const double part = stencil_rows_tma(t, &map, epi, &g.st->status);
   const double tot = block_sum<kBlock>(part, smem);
@@ -347,6 +353,7 @@ __global__ void __launch_bounds__(kBlock) k_mp_spmv_dot_tma(MixedArgs g, TmaTile
 // r -= alpha Ap, rr, inner stop test.
 __global__ void __launch_bounds__(kBlock) k_mp_update_r(MixedArgs g) {
   __shared__ double smem[32];
+  if (inner_done(g)) return;
   if (g.st->inner_break) {
     if (blockIdx.x == 0 && threadIdx.x == 0) set_inner(g, 0);
     return;
@@ -416,9 +423,7 @@ __global__ void __launch_bounds__(kItBlock, 1) k_mp_iter_tma(MixedArgs g, TmaTil
                                                           const __grid_constant__ CUtensorMap dm) {
   __shared__ double smem[4 * 32];
   MixedState *st = g.st;
-  // a pass of an unrolled loop body after the inner solve has ended does nothing
-  // (cont_inner changes only in the last block of a pass, after every block has read it)
-  if (g.skip_done && !st->cont_inner) return;
+  if (inner_done(g)) return;
   const int par = st->passes & 1;
   const bool first = st->passes == 0;
   IterScalars sc;
@@ -801,18 +806,17 @@ static MixedArgs mixed_args(hpccg_ctx *c, MixedRes *m, int precision) {
   return g;
 }
 
-// Fused passes per inner-loop body: the while node's per-iteration cost is paid
-// once per kInnerUnroll passes; passes after the solve has ended return at once.
+// Iterations per inner-loop body: the while node's per-iteration cost is paid once
+// per kInnerUnroll of them; kernels after the solve has ended return at once.
 #ifndef HPCCG_INNER_UNROLL
 #define HPCCG_INNER_UNROLL 4
 #endif
 constexpr int kInnerUnroll = HPCCG_INNER_UNROLL;
 
-static int launch_inner_body(hpccg_ctx *c, MixedRes *m, int precision, const MixedArgs &g, cudaStream_t s) {
+// One iteration of the inner CG: the fused pass, or p update, SpMV + dot, r update.
+static int launch_inner_iteration(hpccg_ctx *c, MixedRes *m, int precision, const MixedArgs &g, cudaStream_t s) {
   if (use_iter(c, m)) {
-    MixedArgs gs = g;
-    gs.skip_done = 1;
-    for (int k = 0; k < kInnerUnroll; ++k) launch_iter(c, m, k ? gs : g, s);
+    launch_iter(c, m, g, s);
     return (int)cudaGetLastError();
   }
   k_mp_update_p<<<c->grid, kBlock, 0, s>>>(g);
@@ -830,6 +834,14 @@ static int launch_inner_body(hpccg_ctx *c, MixedRes *m, int precision, const Mix
   if (rc) return rc;
   k_mp_update_r<<<c->grid, kBlock, 0, s>>>(g);
   return (int)cudaGetLastError();
+}
+
+static int launch_inner_body(hpccg_ctx *c, MixedRes *m, int precision, const MixedArgs &g, cudaStream_t s) {
+  MixedArgs gs = g;
+  gs.skip_done = 1;
+  for (int k = 0; k < kInnerUnroll; ++k)
+    if (const int rc = launch_inner_iteration(c, m, precision, k ? gs : g, s)) return rc;
+  return 0;
 }
 
 // The refinement residual of the fused iteration (FIRST: also b.b).
