@@ -474,6 +474,10 @@ int autotune_spmv(hpccg_ctx *c) {
     if (rc) return rc;
   }
   if (c->pat.count) {
+    if (c->gx && (c->pat.box_nx != c->gx || c->pat.box_ny != c->gy)) {
+      const int rc = pattern_boxes(&c->pat, c->gx, c->gy, c->stream);
+      if (rc) return rc;
+    }
     c->spmv_kind = kSpmvPattern;
     c->spmv_param = 4;
     return HPCCG_OK;

@@ -47,10 +47,17 @@ struct __align__(8) PatEntry32 {
   float v;
 };
 struct RowPatterns {
+  void *memory = nullptr;    // one allocation holds everything below
   int count = 0;             // 0: none (too many patterns, or not looked for)
   uint16_t *code = nullptr;  // [npad] pattern of each row
   PatEntry64 *t64 = nullptr; // [count][27]
   PatEntry32 *t32 = nullptr, *t16 = nullptr;  // the same with values rounded to FP32 / BF16
+  // the values at the 27 neighbours of a grid point, zeros where a row has none (pattern_boxes)
+  double *box64 = nullptr;  // [count][27]
+  float *box32 = nullptr, *box16 = nullptr;
+  int box_nx = 0, box_ny = 0;  // the grid they were made for
+  bool boxes = false;          // they hold every pattern
+  int *flag = nullptr;
 };
 // An SpMV kind that HPCCG_SPMV_AUTO resolves to (not offered by hpccg_gpu_set_spmv).
 constexpr int kSpmvPattern = 100;

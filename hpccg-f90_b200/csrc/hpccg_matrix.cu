@@ -354,7 +354,7 @@ __global__ void check_stencil_kernel(int32_t n, int nx, int ny, int nz, const in
 extern "C" int hpccg_gpu_set_geometry(hpccg_ctx *c, int32_t nx, int32_t ny, int32_t nz) {
   if (!c || nx < 1 || ny < 1 || nz < 1 || (int64_t)nx * ny * nz != (int64_t)c->nrow) return HPCCG_ERR_INVALID_ARG;
   c->gx = c->gy = c->gz = 0;
-  if (c->spmv_kind == HPCCG_SPMV_STENCIL) {
+  if (c->spmv_kind == HPCCG_SPMV_STENCIL || c->spmv_kind == kSpmvPattern) {  // AUTO looks at the new grid
     c->spmv_kind = HPCCG_SPMV_AUTO;
     c->spmv_tuned = false;
   }

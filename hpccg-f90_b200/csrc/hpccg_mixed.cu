@@ -602,8 +602,10 @@ __global__ void k_to_lp(const double *src, float *f32, __nv_bfloat16 *b16, size_
 // Low-precision strategy dispatch: the matrix-free stencil when the context
 // uses it, row patterns likewise, else value type by precision, RPT and MINB by param.
 template <class F>
-inline int dispatch_lp(int kind, int precision, int rpt, F &&f) {
+inline int dispatch_lp(const SpmvArgs &a, int precision, int rpt, F &&f) {
+  const int kind = a.kind;
   if (kind == HPCCG_SPMV_STENCIL) return f(StratLpStencil{}, (float *)nullptr);
+  if (kind == kSpmvPattern && a.pat_box) return f(StratLpBox{}, (float *)nullptr);
   if (kind == kSpmvPattern) return f(StratLpPattern{}, (PatEntry32 *)nullptr);
   if (precision == 1) {
     switch (rpt) {
@@ -684,6 +686,7 @@ __global__ void k_pad_vals27(const double *src, int W, int npad, double *dst) {
 static bool uses_patterns(const hpccg_ctx *c) { return spmv_args(c).kind == kSpmvPattern; }
 // The low-precision values of the context's row kernel.
 static const void *lp_values(const hpccg_ctx *c, const MixedRes *m, int precision) {
+  if (uses_patterns(c) && spmv_args(c).pat_box) return precision == 1 ? c->pat.box32 : c->pat.box16;
   if (uses_patterns(c)) return precision == 1 ? c->pat.t32 : c->pat.t16;
   return precision == 1 ? (const void *)m->val32 : (const void *)m->val16;
 }
@@ -693,7 +696,7 @@ static bool uses_stencil(const hpccg_ctx *c) { return spmv_args(c).kind == HPCCG
 // wave of resident threads (StratLpStencil: 256 threads x 4 blocks per SM) when
 // nx allows it, else the context's plane map.
 static PlaneMap lp_map(const hpccg_ctx *c) {
-  if (uses_patterns(c)) return spmv_args(c).pm;  // rows of one walk share table reads
+  if (uses_patterns(c)) return spmv_args(c).pm;
   // the FP32 one-column walk takes one line a thread
   const PlaneMap pm = c->gx ? plane_map(c->gx, c->gy, c->gz, kMaxPartials) : spmv_args(c).pm;
   if (!uses_stencil(c) || pm.plane <= 0) return pm;
@@ -825,7 +828,7 @@ static int launch_inner_iteration(hpccg_ctx *c, MixedRes *m, int precision, cons
     k_mp_update_r<<<c->grid, kBlock, 0, s>>>(g);
     return (int)cudaGetLastError();
   }
-  int rc = dispatch_lp(spmv_args(c).kind, precision, m->rpt[precision], [&](auto strat, auto *vt) {
+  int rc = dispatch_lp(spmv_args(c), precision, m->rpt[precision], [&](auto strat, auto *vt) {
     using St = decltype(strat);
     using VT = std::remove_pointer_t<decltype(vt)>;
     k_mp_spmv_dot<St, VT><<<St::grid(g.pm, g.geom, c->grid), kBlock, 0, s>>>(g);
@@ -1122,7 +1125,7 @@ extern "C" int hpccg_gpu_spmv_lowp(hpccg_ctx *c, int32_t precision, const float 
   }
   const int32_t *col = m->col27 ? m->col27 : c->d_ell_col;
   const void *val = lp_values(c, m, precision);
-  rc = dispatch_lp(spmv_args(c).kind, precision, m->rpt[precision], [&](auto strat, auto *vt) {
+  rc = dispatch_lp(spmv_args(c), precision, m->rpt[precision], [&](auto strat, auto *vt) {
     using St = decltype(strat);
     using VT = std::remove_pointer_t<decltype(vt)>;
     const PlaneMap pm = lp_map(c);
@@ -1193,7 +1196,7 @@ extern "C" int hpccg_gpu_time_mixed_kernels(hpccg_ctx *c, int32_t precision, int
       } else if (which == 1 && use_tma(c, m)) {
         k_mp_spmv_dot_tma<<<tma_tile_grid(m->tile), kBlock, kTmaRingBytes, c->stream>>>(g, m->tile, m->pmap);
       } else if (which == 1) {
-        dispatch_lp(spmv_args(c).kind, precision, m->rpt[precision], [&](auto strat, auto *vt) {
+        dispatch_lp(spmv_args(c), precision, m->rpt[precision], [&](auto strat, auto *vt) {
           using St = decltype(strat);
           using VT = std::remove_pointer_t<decltype(vt)>;
           k_mp_spmv_dot<St, VT><<<St::grid(g.pm, g.geom, c->grid), kBlock, 0, c->stream>>>(g);

@@ -99,9 +99,7 @@ __global__ void k_pat_assign(const int32_t *col, const double *val, int npad, in
 }
 
 void free_patterns(RowPatterns *p) {
-  void *bufs[] = {p->code, p->t64, p->t32, p->t16};
-  for (void *b : bufs)
-    if (b) cudaFree(b);
+  if (p->memory) cudaFree(p->memory);
   *p = RowPatterns{};
 }
 
@@ -110,8 +108,30 @@ int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n,
   free_patterns(out);
   if (n < 1 || max_count < 1) return HPCCG_OK;
   max_count = std::min(max_count, kPatMax);
-  PatTable *t = nullptr;
-  HPCCG_CUDA(cudaMalloc(&t, sizeof(PatTable)));
+  // one allocation (each costs a synchronisation when it is freed): the search's
+  // table, the tables, the codes
+  const size_t most = (size_t)max_count * kPatW;
+  size_t bytes = 0;
+  auto part = [&](size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  };
+  const size_t at_t = part(sizeof(PatTable)), at64 = part(sizeof(PatEntry64) * most), at32 = part(sizeof(PatEntry32) * most),
+               at16 = part(sizeof(PatEntry32) * most), b64 = part(sizeof(double) * most),
+               b32 = part(sizeof(float) * most), b16 = part(sizeof(float) * most), atf = part(sizeof(int)),
+               atc = part(sizeof(uint16_t) * (size_t)npad);
+  HPCCG_CUDA(cudaMalloc(&out->memory, bytes));
+  unsigned char *mem = static_cast<unsigned char *>(out->memory);
+  PatTable *t = reinterpret_cast<PatTable *>(mem + at_t);
+  out->t64 = reinterpret_cast<PatEntry64 *>(mem + at64);
+  out->t32 = reinterpret_cast<PatEntry32 *>(mem + at32);
+  out->t16 = reinterpret_cast<PatEntry32 *>(mem + at16);
+  out->box64 = reinterpret_cast<double *>(mem + b64);
+  out->box32 = reinterpret_cast<float *>(mem + b32);
+  out->box16 = reinterpret_cast<float *>(mem + b16);
+  out->flag = reinterpret_cast<int *>(mem + atf);
+  out->code = reinterpret_cast<uint16_t *>(mem + atc);
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + kBlock - 1) / kBlock, (int64_t)num_sms * 8));
   std::vector<int> rep(kPatSlots), id(kPatSlots, -1), rows;
   int flags[2] = {0, 0};
@@ -135,10 +155,6 @@ int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n,
       rows.push_back(found[k].first);
     }
     const size_t ne = found.size() * kPatW;
-    if (e == cudaSuccess) e = cudaMalloc(&out->code, sizeof(uint16_t) * (size_t)npad);
-    if (e == cudaSuccess) e = cudaMalloc(&out->t64, sizeof(PatEntry64) * ne);
-    if (e == cudaSuccess) e = cudaMalloc(&out->t32, sizeof(PatEntry32) * ne);
-    if (e == cudaSuccess) e = cudaMalloc(&out->t16, sizeof(PatEntry32) * ne);
     if (e == cudaSuccess) e = cudaMemsetAsync(out->code, 0, sizeof(uint16_t) * (size_t)npad, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(t->id, id.data(), sizeof(t->id), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
@@ -153,9 +169,45 @@ int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n,
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e == cudaSuccess && !flags[1]) out->count = (int)rows.size();
   }
-  cudaFree(t);
   if (e != cudaSuccess || !out->count) free_patterns(out);
   HPCCG_CUDA(e);
+  return HPCCG_OK;
+}
+
+// One thread per pattern: its entries (without the padding slots, offset 0 and value
+// +0.0, at the end) at their places of the 3x3x3 box, in order; *bad where one has none.
+__global__ void k_pat_boxes(const PatEntry64 *t64, int count, int nx, int ny, double *box64, float *box32,
+                            float *box16, int *bad) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= count) return;
+  const PatEntry64 *row = t64 + (size_t)c * kPatW;
+  int len = kPatW;
+  while (len > 0 && row[len - 1].off == 0 && __double_as_longlong(row[len - 1].v) == 0) --len;
+  int k = 0;
+  for (int j = 0; j < kPatW; ++j) {
+    const int off = ((j / 9 - 1) * ny + (j / 3 % 3 - 1)) * nx + (j % 3 - 1);
+    const bool have = k < len && row[k].off == off;
+    const double v = have ? row[k].v : 0.0;
+    k += have;
+    box64[(size_t)c * kPatW + j] = v;
+    box32[(size_t)c * kPatW + j] = (float)v;
+    box16[(size_t)c * kPatW + j] = __bfloat162float(__double2bfloat16(v));
+  }
+  if (k != len) *bad = 1;
+}
+
+int pattern_boxes(RowPatterns *p, int nx, int ny, cudaStream_t s) {
+  p->boxes = false;
+  p->box_nx = nx;
+  p->box_ny = ny;
+  if (!p->count || nx < 3 || ny < 3) return HPCCG_OK;  // narrower: neighbours' offsets coincide
+  int bad = 1;
+  HPCCG_CUDA(cudaMemsetAsync(p->flag, 0, sizeof(int), s));
+  k_pat_boxes<<<(p->count + 31) / 32, 32, 0, s>>>(p->t64, p->count, nx, ny, p->box64, p->box32, p->box16, p->flag);
+  HPCCG_CUDA(cudaGetLastError());
+  HPCCG_CUDA(cudaMemcpyAsync(&bad, p->flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+  HPCCG_CUDA(cudaStreamSynchronize(s));
+  p->boxes = !bad;
   return HPCCG_OK;
 }
 

@@ -32,55 +32,16 @@ __device__ __forceinline__ PatEntry32 pat_entry(const PatEntry32 *p) {
 int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n, int max_count, int num_sms,
                  cudaStream_t s, RowPatterns *out);
 void free_patterns(RowPatterns *p);
+// For a matrix on a known grid: the patterns as values at the 3x3x3 neighbours
+// (p->box64 and its roundings); p->boxes tells whether every one's entries lie
+// there in order.  Synchronises the stream.
+int pattern_boxes(RowPatterns *p, int nx, int ny, cudaStream_t s);
 
 __device__ __forceinline__ double pat_term(double s, const PatEntry64 &e, const double *__restrict__ x) {
   return __dadd_rn(s, __dmul_rn(e.v, __ldg(x + e.off)));  // the ELL kernels' operations
 }
 __device__ __forceinline__ float pat_term(float s, const PatEntry32 &e, const float *__restrict__ x) {
   return fmaf(e.v, __ldg(x + e.off), s);
-}
-
-// Sums of G rows (row(r), r < count), handed to done(row, sum) in order; a row's
-// terms are added in slot order, as in the ELL kernels.  `table` is the block's
-// copy in shared memory: a warp whose lanes share a pattern reads one address.
-// SHARE: the rows lie along a walk of the grid and mostly have one pattern, so
-// when all G agree each entry is read once for them.
-template <int G, bool SHARE, typename Real, typename Entry, class Row, class Done>
-__device__ __forceinline__ void pattern_group(Row &&row, int count, const uint16_t *__restrict__ code,
-                                              const Entry *table, const Real *__restrict__ x, Done &&done) {
-  int t[G];
-  bool same = count == G;
-#pragma unroll
-  for (int r = 0; r < G; ++r) {
-    t[r] = (r < count ? (int)__ldg(code + row(r)) : 0) * kPatW;
-    same = same && t[r] == t[0];
-  }
-  Real s[G];
-#pragma unroll
-  for (int r = 0; r < G; ++r) s[r] = Real(0);
-  if (SHARE && same) {
-#pragma unroll 9
-    for (int k = 0; k < kPatW; ++k) {
-      const Entry e = table[t[0] + k];
-#pragma unroll
-      for (int r = 0; r < G; ++r) s[r] = pat_term(s[r], e, x + row(r));
-    }
-  } else if (!SHARE) {
-#pragma unroll 9
-    for (int k = 0; k < kPatW; ++k)
-#pragma unroll
-      for (int r = 0; r < G; ++r)
-        if (r < count) s[r] = pat_term(s[r], table[t[r] + k], x + row(r));
-  } else {
-#pragma unroll
-    for (int r = 0; r < G; ++r)
-      if (r < count)
-#pragma unroll 9
-        for (int k = 0; k < kPatW; ++k) s[r] = pat_term(s[r], table[t[r] + k], x + row(r));
-  }
-#pragma unroll
-  for (int r = 0; r < G; ++r)
-    if (r < count) done(row(r), s[r]);
 }
 
 // The block's copy of the table.
@@ -92,45 +53,166 @@ __device__ __forceinline__ const Entry *pattern_table(const Entry *__restrict__ 
   return local;
 }
 
-// The calling thread's rows under a map of the grid, in the order of thread_rows
-// (hpccg_rows.cuh): the column pair of a tile or two-line map two planes at a
-// time, or a column two planes at a time.
-template <typename Real, typename Entry, class Done>
-__device__ __forceinline__ void pattern_walk(int n, const PlaneMap &m, const uint16_t *__restrict__ code,
-                                             const Entry *__restrict__ table, int count, const Real *__restrict__ x,
-                                             Done &&done) {
-  const Entry *local = pattern_table(table, count);
-  if (m.ry == 2) {
-    int c, z0, z1;
-    if (m.tiles_x > 0) {
-      const TileSpan sp = tile_span(m, n / m.plane);
-      if (!sp.rows) return;
-      c = sp.c, z0 = sp.z0, z1 = sp.z1;
-    } else {
-      const PlaneSpan sp = plane_span(m, n / m.plane);
-      c = sp.c, z0 = sp.z0, z1 = sp.z1;
-    }
-    for (int z = z0; z < z1; z += 2) {
-      const int i = c + z * m.plane;
-      pattern_group<4, true>([&](int r) { return i + (r & 1) * m.nx + (r >> 1) * m.plane; }, min(4, 2 * (z1 - z)), code,
-                             local, x, done);
-    }
-  } else {
-    const PlaneSpan sp = plane_span(m, n / m.plane);
-    for (int z = sp.z0; z < sp.z1; z += 2) {
-      const int i = sp.c + z * m.plane;
-      pattern_group<2, true>([&](int r) { return i + r * m.plane; }, min(2, sp.z1 - z), code, local, x, done);
-    }
-  }
-}
-// Grid-stride rows, one at a time.
+// Grid-stride rows, one at a time; a row's terms are added in slot order, as in the
+// ELL kernels.  A warp whose lanes share a pattern reads one address of the table.
 template <typename Real, typename Entry, class Done>
 __device__ __forceinline__ void pattern_stride(int n, const uint16_t *__restrict__ code,
                                                const Entry *__restrict__ table, int count,
                                                const Real *__restrict__ x, Done &&done) {
   const Entry *local = pattern_table(table, count);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    pattern_group<1, false>([&](int) { return i; }, 1, code, local, x, done);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Entry *t = local + (int)__ldg(code + i) * kPatW;
+    Real s = Real(0);
+#pragma unroll 9
+    for (int k = 0; k < kPatW; ++k) s = pat_term(s, t[k], x + i);
+    done(i, s);
+  }
+}
+
+// ---- walks of a known grid with the patterns' values as 3x3x3 boxes -----------------
+// A walk along z loads each plane's neighbourhood once (9 values for a column, 12
+// for a column pair) for the three rows that need it, instead of 27 gathers a
+// row; the sums are split at the planes as in stencil_column2 and take each row's
+// own values (its pattern's box, in shared memory).  A neighbour that a row does
+// not have adds 0 * 0 (outside the grid) to a sum that is never -0.0, so the sums
+// are the ELL kernels', bit for bit.
+__device__ __forceinline__ double box_term(double s, double v, double x) { return __dadd_rn(s, __dmul_rn(v, x)); }
+__device__ __forceinline__ float box_term(float s, float v, float x) { return fmaf(v, x, s); }
+
+// The sums in flight of RY rows side by side in y: lead = plane z-1's nine terms of
+// the next plane's rows, mid = the current plane's rows through their own plane.
+template <typename Real, int RY>
+struct BoxSums {
+  Real lead[RY], mid[RY], xc[RY];
+  // plane p's values (lines y-1 .. y+RY, three each) and the boxes of the rows of
+  // planes p-1 (te), p (tm) and p+1 (tl): END the rows of p-1 (into s), MID those of
+  // p, and start the leads of p+1.  Rows of a pair that share a box read it once.
+  template <bool END, bool MID>
+  __device__ __forceinline__ void plane(const Real *v, const Real *const *te, const Real *const *tm,
+                                        const Real *const *tl, Real *s) {
+    bool same = true;
+    if (RY == 2) same = te[0] == te[RY - 1] && tm[0] == tm[RY - 1] && tl[0] == tl[RY - 1];
+    if (RY == 1 || __all_sync(__activemask(), same)) step<END, MID, true>(v, te, tm, tl, s);
+    else step<END, MID, false>(v, te, tm, tl, s);
+  }
+  template <bool END, bool MID, bool SAME>
+  __device__ __forceinline__ void step(const Real *v, const Real *const *te, const Real *const *tm,
+                                       const Real *const *tl, Real *s) {
+    if (END) {
+#pragma unroll
+      for (int r = 0; r < RY; ++r) s[r] = mid[r];
+#pragma unroll
+      for (int j = 0; j < 9; ++j) {
+        const Real t = te[0][18 + j];
+#pragma unroll
+        for (int r = 0; r < RY; ++r) s[r] = box_term(s[r], SAME ? t : te[r][18 + j], v[3 * r + j]);
+      }
+    }
+    if (MID) {
+#pragma unroll
+      for (int r = 0; r < RY; ++r) {
+        mid[r] = lead[r];
+        xc[r] = v[3 * r + 4];
+      }
+#pragma unroll
+      for (int j = 0; j < 9; ++j) {
+        const Real t = tm[0][9 + j];
+#pragma unroll
+        for (int r = 0; r < RY; ++r) mid[r] = box_term(mid[r], SAME ? t : tm[r][9 + j], v[3 * r + j]);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RY; ++r) lead[r] = Real(0);
+#pragma unroll
+    for (int j = 0; j < 9; ++j) {
+      const Real t = tl[0][j];
+#pragma unroll
+      for (int r = 0; r < RY; ++r) lead[r] = box_term(lead[r], SAME ? t : tl[r][j], v[3 * r + j]);
+    }
+  }
+};
+
+// Walks rows [z0, z1) of the column c (and c + nx): load(p, v) gives plane p's values
+// and returns false to stop; done(row, sum, x) in the order of thread_rows.
+template <typename Real, int RY, class Load, class Done>
+__device__ __forceinline__ void box_walk(int c, int z0, int z1, int nx, int plane, int nz,
+                                         const uint16_t *__restrict__ code, const Real *table, Load &&load,
+                                         Done &&done) {
+  const Real *te[RY], *tm[RY], *tl[RY];
+  auto box = [&](int z, int r) {  // the row's box (any, beyond the last plane)
+    return table + (int)__ldg(code + c + r * nx + min(z, nz - 1) * plane) * kPatW;
+  };
+  Real v[3 * (RY + 2)], s[RY];
+  BoxSums<Real, RY> w;
+#pragma unroll
+  for (int r = 0; r < RY; ++r) te[r] = tm[r] = tl[r] = box(z0, r);
+  if (!load(z0 - 1, v)) return;
+  w.template plane<false, false>(v, te, tm, tl, s);
+#pragma unroll
+  for (int r = 0; r < RY; ++r) tl[r] = box(z0 + 1, r);
+  if (!load(z0, v)) return;
+  w.template plane<false, true>(v, te, tm, tl, s);
+  for (int z = z0; z < z1; ++z) {
+#pragma unroll
+    for (int r = 0; r < RY; ++r) {
+      te[r] = tm[r];
+      tm[r] = tl[r];
+      tl[r] = box(z + 2, r);
+    }
+    if (!load(z + 1, v)) return;
+    Real x[RY];
+#pragma unroll
+    for (int r = 0; r < RY; ++r) x[r] = w.xc[r];
+    w.template plane<true, true>(v, te, tm, tl, s);
+#pragma unroll
+    for (int r = 0; r < RY; ++r) done(c + r * nx + z * plane, s[r], x[r]);
+  }
+}
+
+// The block's copy of the boxes.
+template <typename Real>
+__device__ __forceinline__ const Real *box_table(const Real *__restrict__ table, int count) {
+  __shared__ Real local[kPatLocal * kPatW];
+  for (int i = threadIdx.x; i < count * kPatW; i += blockDim.x) local[i] = table[i];
+  __syncthreads();
+  return local;
+}
+
+// The calling thread's rows under a map of the grid, from plain loads.
+template <typename Real, class Done>
+__device__ __forceinline__ void box_rows(const StencilGeom &g, const PlaneMap &m, const uint16_t *__restrict__ code,
+                                         const Real *__restrict__ table, int count, const Real *__restrict__ x,
+                                         Done &&done) {
+  const Real *local = box_table(table, count);
+  int c, z0, z1;
+  if (m.tiles_x > 0) {
+    const TileSpan sp = tile_span(m, g.nz);
+    if (!sp.rows) return;
+    c = sp.c, z0 = sp.z0, z1 = sp.z1;
+  } else {
+    const PlaneSpan sp = plane_span(m, g.nz);
+    c = sp.c, z0 = sp.z0, z1 = sp.z1;
+  }
+  if (z0 >= z1) return;
+  const int iy = c / g.nx, ix = c - iy * g.nx;
+  const Real *xc = x + c;
+  if (m.ry == 2) {
+    const unsigned mask = stencil_mask4(g, ix, iy);
+    box_walk<Real, 2>(c, z0, z1, g.nx, m.plane, g.nz, code, local,
+                      [&](int p, Real *v) {
+                        stencil_plane4<Real, false>(xc + (int64_t)p * m.plane, g.nx, mask, (unsigned)p < (unsigned)g.nz, v);
+                        return true;
+                      },
+                      done);
+  } else {
+    const unsigned mask = stencil_mask(g, ix, iy);
+    box_walk<Real, 1>(c, z0, z1, g.nx, m.plane, g.nz, code, local,
+                      [&](int p, Real *v) {
+                        stencil_plane<Real>(xc + (int64_t)p * m.plane, g.nx, mask, (unsigned)p < (unsigned)g.nz, v);
+                        return true;
+                      },
+                      done);
+  }
 }
 
 }  // namespace hpccg

@@ -14,7 +14,7 @@
 //    keeps x.
 //  * csr_vector_rows<LPR>: LPR lanes per CSR row (LPR = 32 is warp-per-row),
 //    lane-strided loads, butterfly shuffle reduction.  Reassociates the sum.
-//  * StratPatternWalk / Stride (hpccg_pattern.cuh): the ELL as row patterns, for a matrix that
+//  * StratPatternBox / Stride (hpccg_pattern.cuh): the ELL as row patterns, for a matrix that
 //    has few; the ELL kernel's rows, terms and order, so bit-identical to it.
 //  * stencil_rows (hpccg_stencil.cuh): matrix-free, for a context whose CSR
 //    was checked equal to generate_matrix(nx,ny,nz); bit-identical to ELL
@@ -206,6 +206,7 @@ struct SpmvArgs {
   const uint16_t *pat_code;   // row patterns
   const PatEntry64 *pat;
   int pat_count;
+  const double *pat_box;      // the patterns as 3x3x3 boxes (null: not in use)
   StencilGeom geom;  // grid of generate_matrix (STENCIL only)
   PlaneMap pm;       // row map of ELL (one row per thread) and STENCIL when the grid is known
   // STENCIL under the tile map: tensor maps of the two vectors tma_vec[0..1],
@@ -238,22 +239,32 @@ struct StratEll1 {
     return ell_rows<27, 1, 27>(a.n, a.npad, a.ell_col, a.ell_val, x, e, a.pm);
   }
 };
-// Row patterns: 2 bytes per row instead of 12 per slot, so the x gathers bound it
-// (a misaligned 256-byte L1 read costs 4 to 5 cycles, 27 of them per 32 rows) and
-// not HBM.  FP64 SpMV + dot: on a known grid, walking it with four rows to a table
-// read, 117 -> 38 us at 128^3 (four rows from global memory 41, two 46, one
-// table read per row 67; more or fewer blocks per SM slower); without a grid one
-// row at a time at full occupancy, 26.7 -> 14.7 us at 97 x 75 x 61 (two rows and
-// half the occupancy: 17.1).
-struct StratPatternWalk {  // the grid is known
+// Row patterns: 2 bytes per row instead of 12 per slot, so the x reads bound it and
+// not HBM: 27 gathers a row cost 4 to 5 L1 cycles each (misaligned 256-byte reads).
+// On a known grid a walk reads each plane once for three rows (StratPatternBox), by
+// TMA where x has a tensor map; without a grid, or where the walk has too few
+// blocks, one row at a time at full occupancy.  FP64 SpMV + dot at 128^3: ELL 117
+// us, gathers 38 (four rows of a walk to a table read), box walk by TMA 21.7
+// (two, four and five blocks per SM: 23.6, 23.6, 31.3); CSR of
+// 97 x 75 x 61: 26.7 -> 14.7 (two rows a thread and half the occupancy: 17.1).
+struct StratPatternBox {  // the grid is known and every pattern lies in its 3x3x3 boxes
   static constexpr int kMinBlocks = 4;
   static int grid(const SpmvArgs &a, int) { return plane_grid(a.pm); }
   template <class Epi>
   static __device__ __forceinline__ double rows(const SpmvArgs &a, const double *x, Epi &e) {
     double part = 0.0;
-    pattern_walk(a.n, a.pm, a.pat_code, a.pat, a.pat_count, x,
-                 [&](int i, double s) { part = __dadd_rn(part, e(i, s)); });
+    box_rows(a.geom, a.pm, a.pat_code, a.pat_box, a.pat_count, x,
+             [&](int i, double s, double xi) { part = __dadd_rn(part, e(i, s, xi)); });
     return part;
+  }
+};
+struct StratPatternBoxTma {  // the same with x by TMA
+  static constexpr int kMinBlocks = 3;
+  static int grid(const SpmvArgs &a, int) { return plane_grid(a.pm); }
+  template <class Epi>
+  static __device__ __forceinline__ double rows(const SpmvArgs &a, const double *x, Epi &e) {
+    return box_rows_tma64(a.geom, a.pm, a.pat_code, a.pat_box, a.pat_count, &a.tmap[x == a.tma_vec[0] ? 0 : 1], e,
+                          a.status);
   }
 };
 struct StratPatternStride {
@@ -336,7 +347,11 @@ inline int dispatch_strategy(const SpmvArgs &a, F &&f, const double *x = nullptr
     if (x && a.tma_ok && a.pm.tiles_x > 0 && (x == a.tma_vec[0] || x == a.tma_vec[1])) return f(StratStencilTma{});
     return f(StratStencil{});
   }
-  if (a.kind == kSpmvPattern) return a.pm.plane > 0 ? f(StratPatternWalk{}) : f(StratPatternStride{});
+  if (a.kind == kSpmvPattern) {
+    if (!a.pat_box) return f(StratPatternStride{});
+    if (x && a.tma_ok && (x == a.tma_vec[0] || x == a.tma_vec[1])) return f(StratPatternBoxTma{});
+    return f(StratPatternBox{});
+  }
   if (a.kind == HPCCG_SPMV_CSR_VECTOR) {
     switch (a.param) {
       case 4: return f(StratCsr<4>{});
@@ -399,6 +414,8 @@ inline SpmvArgs spmv_args(const hpccg_ctx *c) {
   a.pat_count = c->pat.count;
   a.geom = StencilGeom{c->gx, c->gy, c->gz};
   a.pm = c->gx ? fp64_map(c->gx, c->gy, c->gz, c->num_sms) : PlaneMap{0, 0, 0, 1, 1, 0};
+  // worth it where the walk's blocks fill the SMs three times over (fewer: gathers)
+  a.pat_box = c->gx && a.pm.plane > 0 && plane_grid(a.pm) >= 3 * c->num_sms && c->pat.boxes ? c->pat.box64 : nullptr;
   a.tma_ok = a.pm.tiles_x > 0 && c->tmaps_ok;
   if (a.tma_ok) {
     a.tmap[0] = c->tmaps[0];

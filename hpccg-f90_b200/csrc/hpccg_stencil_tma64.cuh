@@ -25,6 +25,7 @@
 // HPCCG_ERR_TIMEOUT in the caller's status word, waits (bounded) for its own
 // loads in flight and finishes without the remaining rows.
 #pragma once
+#include "hpccg_pattern.cuh"
 #include "hpccg_stencil.cuh"
 #include "hpccg_stencil_tma.cuh"
 
@@ -264,6 +265,40 @@ __device__ __forceinline__ double stencil_rows_tma64ref(const StencilGeom &g, co
       }
     }
   }
+  if (ring.consumed < sp.z1) ring.drain();
+  return part;
+}
+
+// The same walk with each row's values from its pattern's box (hpccg_pattern.cuh).
+template <class Epi>
+__device__ __forceinline__ double box_rows_tma64(const StencilGeom &g, const PlaneMap &m, const uint16_t *code,
+                                                 const double *table, int count, const CUtensorMap *map, Epi &epi,
+                                                 int *status) {
+  __shared__ __align__(128) unsigned char ring_slots[kR64RingBytes];
+  __shared__ uint64_t full[kR64Stages];
+  double part = 0.0;
+  const TileSpan sp = tile_span(m, g.nz);
+  PlaneRing<kR64Stages> ring{ring_slots, kR64Slot, full, map, sp.x0 - 2, sp.y0 - 1, kR64BoxBytes, sp.z0 - 1, sp.z1,
+                             0, 0};
+  ring.init();
+  const double *local = box_table(table, count);  // has the CTA barrier
+  ring.prime();
+  const int tx = threadIdx.x % kR64TileX, ty = threadIdx.x / kR64TileX;
+  const int ofs = (2 * ty) * kR64BoxX + 1 + tx;  // box position of (x-1, y-1)
+  // a thread without rows walks along (the barriers need it) with the codes of column 0
+  box_walk<double, 2>(sp.rows ? sp.c : 0, sp.z0, sp.z1, g.nx, m.plane, g.nz, code, local,
+                      [&](int p, double *v) -> bool {
+                        const bool ok = ring.wait(p, status);
+                        if (ok) {
+                          const double *c = reinterpret_cast<const double *>(ring.data(p)) + ofs;
+#pragma unroll
+                          for (int j = 0; j < 12; ++j) v[j] = c[(j / 3) * kR64BoxX + j % 3];
+                        }
+                        return ring.release(p, ok);
+                      },
+                      [&](int i, double s, double x) {
+                        if (sp.rows) part = __dadd_rn(part, epi(i, s, x));
+                      });
   if (ring.consumed < sp.z1) ring.drain();
   return part;
 }

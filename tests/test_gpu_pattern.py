@@ -52,6 +52,28 @@ def test_patterns_equal_ell_on_grids(env, nx, ny, nz, known_grid):
         assert np.array_equal(g, w)
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(128, 128, 112), (130, 132, 90), (151, 131, 97), (161, 160, 160)])
+def test_box_walks_equal_ell(env, nx, ny, nz):
+    """Grids large enough for the walks: tiles (whole and partial) by TMA and by plain
+    loads, one line and two lines a thread.  CG runs its graph at these sizes: the
+    same sums in the same order, so the same bits."""
+    torch, hp = env
+    M = hp.Matrix.generated(nx, ny, nz)
+    x = np.random.default_rng(nx).uniform(-1, 1, M.nrow)
+    got, want = _products(torch, hp, M, hp.SPMV_AUTO, x), _products(torch, hp, M, hp.SPMV_ELL, x)
+    for g, w in zip(got, want):
+        assert np.array_equal(g, w)
+    b = torch.from_numpy(x).cuda()
+    runs = []
+    for kind in (hp.SPMV_AUTO, hp.SPMV_ELL):
+        M.set_spmv(kind)
+        d = torch.full_like(b, 0.5)
+        it, normr, hist, st = M.cg_device(b, d, 7, 0.0)
+        runs.append((it, normr, hist, st, d.cpu().numpy()))
+    for g, w in zip(*runs):
+        assert np.array_equal(g, w)
+
+
 def _mixed_rows(rng, n, npat):
     """A CSR of n rows with npat patterns of up to 27 entries (one of them full)."""
     pats = []
