@@ -187,18 +187,14 @@ static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, c
   a.nz = Lv.nz;
   a.nb = u->nb;
   a.nin = nin;
-  a.cin = bwd_group >= 0 ? 16 : d.cin;
   a.in0 = in0;
   a.in1 = in1;
-  a.in_f32 = in_f32;
   a.W = bwd_group >= 0 ? u->flip[layer][bwd_group] : W;
   a.bias = bwd_group >= 0 ? nullptr : bias;
   a.proj = proj;
   a.epi = epi;
   a.out = out;
-  k_conv3_cc<<<grid1d(u, Lv.nvox), 256, 0, u->stream>>>(a);
-  HPCCG_CUDA(cudaGetLastError());
-  return HPCCG_OK;
+  return launch_conv3_cc(a, u->num_sms, u->stream);
 }
 
 #define UNET_TRY(x)              \
@@ -605,16 +601,14 @@ extern "C" int hpccg_unet_conv3_layer(int32_t nx, int32_t ny, int32_t nz, int32_
     a.nz = nz;
     a.nb = nb;
     a.nin = nin;
-    a.cin = 16 * nin;
     a.in0 = static_cast<const __nv_bfloat16 *>(d_in0);
     a.in1 = static_cast<const __nv_bfloat16 *>(d_in1);
-    a.in_f32 = nullptr;
     a.W = d_w;
     a.bias = d_bias;
     a.proj = d_proj;
     a.epi = epi;
     a.out = d_out;
-    k_conv3_cc<<<sms * 8, 256>>>(a);
+    rc = launch_conv3_cc(a, sms, 0);
     if (cudaDeviceSynchronize() != cudaSuccess) rc = set_cuda_error(cudaGetLastError(), "conv3 cc", __FILE__, __LINE__);
   }
   int err = 0;

@@ -3,6 +3,8 @@
 // upsampling, ReLU masks, weight/bias gradients, the output projection, the
 // loss and the Adam update.  All are memory-bound or tiny.  16-channel
 // tensors use the row-planar layout of unet_conv.cuh (act_unit / act_elem).
+#include <algorithm>
+
 #include "unet_ops.cuh"
 
 namespace hpccg {
@@ -35,59 +37,176 @@ __global__ void k_flip_fp32(const float *W, int cin, int g, float *Wf) {
 }
 
 // ---- direct conv on CUDA cores --------------------------------------------------------
-// out[v][co] = sum_tap sum_ci in[v + off(tap)][ci] * W[tap][ci][co] (+ bias, ReLU).
-// Inputs: in0/in1 row-planar BF16 16-channel tensors (in1 nullable), or in_f32
-// one-channel FP32 (cin = 1).  One thread per output voxel.
-__global__ void k_conv3_cc(CcConvArgs a) {
-  const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const int64_t nvox = (int64_t)nx * ny * nz * a.nb;
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nvox; v += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(v % nx), y = (int)((v / nx) % ny), z = (int)((v / ((int64_t)nx * ny)) % nz);
-    const int64_t b = v / ((int64_t)nx * ny * nz);
-    float acc[16];
+// out[v][co] = sum_tap sum_ci in[v + off(tap)][ci] * W[tap][ci][co] (+ bias, ReLU), for
+// volumes without 128-voxel bricks; FP32 weights.  Inputs: in0/in1 row-planar BF16
+// 16-channel tensors (in1 nullable).  A thread forms CO of the 16 channels of V
+// voxels (x, y .. y+V-1), lanes along x: per tap and input group it loads its voxels'
+// channels as 16-byte units, and every weight, read from the block's copy in shared
+// memory (one address for the warp, or one per channel group), feeds V fused
+// multiply-adds, two channels at a time.  A voxel's terms are added in the order
+// tap, group, channel; taps outside the grid are left out.  V and CO fall with the
+// volume so that it fills the SMs (launch_conv3_cc).
+// One voxel a thread with scalar loads, against this: forward pass at 192^3 27.7 ->
+// 8.4 ms, 96^3 4.30 -> 1.36, 24^3 1.41 -> 0.27.  Bound by the FP32 pipe on large volumes
+// (6912 multiply-adds a voxel and group: 226 G of them at 192^3, 7.8 ms, 80% of its
+// rate), by the latency of the 27 taps on small ones.
+__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(unsigned long long v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma_f32x2(unsigned long long &d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+// One tap and input group of N voxels: q = their 16 channels, w = the weights [16 ci][16 co]
+// from the thread's first channel on.
+template <int N, int CO>
+__device__ __forceinline__ void cc_tap(const uint4 (*q)[2], const float *w, unsigned long long (*acc)[CO / 2]) {
 #pragma unroll
-    for (int c = 0; c < 16; ++c) acc[c] = 0.f;
+  for (int ci = 0; ci < 16; ++ci) {
+    unsigned long long wv[CO / 2];
+#pragma unroll
+    for (int c = 0; c < CO / 4; ++c) {
+      const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(w + ci * 16 + 4 * c);
+      wv[2 * c] = t.x;
+      wv[2 * c + 1] = t.y;
+    }
+#pragma unroll
+    for (int v = 0; v < N; ++v) {
+      const uint4 &u = q[v][ci >> 3];
+      const uint32_t p = (ci & 7) < 2 ? u.x : (ci & 7) < 4 ? u.y : (ci & 7) < 6 ? u.z : u.w;
+      const float f = __uint_as_float(ci & 1 ? p & 0xffff0000u : p << 16);
+      const unsigned long long ff = pack_f32x2(f, f);
+#pragma unroll
+      for (int c = 0; c < CO / 2; ++c) fma_f32x2(acc[v][c], ff, wv[c]);
+    }
+  }
+}
+
+constexpr int kCcThreads = 128;
+// resident blocks an SM (the registers of V * CO sums)
+template <int V, int CO>
+constexpr int cc_blocks() { return V == 4 ? 3 : 8; }
+
+template <int V, int CO>
+__global__ void __launch_bounds__(kCcThreads, cc_blocks<V, CO>()) k_conv3_cc(CcConvArgs a) {
+  extern __shared__ __align__(16) float cc_w[];  // [27][cin][16]
+  const int nx = a.nx, ny = a.ny, nz = a.nz, cin = 16 * a.nin;
+  for (int e = threadIdx.x; e < 27 * cin * 4; e += blockDim.x)
+    reinterpret_cast<float4 *>(cc_w)[e] = __ldg(reinterpret_cast<const float4 *>(a.W) + e);
+  __syncthreads();
+  constexpr int NG = 16 / CO;
+  const int nyg = (ny + V - 1) / V;
+  const int64_t total = (int64_t)nx * nyg * nz * a.nb * NG;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+    const int c0 = (int)(e % NG) * CO;
+    int64_t t = e / NG;
+    const int x = (int)(t % nx);
+    t /= nx;
+    const int y = (int)(t % nyg) * V;
+    t /= nyg;
+    const int z = (int)(t % nz);
+    const int64_t row = t * ny + y;  // (b * nz + z) * ny + y
+    const int nv = min(V, ny - y);
+    unsigned long long acc[V][CO / 2];
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int c = 0; c < CO / 2; ++c) acc[v][c] = 0ull;
     for (int tap = 0; tap < 27; ++tap) {
-      const int xx = x + tap % 3 - 1, yy = y + (tap / 3) % 3 - 1, zz = z + tap / 9 - 1;
-      if (xx < 0 || xx >= nx || yy < 0 || yy >= ny || zz < 0 || zz >= nz) continue;
-      const int64_t row = (b * nz + zz) * ny + yy;
-      if (a.in_f32) {
-        const float s = a.in_f32[row * nx + xx];
-        const float *w = a.W + (size_t)tap * 16;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) acc[c] = fmaf(s, w[c], acc[c]);
-        continue;
-      }
+      const int dx = tap % 3 - 1, dy = tap / 3 % 3 - 1, dz = tap / 9 - 1;
+      if ((unsigned)(x + dx) >= (unsigned)nx || (unsigned)(z + dz) >= (unsigned)nz) continue;
+      const int64_t r0 = row + dz * ny + dy;
+      const int lo = max(0, -(y + dy)), hi = min(nv, ny - (y + dy));  // voxels whose row y+v+dy is inside
       for (int g = 0; g < a.nin; ++g) {
-        const __nv_bfloat16 *src = g ? a.in1 : a.in0;
-        for (int ci = 0; ci < 16; ++ci) {
-          const float s = __bfloat162float(src[act_elem(row, xx, ci, nx)]);
-          const float *w = a.W + ((size_t)tap * a.cin + g * 16 + ci) * 16;
+        const uint4 *src = reinterpret_cast<const uint4 *>(g ? a.in1 : a.in0);
+        const float *w = cc_w + (tap * cin + g * 16) * 16 + c0;
+        uint4 q[V][2];
+        if (lo == 0 && hi == V) {
 #pragma unroll
-          for (int c = 0; c < 16; ++c) acc[c] = fmaf(s, w[c], acc[c]);
+          for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) q[v][h] = __ldg(src + act_unit(r0 + v, h, x + dx, nx));
+          cc_tap<V, CO>(q, w, acc);
+        } else {
+#pragma unroll
+          for (int v = 0; v < V; ++v)
+            if (v >= lo && v < hi) {
+#pragma unroll
+              for (int h = 0; h < 2; ++h) q[v][h] = __ldg(src + act_unit(r0 + v, h, x + dx, nx));
+              cc_tap<1, CO>(q + v, w, acc + v);
+            }
         }
       }
     }
-    const int64_t orow = (b * nz + z) * ny + y;
-    if (a.epi == kEpiRawF32) {
-      float *o = static_cast<float *>(a.out);
 #pragma unroll
-      for (int c = 0; c < 16; ++c) o[act_elem(orow, x, c, nx)] = acc[c];
-    } else if (a.epi == kEpiProject) {
-      float r = a.proj[16];
+    for (int v = 0; v < V; ++v) {
+      if (v >= nv) break;
+      float o[CO];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) r = fmaf(a.proj[c], fmaxf(acc[c] + a.bias[c], 0.f), r);
-      static_cast<float *>(a.out)[v] = r;
-    } else {
-      __nv_bfloat16 *o = static_cast<__nv_bfloat16 *>(a.out);
+      for (int c = 0; c < CO / 2; ++c) unpack_f32x2(acc[v][c], o[2 * c], o[2 * c + 1]);
+      if (a.epi == kEpiRawF32) {
+        float *dst = static_cast<float *>(a.out);
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        float t = acc[c] + (a.bias ? a.bias[c] : 0.f);
-        if (a.epi == kEpiBiasRelu) t = fmaxf(t, 0.f);
-        o[act_elem(orow, x, c, nx)] = __float2bfloat16(t);
+        for (int c = 0; c < CO; c += 4)
+          *reinterpret_cast<float4 *>(dst + act_elem(row + v, x, c0 + c, nx)) =
+              make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
+      } else if (CO == 16 && a.epi == kEpiProject) {
+        float r = a.proj[16];
+#pragma unroll
+        for (int c = 0; c < CO; ++c) r = fmaf(a.proj[c], fmaxf(o[c] + a.bias[c], 0.f), r);
+        static_cast<float *>(a.out)[(row + v) * nx + x] = r;
+      } else {
+        __nv_bfloat16 *dst = static_cast<__nv_bfloat16 *>(a.out);
+#pragma unroll
+        for (int c = 0; c < CO; c += 4) {
+          uint32_t p[2];
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            float f[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              f[j] = o[c + 2 * k + j] + (a.bias ? a.bias[c0 + c + 2 * k + j] : 0.f);
+              if (a.epi == kEpiBiasRelu) f[j] = fmaxf(f[j], 0.f);
+            }
+            const __nv_bfloat162 b = __floats2bfloat162_rn(f[0], f[1]);
+            p[k] = *reinterpret_cast<const uint32_t *>(&b);
+          }
+          *reinterpret_cast<uint2 *>(dst + act_elem(row + v, x, c0 + c, nx)) = make_uint2(p[0], p[1]);
+        }
       }
     }
   }
+}
+
+template <int V, int CO>
+static int launch_cc(const CcConvArgs &a, int num_sms, cudaStream_t s) {
+  const int smem = 27 * 16 * a.nin * 16 * (int)sizeof(float);
+  // the attribute is per device: set every time
+  HPCCG_CUDA(cudaFuncSetAttribute(k_conv3_cc<V, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  27 * 32 * 16 * (int)sizeof(float)));
+  const int64_t threads = (int64_t)a.nx * ((a.ny + V - 1) / V) * a.nz * a.nb * (16 / CO);
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((threads + kCcThreads - 1) / kCcThreads,
+                                                          (int64_t)num_sms * cc_blocks<V, CO>()));
+  k_conv3_cc<V, CO><<<grid, kCcThreads, smem, s>>>(a);
+  HPCCG_CUDA(cudaGetLastError());
+  return HPCCG_OK;
+}
+
+// Four voxels a thread where that leaves every SM 256 threads, one where one does, else
+// several threads a voxel (the projection needs all channels in one).  Forward pass
+// with the lines at half | this | eight times the size: 56^3 0.54 | 0.52 | 0.59 ms,
+// 72^3 0.75 | 0.75 | 0.95, 88^3 1.29 | 1.20 | 1.58, 40x72x24 0.34 | 0.34 | 0.37.
+int launch_conv3_cc(const CcConvArgs &a, int num_sms, cudaStream_t s) {
+  const int64_t n = (int64_t)a.nx * a.ny * a.nz * a.nb, fill = (int64_t)num_sms * 256;
+  if (n >= 4 * fill) return launch_cc<4, 16>(a, num_sms, s);
+  if (n >= fill || a.epi == kEpiProject) return launch_cc<1, 16>(a, num_sms, s);
+  if (2 * n >= fill) return launch_cc<1, 8>(a, num_sms, s);
+  return launch_cc<1, 4>(a, num_sms, s);
 }
 
 // The 1-channel input layer: out[v][co] = act(sum_tap in[v+off] W[tap][co] + b[co]).

@@ -6,10 +6,9 @@ namespace hpccg {
 
 struct CcConvArgs {
   int nx, ny, nz, nb;
-  int nin, cin;                      // 16-channel input groups and total input channels
+  int nin;                           // 16-channel input groups
   const __nv_bfloat16 *in0, *in1;    // row-planar BF16 inputs
-  const float *in_f32;               // or a 1-channel FP32 input (cin = 1)
-  const float *W;                    // FP32 [27][cin][16]
+  const float *W;                    // FP32 [27][16 nin][16]
   const float *bias;                 // [16] or null
   const float *proj;                 // [17] for kEpiProject
   int epi;
@@ -27,7 +26,7 @@ struct DwArgs {
 __global__ void k_pack_fwd(const float *W, int cin, int nin, __nv_bfloat16 *packed);
 __global__ void k_pack_bwd(const float *W, int cin, int g, __nv_bfloat16 *packed);
 __global__ void k_flip_fp32(const float *W, int cin, int g, float *Wf);
-__global__ void k_conv3_cc(CcConvArgs a);
+int launch_conv3_cc(const CcConvArgs &a, int num_sms, cudaStream_t s);
 __global__ void k_conv3_in1(const float *in, const float *W, const float *bias, __nv_bfloat16 *out, int nx, int ny,
                             int nz, int nb, int relu);
 __global__ void k_conv3_in1x4(const float *in, const float *W, const float *bias, __nv_bfloat16 *out, int nx, int ny,

@@ -145,6 +145,38 @@ def test_conv_layer_window_edges(env, nx, ny, nz, nb, nin, epi):
         assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("nx,ny,nz,nb,nin,epi", [(1, 1, 1, 1, 1, 0), (3, 5, 2, 3, 2, 3), (24, 24, 24, 1, 1, 0), (24, 24, 24, 1, 2, 2),
+                                                (40, 37, 40, 1, 2, 0), (41, 69, 70, 1, 1, 3), (40, 67, 64, 1, 2, 2), (72, 1, 2200, 1, 1, 0)])
+def test_conv_layer_cuda_core_splits(env, nx, ny, nz, nb, nin, epi):
+    """Each split of the CUDA-core form (4, 8 and 16 channels a thread, four voxels) with rows
+    left over, FP32 weights.  Sums of 27 * 16 * nin products in FP32: an error of at most
+    432 nin * 2^-24 of the sum of their magnitudes, and half a BF16 unit on BF16 outputs."""
+    torch, hp = env
+    rng = np.random.default_rng(nx + 3 * ny + nin)
+    xs = [uo.bf16_round(rng.normal(0, 1, (nb, nz, ny, nx, 16))) for _ in range(nin)]
+    W = rng.normal(0, 0.1, (27, 16 * nin, 16)).astype(np.float32)
+    b = rng.normal(0, 0.1, 16).astype(np.float32)
+    proj = rng.normal(0, 0.3, 17).astype(np.float32)
+    dW, db, dp = (torch.from_numpy(v).cuda() for v in (W, b, proj))
+    din = [_bf16_tensor(torch, to_planar(v)) for v in xs] + [None]
+    n = nx * ny * nz * nb
+    dtype, size = {0: (torch.bfloat16, 16 * n), 2: (torch.float32, n), 3: (torch.float32, 16 * n)}[epi]
+    out = torch.full((size,), float("nan"), dtype=dtype, device="cuda")
+    hp.conv3_layer(din[0], din[1], dW, db, dp, epi, 1, out, nx, ny, nz, nb)
+    x = np.concatenate(xs, -1).astype(np.float64)
+    pre = uo.conv3(x, W.astype(np.float64))
+    mag = (uo.conv3(np.abs(x), np.abs(W).astype(np.float64)) + np.abs(b)) * 440 * nin * 2.0 ** -24
+    if epi == 2:
+        want = np.maximum(pre + b, 0) @ proj[:16].astype(np.float64) + proj[16]
+        bar = mag @ np.abs(proj[:16]) + 20 * 2.0 ** -24 * (np.maximum(pre + b, 0) @ np.abs(proj[:16]) + abs(proj[16]))
+        got = out.cpu().numpy().reshape(nb, nz, ny, nx)
+    else:
+        want = pre if epi == 3 else np.maximum(pre + b, 0)
+        bar = mag + (np.abs(want) * 2.0 ** -8 if epi == 0 else 0)
+        got = from_planar(out.float().cpu().numpy().reshape(nb, nz, ny, 2, nx, 8))
+    assert (np.abs(got - want) <= bar).all(), (np.abs(got - want) / bar).max()
+
+
 def _net_and_params(hp, seed=3):
     net = hp.Unet(seed)
     p = net.get_params().astype(np.float64)
