@@ -50,6 +50,7 @@ struct hpccg_unet {
   float *flip[kNumLayers][2] = {};  // FP32 flipped weights for CUDA-core backward-data
   float *partial = nullptr;         // gradient partials
   int partial_blocks = 0;
+  float *loss_partial = nullptr;  // [8 * num_sms]
   int *d_err = nullptr;
   // activations for the current shape
   int nx = 0, ny = 0, nz = 0, nb = 0;
@@ -59,9 +60,10 @@ struct hpccg_unet {
   __nv_bfloat16 *d1 = nullptr, *e2a = nullptr, *e2b = nullptr, *u2 = nullptr, *c2a = nullptr, *c2b = nullptr;
   __nv_bfloat16 *d2 = nullptr, *e3a = nullptr, *e3b = nullptr, *u3 = nullptr, *c3a = nullptr, *c3b = nullptr;
   __nv_bfloat16 *d3 = nullptr, *e4a = nullptr, *e4b = nullptr;
-  // backward buffers (FP32 gradients per level, BF16 masked pre-activation gradients)
-  float *g[4] = {}, *gs[4] = {}, *gt[4] = {};
-  __nv_bfloat16 *pre[4] = {};
+  // backward buffers per level: FP32 gradients of a skip tensor and of a resampled
+  // one, and two masked pre-activation gradients in BF16
+  float *gs[4] = {}, *gt[4] = {};
+  __nv_bfloat16 *pre[4] = {}, *pre2[4] = {};
   float *out_train = nullptr, *dout = nullptr;
   int loss_kind = 0;  // 0 = mean squared error, 1 = energy norm of the HPCCG operator
   std::vector<void *> act_allocs;
@@ -112,10 +114,10 @@ static int ensure_shape(hpccg_unet *u, int nx, int ny, int nz, int nb, bool trai
     if ((rc = alloc_act(u, &u->c1, c0))) return rc;
     for (int l = 0; l < 4; ++l) {
       const int64_t c = u->L[l].nvox * 16;
-      if ((rc = alloc_act(u, &u->g[l], c))) return rc;
-      if ((rc = alloc_act(u, &u->gs[l], c))) return rc;
+      if (l < 3 && (rc = alloc_act(u, &u->gs[l], c))) return rc;
       if ((rc = alloc_act(u, &u->gt[l], c))) return rc;
       if ((rc = alloc_act(u, &u->pre[l], c))) return rc;
+      if ((rc = alloc_act(u, &u->pre2[l], c))) return rc;
     }
     if ((rc = alloc_act(u, &u->out_train, u->L[0].nvox))) return rc;
     if ((rc = alloc_act(u, &u->dout, u->L[0].nvox))) return rc;
@@ -148,7 +150,7 @@ static int repack(hpccg_unet *u) {
 // CUDA cores otherwise.  `bwd_group` >= 0 selects the backward-data conv of
 // that input group (input in0 = the 16-channel pre-activation gradient).
 static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, const __nv_bfloat16 *in1,
-                const float *in_f32, int epi, void *out, int bwd_group = -1) {
+                const float *in_f32, int epi, void *out, int bwd_group = -1, const __nv_bfloat16 *act = nullptr) {
   const LayerDef &d = kLayers[layer];
   const Level &Lv = u->L[level];
   const float *W = u->params + u->off[layer];
@@ -164,6 +166,7 @@ static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, c
     a.wpack = bwd_group >= 0 ? u->packed_bwd[layer][bwd_group] : u->packed_fwd[layer];
     a.bias = bwd_group >= 0 ? nullptr : bias;
     a.proj = proj;
+    a.act = act;
     a.out = out;
     a.err = u->d_err;
     return launch_conv3_win(nin, epi, a, u->num_sms, u->stream);
@@ -192,6 +195,7 @@ static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, c
   a.W = bwd_group >= 0 ? u->flip[layer][bwd_group] : W;
   a.bias = bwd_group >= 0 ? nullptr : bias;
   a.proj = proj;
+  a.act = act;
   a.epi = epi;
   a.out = out;
   return launch_conv3_cc(a, u->num_sms, u->stream);
@@ -259,73 +263,65 @@ static int weight_grad(hpccg_unet *u, int layer, int level, const __nv_bfloat16 
   return HPCCG_OK;
 }
 
-static void mask(hpccg_unet *u, int level, const float *gsrc, const __nv_bfloat16 *act, __nv_bfloat16 *dst) {
-  const int64_t n = u->L[level].nvox * 16;
-  k_relu_mask<<<grid1d(u, n), 256, 0, u->stream>>>(gsrc, act, dst, n);
-}
-
-// Backward pass from u->dout (dL/dout), accumulating into u->grads.
+// Backward pass from u->dout (dL/dout), accumulating into u->grads.  `pre` and
+// `pre2` take turns: a conv reads one masked gradient and writes the next layer's.
 static int backward(hpccg_unet *u, const float *in) {
   const Level *L = u->L;
   const int nb = u->nb;
   cudaStream_t s = u->stream;
+  auto up_bwd = [&](int l, const __nv_bfloat16 *act) {  // gt[l - 1] -> pre[l]
+    k_up_bwd<<<grid1d(u, L[l].nvox * 2), 256, 0, s>>>(u->gt[l - 1], act, u->pre[l], L[l - 1].nx, L[l - 1].ny,
+                                                      L[l - 1].nz, nb);
+  };
+  auto pool_bwd = [&](int l, const __nv_bfloat16 *act) {  // gt[l + 1], gs[l] -> pre[l]
+    k_pool_bwd<<<grid1d(u, L[l].nvox * 2), 256, 0, s>>>(u->gt[l + 1], u->gs[l], act, u->pre[l], L[l].nx, L[l].ny,
+                                                        L[l].nz, nb);
+  };
   // projection and dec1a (level 0)
-  const int pb = (int)std::min<int64_t>(u->partial_blocks, (L[0].nvox + 255) / 256);
+  const int pb = (int)std::min<int64_t>(u->num_sms * 4, (L[0].nvox + 255) / 256);
   k_proj_bwd<<<pb, 256, 0, s>>>(u->c1, u->params + u->off[kNumLayers], u->dout, u->pre[0], u->partial, L[0].nvox,
                                 L[0].nx);
   k_reduce_partials<<<1, 256, 0, s>>>(u->partial, pb, 17, u->grads + u->off[kNumLayers], 1);
   UNET_TRY(weight_grad(u, 12, 0, u->e1b, u->u1, nullptr, u->pre[0]));
   UNET_TRY(conv(u, 12, 0, u->pre[0], nullptr, nullptr, kEpiRawF32, u->gs[0], 0));  // d e1b (skip)
   UNET_TRY(conv(u, 12, 0, u->pre[0], nullptr, nullptr, kEpiRawF32, u->gt[0], 1));  // d u1
-  k_up_bwd<<<grid1d(u, L[1].nvox * 16), 256, 0, s>>>(u->gt[0], u->g[1], L[0].nx, L[0].ny, L[0].nz, nb);
   // dec2b, dec2a (level 1)
-  mask(u, 1, u->g[1], u->c2b, u->pre[1]);
+  up_bwd(1, u->c2b);
   UNET_TRY(weight_grad(u, 11, 1, u->c2a, nullptr, nullptr, u->pre[1]));
-  UNET_TRY(conv(u, 11, 1, u->pre[1], nullptr, nullptr, kEpiRawF32, u->g[1], 0));
-  mask(u, 1, u->g[1], u->c2a, u->pre[1]);
-  UNET_TRY(weight_grad(u, 10, 1, u->e2b, u->u2, nullptr, u->pre[1]));
-  UNET_TRY(conv(u, 10, 1, u->pre[1], nullptr, nullptr, kEpiRawF32, u->gs[1], 0));  // d e2b (skip)
-  UNET_TRY(conv(u, 10, 1, u->pre[1], nullptr, nullptr, kEpiRawF32, u->gt[1], 1));  // d u2
-  k_up_bwd<<<grid1d(u, L[2].nvox * 16), 256, 0, s>>>(u->gt[1], u->g[2], L[1].nx, L[1].ny, L[1].nz, nb);
+  UNET_TRY(conv(u, 11, 1, u->pre[1], nullptr, nullptr, kEpiMask, u->pre2[1], 0, u->c2a));
+  UNET_TRY(weight_grad(u, 10, 1, u->e2b, u->u2, nullptr, u->pre2[1]));
+  UNET_TRY(conv(u, 10, 1, u->pre2[1], nullptr, nullptr, kEpiRawF32, u->gs[1], 0));  // d e2b (skip)
+  UNET_TRY(conv(u, 10, 1, u->pre2[1], nullptr, nullptr, kEpiRawF32, u->gt[1], 1));  // d u2
   // dec3b, dec3a (level 2)
-  mask(u, 2, u->g[2], u->c3b, u->pre[2]);
+  up_bwd(2, u->c3b);
   UNET_TRY(weight_grad(u, 9, 2, u->c3a, nullptr, nullptr, u->pre[2]));
-  UNET_TRY(conv(u, 9, 2, u->pre[2], nullptr, nullptr, kEpiRawF32, u->g[2], 0));
-  mask(u, 2, u->g[2], u->c3a, u->pre[2]);
-  UNET_TRY(weight_grad(u, 8, 2, u->e3b, u->u3, nullptr, u->pre[2]));
-  UNET_TRY(conv(u, 8, 2, u->pre[2], nullptr, nullptr, kEpiRawF32, u->gs[2], 0));  // d e3b (skip)
-  UNET_TRY(conv(u, 8, 2, u->pre[2], nullptr, nullptr, kEpiRawF32, u->gt[2], 1));  // d u3
-  k_up_bwd<<<grid1d(u, L[3].nvox * 16), 256, 0, s>>>(u->gt[2], u->g[3], L[2].nx, L[2].ny, L[2].nz, nb);
+  UNET_TRY(conv(u, 9, 2, u->pre[2], nullptr, nullptr, kEpiMask, u->pre2[2], 0, u->c3a));
+  UNET_TRY(weight_grad(u, 8, 2, u->e3b, u->u3, nullptr, u->pre2[2]));
+  UNET_TRY(conv(u, 8, 2, u->pre2[2], nullptr, nullptr, kEpiRawF32, u->gs[2], 0));  // d e3b (skip)
+  UNET_TRY(conv(u, 8, 2, u->pre2[2], nullptr, nullptr, kEpiRawF32, u->gt[2], 1));  // d u3
   // enc4b, enc4a (level 3)
-  mask(u, 3, u->g[3], u->e4b, u->pre[3]);
+  up_bwd(3, u->e4b);
   UNET_TRY(weight_grad(u, 7, 3, u->e4a, nullptr, nullptr, u->pre[3]));
-  UNET_TRY(conv(u, 7, 3, u->pre[3], nullptr, nullptr, kEpiRawF32, u->g[3], 0));
-  mask(u, 3, u->g[3], u->e4a, u->pre[3]);
-  UNET_TRY(weight_grad(u, 6, 3, u->d3, nullptr, nullptr, u->pre[3]));
-  UNET_TRY(conv(u, 6, 3, u->pre[3], nullptr, nullptr, kEpiRawF32, u->g[3], 0));  // d d3
-  k_pool_bwd<<<grid1d(u, L[2].nvox * 16), 256, 0, s>>>(u->g[3], u->gs[2], L[2].nx, L[2].ny, L[2].nz, nb);
+  UNET_TRY(conv(u, 7, 3, u->pre[3], nullptr, nullptr, kEpiMask, u->pre2[3], 0, u->e4a));
+  UNET_TRY(weight_grad(u, 6, 3, u->d3, nullptr, nullptr, u->pre2[3]));
+  UNET_TRY(conv(u, 6, 3, u->pre2[3], nullptr, nullptr, kEpiRawF32, u->gt[3], 0));  // d d3
   // enc3b, enc3a (level 2)
-  mask(u, 2, u->gs[2], u->e3b, u->pre[2]);
+  pool_bwd(2, u->e3b);
   UNET_TRY(weight_grad(u, 5, 2, u->e3a, nullptr, nullptr, u->pre[2]));
-  UNET_TRY(conv(u, 5, 2, u->pre[2], nullptr, nullptr, kEpiRawF32, u->g[2], 0));
-  mask(u, 2, u->g[2], u->e3a, u->pre[2]);
-  UNET_TRY(weight_grad(u, 4, 2, u->d2, nullptr, nullptr, u->pre[2]));
-  UNET_TRY(conv(u, 4, 2, u->pre[2], nullptr, nullptr, kEpiRawF32, u->g[2], 0));  // d d2
-  k_pool_bwd<<<grid1d(u, L[1].nvox * 16), 256, 0, s>>>(u->g[2], u->gs[1], L[1].nx, L[1].ny, L[1].nz, nb);
+  UNET_TRY(conv(u, 5, 2, u->pre[2], nullptr, nullptr, kEpiMask, u->pre2[2], 0, u->e3a));
+  UNET_TRY(weight_grad(u, 4, 2, u->d2, nullptr, nullptr, u->pre2[2]));
+  UNET_TRY(conv(u, 4, 2, u->pre2[2], nullptr, nullptr, kEpiRawF32, u->gt[2], 0));  // d d2
   // enc2b, enc2a (level 1)
-  mask(u, 1, u->gs[1], u->e2b, u->pre[1]);
+  pool_bwd(1, u->e2b);
   UNET_TRY(weight_grad(u, 3, 1, u->e2a, nullptr, nullptr, u->pre[1]));
-  UNET_TRY(conv(u, 3, 1, u->pre[1], nullptr, nullptr, kEpiRawF32, u->g[1], 0));
-  mask(u, 1, u->g[1], u->e2a, u->pre[1]);
-  UNET_TRY(weight_grad(u, 2, 1, u->d1, nullptr, nullptr, u->pre[1]));
-  UNET_TRY(conv(u, 2, 1, u->pre[1], nullptr, nullptr, kEpiRawF32, u->g[1], 0));  // d d1
-  k_pool_bwd<<<grid1d(u, L[0].nvox * 16), 256, 0, s>>>(u->g[1], u->gs[0], L[0].nx, L[0].ny, L[0].nz, nb);
+  UNET_TRY(conv(u, 3, 1, u->pre[1], nullptr, nullptr, kEpiMask, u->pre2[1], 0, u->e2a));
+  UNET_TRY(weight_grad(u, 2, 1, u->d1, nullptr, nullptr, u->pre2[1]));
+  UNET_TRY(conv(u, 2, 1, u->pre2[1], nullptr, nullptr, kEpiRawF32, u->gt[1], 0));  // d d1
   // enc1b, enc1a (level 0)
-  mask(u, 0, u->gs[0], u->e1b, u->pre[0]);
+  pool_bwd(0, u->e1b);
   UNET_TRY(weight_grad(u, 1, 0, u->e1a, nullptr, nullptr, u->pre[0]));
-  UNET_TRY(conv(u, 1, 0, u->pre[0], nullptr, nullptr, kEpiRawF32, u->g[0], 0));
-  mask(u, 0, u->g[0], u->e1a, u->pre[0]);
-  UNET_TRY(weight_grad(u, 0, 0, nullptr, nullptr, in, u->pre[0]));
+  UNET_TRY(conv(u, 1, 0, u->pre[0], nullptr, nullptr, kEpiMask, u->pre2[0], 0, u->e1a));
+  UNET_TRY(weight_grad(u, 0, 0, nullptr, nullptr, in, u->pre2[0]));
   HPCCG_CUDA(cudaGetLastError());
   return HPCCG_OK;
 }
@@ -360,7 +356,7 @@ static double u_pm1(uint64_t seed, uint64_t i) {
 extern "C" void hpccg_unet_destroy(hpccg_unet *u) {
   if (!u) return;
   free_acts(u);
-  void *bufs[] = {u->params, u->grads, u->adam_m, u->adam_v, u->partial, u->d_err};
+  void *bufs[] = {u->params, u->grads, u->adam_m, u->adam_v, u->loss_partial, u->partial, u->d_err};
   for (void *p : bufs)
     if (p) cudaFree(p);
   for (int l = 0; l < kNumLayers; ++l) {
@@ -427,7 +423,8 @@ extern "C" int hpccg_unet_create(uint64_t seed, hpccg_unet **out) {
         return fail(HPCCG_ERR_OOM);
   }
   u->partial_blocks = u->num_sms * 2;
-  if (cudaMalloc(&u->partial, sizeof(float) * (size_t)u->partial_blocks * (27 * 32 + 1) * 16))
+  if (cudaMalloc(&u->loss_partial, sizeof(float) * (size_t)u->num_sms * 8) ||
+      cudaMalloc(&u->partial, sizeof(float) * (size_t)u->partial_blocks * (27 * 32 + 1) * 16))
     return fail(HPCCG_ERR_OOM);
   int rc = repack(u);
   if (!rc && cudaStreamSynchronize(u->stream) != cudaSuccess) rc = HPCCG_ERR_CUDA;
@@ -475,22 +472,23 @@ extern "C" int hpccg_unet_loss_grad(hpccg_unet *u, int32_t nx, int32_t ny, int32
   HPCCG_CUDA(cudaMemsetAsync(u->grads, 0, sizeof(float) * u->nparams, u->stream));
   if ((rc = forward(u, d_in, u->out_train, true))) return rc;
   const int64_t n = u->L[0].nvox;
-  const int mb = std::min(u->partial_blocks, grid1d(u, n));
+  const int mb = std::min(u->num_sms * 8, grid1d(u, u->loss_kind == 1 ? n / 4 : n));
   if (u->loss_kind == 1)
-    k_energy<<<mb, 256, 0, u->stream>>>(u->out_train, d_target, u->dout, u->partial, nx, ny, nz, nb);
+    k_energy<<<mb, 256, 0, u->stream>>>(u->out_train, d_target, u->dout, u->loss_partial, nx, ny, nz, nb);
   else
-    k_mse<<<mb, 256, 0, u->stream>>>(u->out_train, d_target, u->dout, u->partial, n);
-  std::vector<float> lp(mb);
-  HPCCG_CUDA(cudaMemcpyAsync(lp.data(), u->partial, sizeof(float) * mb, cudaMemcpyDeviceToHost, u->stream));
-  HPCCG_CUDA(cudaStreamSynchronize(u->stream));
-  double l = 0.0;
-  for (float v : lp) l += v;
-  if (loss) *loss = (float)(l / (double)n);
+    k_mse<<<mb, 256, 0, u->stream>>>(u->out_train, d_target, u->dout, u->loss_partial, n);
   if ((rc = backward(u, d_in))) return rc;
+  // read after the backward pass: nothing on the host waits between the two
+  std::vector<float> lp(mb);
+  HPCCG_CUDA(cudaMemcpyAsync(lp.data(), u->loss_partial, sizeof(float) * mb, cudaMemcpyDeviceToHost, u->stream));
   if (grad_host) {
     HPCCG_CUDA(cudaMemcpyAsync(grad_host, u->grads, sizeof(float) * u->nparams, cudaMemcpyDeviceToHost, u->stream));
   }
-  return check_err(u);
+  rc = check_err(u);
+  double l = 0.0;
+  for (float v : lp) l += v;
+  if (loss) *loss = (float)(l / (double)n);
+  return rc;
 }
 
 extern "C" int hpccg_unet_set_loss(hpccg_unet *u, int32_t kind) {
@@ -589,6 +587,7 @@ extern "C" int hpccg_unet_conv3_layer(int32_t nx, int32_t ny, int32_t nz, int32_
     a.wpack = packed;
     a.bias = d_bias;
     a.proj = d_proj;
+    a.act = nullptr;
     a.out = d_out;
     a.err = d_err;
     rc = path == 2 ? launch_conv3_brick(nin, epi, a, sms, 0) : launch_conv3_win(nin, epi, a, sms, 0);
@@ -606,6 +605,7 @@ extern "C" int hpccg_unet_conv3_layer(int32_t nx, int32_t ny, int32_t nz, int32_
     a.W = d_w;
     a.bias = d_bias;
     a.proj = d_proj;
+    a.act = nullptr;
     a.epi = epi;
     a.out = d_out;
     rc = launch_conv3_cc(a, sms, 0);

@@ -50,6 +50,7 @@ enum ConvEpi : int {
   kEpiBias = 1,       // out_bf16 = acc + bias
   kEpiProject = 2,    // out_f32[voxel] = proj . relu(acc + bias) + proj_bias
   kEpiRawF32 = 3,     // out_f32 = acc (16 channels, row-planar)
+  kEpiMask = 4,       // out_bf16 = act > 0 ? acc : 0, act as wide as out (backward of a ReLU; one input group)
 };
 
 struct ConvGeom {
@@ -65,9 +66,15 @@ struct ConvArgs {
   const __nv_bfloat16 *wpack;      // [nin][27][2][16][8] BF16
   const float *bias;               // [16] (null for kEpiRawF32)
   const float *proj;               // [17] for kEpiProject
+  const __nv_bfloat16 *act;        // for kEpiMask
   void *out;
   int *err;
 };
+
+// Two BF16 gradients where the activations' pair is positive, zeros elsewhere.
+__device__ __forceinline__ uint32_t relu_mask2(uint32_t grad, uint32_t act) {
+  return grad & __hgt2_mask(*reinterpret_cast<const __nv_bfloat162 *>(&act), __float2bfloat162_rn(0.f));
+}
 
 // Host: brick and tile counts for a volume (dims must be divisible by the brick).
 inline bool conv_geom(int nx, int ny, int nz, int nb, ConvGeom *g) {

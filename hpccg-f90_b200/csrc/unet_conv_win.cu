@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
       b0 = a.bias[lane & 15];
 #pragma unroll
       for (int c = 0; c < 17; ++c) proj[c] = a.proj[c];
-    } else if (EPI != kEpiRawF32 && a.bias) {
+      } else if (EPI != kEpiRawF32 && EPI != kEpiMask && a.bias) {
       b0 = a.bias[tr];
       b1 = a.bias[tr + 8];
     }
@@ -315,6 +315,21 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
             }
           } else {
             for (int c0 = 32 * part; c0 < p.nn; c0 += 64) {
+              uint32_t act[EPI == kEpiMask ? 4 : 1][2][2];  // all loads of the mask ahead of the sums
+              if constexpr (EPI == kEpiMask) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                  int ci = 0;
+                  const int x = c0 + 8 * i < p.nn ? column(c0 + 8 * i + tr, &ci) : -1;
+                  const uint32_t *m = reinterpret_cast<const uint32_t *>(a.act) +
+                                      act_unit(row0 + (int64_t)ci * p.sc, 0, w0.x0 + x, g.nx) * 4 + (lane & 3);
+#pragma unroll
+                  for (int gs = 0; gs < 2; ++gs)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h)
+                      act[i][gs][h] = x >= 0 && rok[gs] ? __ldg(m + ((int64_t)gs * p.sr * 2 + h) * g.nx * 4) : 0;
+                }
+              }
               uint32_t d[2][16];
               tmem_ld_16x256_x4(base + sub * p.nn + c0, d[0]);
               tmem_ld_16x256_x4(base + (16u << 16) + sub * p.nn + c0, d[1]);
@@ -348,13 +363,18 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                       const float bias = h ? b1 : b0;
-                      float lo = __uint_as_float(d[gs][4 * i + 2 * h]) + bias;
-                      float hi = __uint_as_float(d[gs][4 * i + 2 * h + 1]) + bias;
+                      float lo = __uint_as_float(d[gs][4 * i + 2 * h]);
+                      float hi = __uint_as_float(d[gs][4 * i + 2 * h + 1]);
+                      if (EPI != kEpiMask) {
+                        lo += bias;
+                        hi += bias;
+                      }
                       if (EPI == kEpiBiasRelu) {
                         lo = fmaxf(lo, 0.f);
                         hi = fmaxf(hi, 0.f);
                       }
-                      const uint32_t v = transpose8x8(pack2(lo, hi));  // channels tc2, tc2+1 of half h, voxel tr
+                      uint32_t v = transpose8x8(pack2(lo, hi));  // channels tc2, tc2+1 of half h, voxel tr
+                      if constexpr (EPI == kEpiMask) v = relu_mask2(v, act[i][gs][h]);
                       if (x >= 0 && rok[gs]) o[((int64_t)gs * p.sr * 2 + h) * g.nx * 4] = v;
                     }
                 }
@@ -454,6 +474,7 @@ int launch_conv3_win(int nin, int epi, const ConvArgs &a, int num_sms, cudaStrea
       case kEpiBiasRelu: return launch_win<1, kEpiBiasRelu>(w, num_sms, s);
       case kEpiBias: return launch_win<1, kEpiBias>(w, num_sms, s);
       case kEpiProject: return launch_win<1, kEpiProject>(w, num_sms, s);
+      case kEpiMask: return launch_win<1, kEpiMask>(w, num_sms, s);
       default: return launch_win<1, kEpiRawF32>(w, num_sms, s);
     }
   }

@@ -238,89 +238,135 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__
 }
 
 // ---- the 1-channel FP32 input ----------------------------------------------------------
-// A block walks rows (b, z, y) in pieces of up to 128 voxels: the nine input
-// lines around the piece and its dY (as FP32) are staged in shared memory; a
-// thread owns one (dz, dy) line, four output channels and one of seven x
-// segments, and slides a three-voxel window along it: one input value and one
-// 16-byte dY quad feed 12 FMAs.  The seven segments' sums are added in order at
-// the end.  (A thread per tap
-// re-reading global memory 2.29 ms at 64^3, batch 4; this 0.12 ms, bound by the
-// shared-memory reads: 2 per 12 FMAs.)
-constexpr int kDwInThreads = 256;
-constexpr int kDwInX = 128, kDwInSeg = 7, kDwInPerSm = 6;
-constexpr int kDwInLine = kDwInX + 4;
+// A unit is 16 rows of y by up to 32 voxels of x at one z: its dY as FP32 and the
+// inputs around it (three z planes of 18 rows) are staged in shared memory.  A lane
+// owns a row and eight output channels, a warp the inputs of one dz and one half
+// of the voxels: a thread slides a 3 x 3 window along its row, so that three
+// inputs and two 16-byte dY quads feed 72 multiply-adds (paired, two channels an
+// instruction).  The rows of a warp and then the two halves of x are added up at
+// the end.  (Pieces of one row, each staging nine lines, four channels and three taps
+// a thread: 127 us at 64^3, batch 4; this 53 us, bound by the multiply-adds (14 us)
+// and by the staging between them, 12 warps an SM.)
+constexpr int kDwInThreads = 192;  // x half (2), dz (3), lane = row (16) x channel half (2)
+constexpr int kDwInX = 32, kDwInRows = 16, kDwInPerSm = 2;
+constexpr int kDwInLine = kDwInX + 3;                     // odd: the 16 rows of a warp in 16 banks
+constexpr int kDwInRow = kDwInX * 8 + 8;                  // dY: 8 channels a voxel; rows 8 banks apart,
+constexpr int kDwInHalf = kDwInRows * kDwInRow + 4;       // halves 4
+constexpr int kDwInSmem = (2 * kDwInHalf + 3 * (kDwInRows + 2) * kDwInLine) * (int)sizeof(float);
 
-__global__ void __launch_bounds__(kDwInThreads) k_dW_in1(DwArgs a) {
-  __shared__ __align__(16) float sin[9 * kDwInLine];
-  __shared__ __align__(16) float sdy[kDwInX * 16];
-  __shared__ float red[28 * 16];
+__global__ void __launch_bounds__(kDwInThreads, kDwInPerSm) k_dW_in1(DwArgs a, int xb) {
+  __shared__ __align__(16) float sm[kDwInSmem / sizeof(float)];
+  float *sdy = sm, *sin = sm + 2 * kDwInHalf;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
-  const int nxb = (nx + kDwInX - 1) / kDwInX;
-  const int64_t nrow = (int64_t)ny * nz * a.nb, nunit = nrow * nxb;
-  const int t = threadIdx.x, seg = t / 36, line = (t % 36) / 4, q = t & 3;
-  float acc[3][4], bs[4];
+  const int nxb = (nx + xb - 1) / xb, nyb = (ny + kDwInRows - 1) / kDwInRows;
+  const int64_t nunit = (int64_t)nxb * nyb * nz * a.nb;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, xh = warp / 3, dzi = warp % 3;
+  const int h = lane & 1, r = lane >> 1;
+  unsigned long long acc[9][4], bs[4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) acc[0][c] = acc[1][c] = acc[2][c] = bs[c] = 0.f;
+  for (int c = 0; c < 4; ++c) {
+    bs[c] = 0ull;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc[k][c] = 0ull;
+  }
   for (int64_t u = blockIdx.x; u < nunit; u += gridDim.x) {
-    const int64_t row = u / nxb;
-    const int x0 = (int)(u - row * nxb) * kDwInX, w = min(kDwInX, nx - x0);
-    const int y = (int)(row % ny), z = (int)(row / ny % nz);
-    __syncthreads();  // the previous piece has been read
-    for (int e = t; e < 9 * (kDwInX + 2); e += kDwInThreads) {
-      const int l = e / (kDwInX + 2), i = e - l * (kDwInX + 2), x = x0 + i - 1;
-      const int dz = l / 3 - 1, dy = l % 3 - 1;
-      const bool in = (unsigned)x < (unsigned)nx && (unsigned)(y + dy) < (unsigned)ny && (unsigned)(z + dz) < (unsigned)nz;
-      sin[l * kDwInLine + i] = in ? __ldg(a.x_f32 + (row + dz * ny + dy) * nx + x) : 0.f;
+    const int64_t p = u / nxb, plane = p / nyb;  // (b, z)
+    const int x0 = (int)(u - p * nxb) * xb, y0 = (int)(p - plane * nyb) * kDwInRows, z = (int)(plane % nz);
+    const int w = min(xb, nx - x0), rows = min(kDwInRows, ny - y0);
+    // all loads of the unit in flight before the first store
+    constexpr int kIn = 3 * (kDwInRows + 2) * (kDwInX + 2), kInN = (kIn + kDwInThreads - 1) / kDwInThreads;
+    constexpr int kDy = 2 * kDwInRows * kDwInX, kDyN = (kDy + kDwInThreads - 1) / kDwInThreads;
+    float iv[kInN];
+    uint4 dv[kDyN];
+#pragma unroll
+    for (int k = 0; k < kInN; ++k) {
+      const int e = t + k * kDwInThreads, l = e / (kDwInX + 2), i = e % (kDwInX + 2);
+      const int dz = l / (kDwInRows + 2) - 1, y = y0 + l % (kDwInRows + 2) - 1, x = x0 + i - 1;
+      iv[k] = e < kIn && i < w + 2 && (unsigned)x < (unsigned)nx && (unsigned)y < (unsigned)ny && (unsigned)(z + dz) < (unsigned)nz
+                  ? __ldg(a.x_f32 + ((plane + dz) * ny + y) * nx + x) : 0.f;
     }
-    for (int e = t; e < 2 * w; e += kDwInThreads) {
-      const int h = e / w, x = e - h * w;
-      const uint4 p = *reinterpret_cast<const uint4 *>(a.dy + act_unit(row, h, x0 + x, nx) * 8);
-      const __nv_bfloat162 *p2 = reinterpret_cast<const __nv_bfloat162 *>(&p);
-      const float2 f0 = __bfloat1622float2(p2[0]), f1 = __bfloat1622float2(p2[1]);
-      const float2 f2 = __bfloat1622float2(p2[2]), f3 = __bfloat1622float2(p2[3]);
-      float4 *d = reinterpret_cast<float4 *>(sdy + x * 16 + 8 * h);
-      d[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
-      d[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+#pragma unroll
+    for (int k = 0; k < kDyN; ++k) {
+      const int e = t + k * kDwInThreads, x = e % kDwInX, l = e / kDwInX;
+      if (x < w && l < 2 * rows)
+        dv[k] = __ldg(reinterpret_cast<const uint4 *>(a.dy) + act_unit(plane * ny + y0 + (l >> 1), l & 1, x0 + x, nx));
+    }
+    __syncthreads();  // the previous unit has been read
+#pragma unroll
+    for (int k = 0; k < kInN; ++k) {
+      const int e = t + k * kDwInThreads;
+      if (e < kIn) sin[e / (kDwInX + 2) * kDwInLine + e % (kDwInX + 2)] = iv[k];
+    }
+#pragma unroll
+    for (int k = 0; k < kDyN; ++k) {
+      const int e = t + k * kDwInThreads, x = e % kDwInX, l = e / kDwInX;
+      if (x < w && l < 2 * rows) {
+        const __nv_bfloat162 *p2 = reinterpret_cast<const __nv_bfloat162 *>(&dv[k]);
+        const float2 f0 = __bfloat1622float2(p2[0]), f1 = __bfloat1622float2(p2[1]);
+        const float2 f2 = __bfloat1622float2(p2[2]), f3 = __bfloat1622float2(p2[3]);
+        float4 *d = reinterpret_cast<float4 *>(sdy + (l & 1) * kDwInHalf + (l >> 1) * kDwInRow + x * 8);
+        d[0] = make_float4(f0.x, f0.y, f1.x, f1.y);
+        d[1] = make_float4(f2.x, f2.y, f3.x, f3.y);
+      }
     }
     __syncthreads();
-    if (seg < kDwInSeg) {
-      const int segx = (w + kDwInSeg - 1) / kDwInSeg, xa = seg * segx, xb = min(w, xa + segx);
-      if (xa < xb) {
-        const float *s = sin + line * kDwInLine;  // voxel x's taps: s[x], s[x + 1], s[x + 2]
-        float v0 = s[xa], v1 = s[xa + 1];
-        for (int x = xa; x < xb; ++x) {
-          const float v2 = s[x + 2];
-          const float4 d = *reinterpret_cast<const float4 *>(sdy + x * 16 + 4 * q);
-          const float dv[4] = {d.x, d.y, d.z, d.w};
+    const int xm = (w + 1) / 2, xa = xh ? xm : 0, xe = xh ? w : xm;
+    if (r < rows && xa < xe) {
+      const float *s = sin + (dzi * (kDwInRows + 2) + r) * kDwInLine;  // voxel x's taps: s[x], s[x + 1], s[x + 2]
+      const float *dy = sdy + h * kDwInHalf + r * kDwInRow;
+      unsigned long long v[3][3];
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            acc[0][c] = fmaf(v0, dv[c], acc[0][c]);
-            acc[1][c] = fmaf(v1, dv[c], acc[1][c]);
-            acc[2][c] = fmaf(v2, dv[c], acc[2][c]);
-            bs[c] += dv[c];
-          }
-          v0 = v1;
-          v1 = v2;
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) v[j][k] = pack_f32x2(s[j * kDwInLine + xa + k], s[j * kDwInLine + xa + k]);
+      for (int x = xa; x < xe; ++x) {
+        const ulonglong2 d0 = *reinterpret_cast<const ulonglong2 *>(dy + x * 8);
+        const ulonglong2 d1 = *reinterpret_cast<const ulonglong2 *>(dy + x * 8 + 4);
+        const unsigned long long d[4] = {d0.x, d0.y, d1.x, d1.y};
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float n = s[j * kDwInLine + x + 2];
+          v[j][2] = pack_f32x2(n, n);
+#pragma unroll
+          for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) fma_f32x2(acc[j * 3 + k][c], v[j][k], d[c]);
+          v[j][0] = v[j][1];
+          v[j][1] = v[j][2];
+        }
+        if (dzi == 1) {
+          const unsigned long long one = pack_f32x2(1.f, 1.f);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) fma_f32x2(bs[c], one, d[c]);
         }
       }
     }
   }
-  for (int s = 0; s < kDwInSeg; ++s) {  // the segments in order
+  // rows of the warp by shuffles, then the two x halves in order: red[tap][co], the bias as tap 27
+  float *red = sm;
+  auto finish = [&](int tap, const unsigned long long *v) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float lo, hi;
+      unpack_f32x2(v[c], lo, hi);
+#pragma unroll
+      for (int o = 2; o < 32; o <<= 1) {
+        lo += __shfl_xor_sync(0xffffffffu, lo, o);
+        hi += __shfl_xor_sync(0xffffffffu, hi, o);
+      }
+      if (lane < 2) {
+        float *d = red + tap * 16 + 8 * h + 2 * c;
+        d[0] = xh ? d[0] + lo : lo;
+        d[1] = xh ? d[1] + hi : hi;
+      }
+    }
+  };
+  for (int k = 0; k < 2; ++k) {
     __syncthreads();
-    if (seg == s) {
+    if (xh == k) {
 #pragma unroll
-      for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float *r = red + (line * 3 + dx) * 16 + 4 * q + c;
-          *r = s ? *r + acc[dx][c] : acc[dx][c];
-        }
-      if (line == 4)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float *r = red + 27 * 16 + 4 * q + c;
-          *r = s ? *r + bs[c] : bs[c];
-        }
+      for (int j = 0; j < 9; ++j) finish(dzi * 9 + j, acc[j]);
+      if (dzi == 1) finish(27, bs);
     }
   }
   __syncthreads();
@@ -330,10 +376,11 @@ __global__ void __launch_bounds__(kDwInThreads) k_dW_in1(DwArgs a) {
 // Partials of one layer's gradient (a.partial holds max_blocks of them); *blocks: how many.
 int launch_dW(const DwArgs &a, int max_blocks, int *err, int num_sms, cudaStream_t s, int *blocks) {
   if (a.x_f32) {
-    const int64_t units = (int64_t)a.ny * a.nz * a.nb * ((a.nx + kDwInX - 1) / kDwInX);
+    const int nxb = (a.nx + kDwInX - 1) / kDwInX, xb = (a.nx + nxb - 1) / nxb;
+    const int64_t units = (int64_t)((a.ny + kDwInRows - 1) / kDwInRows) * a.nz * a.nb * nxb;
     // its partials are 1/30 of a 32-channel layer's, which max_blocks counts
     *blocks = (int)std::min<int64_t>(std::min(30 * max_blocks, kDwInPerSm * num_sms), units);
-    k_dW_in1<<<*blocks, kDwInThreads, 0, s>>>(a);
+    k_dW_in1<<<*blocks, kDwInThreads, 0, s>>>(a, xb);
     HPCCG_CUDA(cudaGetLastError());
     return HPCCG_OK;
   }

@@ -50,18 +50,6 @@ __global__ void k_flip_fp32(const float *W, int cin, int g, float *Wf) {
 // 8.4 ms, 96^3 4.30 -> 1.36, 24^3 1.41 -> 0.27.  Bound by the FP32 pipe on large volumes
 // (6912 multiply-adds a voxel and group: 226 G of them at 192^3, 7.8 ms, 80% of its
 // rate), by the latency of the 27 taps on small ones.
-__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack_f32x2(unsigned long long v, float &lo, float &hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ void fma_f32x2(unsigned long long &d, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-
 // One tap and input group of N voxels: q = their 16 channels, w = the weights [16 ci][16 co]
 // from the thread's first channel on.
 template <int N, int CO>
@@ -164,19 +152,26 @@ __global__ void __launch_bounds__(kCcThreads, cc_blocks<V, CO>()) k_conv3_cc(CcC
         __nv_bfloat16 *dst = static_cast<__nv_bfloat16 *>(a.out);
 #pragma unroll
         for (int c = 0; c < CO; c += 4) {
+          const int64_t at = act_elem(row + v, x, c0 + c, nx);
           uint32_t p[2];
 #pragma unroll
           for (int k = 0; k < 2; ++k) {
             float f[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-              f[j] = o[c + 2 * k + j] + (a.bias ? a.bias[c0 + c + 2 * k + j] : 0.f);
+              f[j] = o[c + 2 * k + j];
+              if (a.bias) f[j] += a.bias[c0 + c + 2 * k + j];
               if (a.epi == kEpiBiasRelu) f[j] = fmaxf(f[j], 0.f);
             }
             const __nv_bfloat162 b = __floats2bfloat162_rn(f[0], f[1]);
             p[k] = *reinterpret_cast<const uint32_t *>(&b);
           }
-          *reinterpret_cast<uint2 *>(dst + act_elem(row + v, x, c0 + c, nx)) = make_uint2(p[0], p[1]);
+          if (a.epi == kEpiMask) {
+            const uint2 m = __ldg(reinterpret_cast<const uint2 *>(a.act + at));
+            p[0] = relu_mask2(p[0], m.x);
+            p[1] = relu_mask2(p[1], m.y);
+          }
+          *reinterpret_cast<uint2 *>(dst + at) = make_uint2(p[0], p[1]);
         }
       }
     }
@@ -376,43 +371,72 @@ __global__ void k_upsample(const __nv_bfloat16 *in, __nv_bfloat16 *out, int nx, 
     }
   }
 }
-// Backward of pooling: d_fine += d_coarse / 8 (FP32 row-planar tensors).
-__global__ void k_pool_bwd(const float *dc, float *df, int nx, int ny, int nz, int nb) {
+// Backward of pooling, of the skip connection beside it and of the ReLU before
+// both: out = act > 0 ? skip + d_coarse / 8 : 0 in BF16 (skip and d_coarse FP32
+// row-planar).  One thread per 16-byte unit of out.  One pass over the three
+// tensors where a pass each for the sum and the mask, a float a thread, took
+// 144 us at 64^3, batch 4; 22 us here.
+__global__ void k_pool_bwd(const float *dc, const float *skip, const __nv_bfloat16 *act, __nv_bfloat16 *out, int nx,
+                           int ny, int nz, int nb) {
   const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
-  const int64_t n = (int64_t)nx * ny * nz * nb * 16;
+  const int64_t n = (int64_t)nx * ny * nz * nb * 2;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t row, b;
     int h, x, z, y;
-    unit_coords(e >> 3, nx, &row, &h, &x);
+    unit_coords(e, nx, &row, &h, &x);
     row_coords(row, ny, nz, &b, &z, &y);
-    df[e] += 0.125f * dc[act_unit((b * cz + z / 2) * cy + y / 2, h, x / 2, cx) * 8 + (e & 7)];
+    const float4 *c4 = reinterpret_cast<const float4 *>(dc) + 2 * act_unit((b * cz + z / 2) * cy + y / 2, h, x / 2, cx);
+    const float4 *s4 = reinterpret_cast<const float4 *>(skip) + 2 * e;
+    const uint4 m = __ldg(reinterpret_cast<const uint4 *>(act) + e);
+    const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const float4 c = __ldg(c4 + k), f = __ldg(s4 + k);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(fmaf(0.125f, c.x, f.x), fmaf(0.125f, c.y, f.y));
+      const __nv_bfloat162 hi = __floats2bfloat162_rn(fmaf(0.125f, c.z, f.z), fmaf(0.125f, c.w, f.w));
+      o[2 * k] = relu_mask2(*reinterpret_cast<const uint32_t *>(&lo), mw[2 * k]);
+      o[2 * k + 1] = relu_mask2(*reinterpret_cast<const uint32_t *>(&hi), mw[2 * k + 1]);
+    }
+    reinterpret_cast<uint4 *>(out)[e] = make_uint4(o[0], o[1], o[2], o[3]);
   }
 }
-// Backward of nearest upsampling: d_coarse = sum of the 8 fine children.
-__global__ void k_up_bwd(const float *df, float *dc, int nx, int ny, int nz, int nb) {
+// Backward of nearest upsampling and of the ReLU before it: out = act > 0 ? the
+// sum of the 8 fine children : 0 in BF16.  One thread per 16-byte unit of out.
+__global__ void k_up_bwd(const float *df, const __nv_bfloat16 *act, __nv_bfloat16 *out, int nx, int ny, int nz,
+                         int nb) {
   const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
-  const int64_t n = (int64_t)cx * cy * cz * nb * 16;
+  const int64_t n = (int64_t)cx * cy * cz * nb * 2;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
     int64_t row, b;
     int h, xc, zc, yc;
-    unit_coords(e >> 3, cx, &row, &h, &xc);
+    unit_coords(e, cx, &row, &h, &xc);
     row_coords(row, cy, cz, &b, &zc, &yc);
-    float s = 0.f;
+    const uint4 m = __ldg(reinterpret_cast<const uint4 *>(act) + e);
+    float4 s[2] = {};
+#pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int64_t rf = (b * nz + 2 * zc + (k >> 2)) * ny + 2 * yc + ((k >> 1) & 1);
-      s += df[act_unit(rf, h, 2 * xc + (k & 1), nx) * 8 + (e & 7)];
+      const float4 *f4 = reinterpret_cast<const float4 *>(df) + 2 * act_unit(rf, h, 2 * xc + (k & 1), nx);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float4 f = __ldg(f4 + j);
+        s[j].x += f.x;
+        s[j].y += f.y;
+        s[j].z += f.z;
+        s[j].w += f.w;
+      }
     }
-    dc[e] = s;
+    const uint32_t mw[4] = {m.x, m.y, m.z, m.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(s[j].x, s[j].y), hi = __floats2bfloat162_rn(s[j].z, s[j].w);
+      o[2 * j] = relu_mask2(*reinterpret_cast<const uint32_t *>(&lo), mw[2 * j]);
+      o[2 * j + 1] = relu_mask2(*reinterpret_cast<const uint32_t *>(&hi), mw[2 * j + 1]);
+    }
+    reinterpret_cast<uint4 *>(out)[e] = make_uint4(o[0], o[1], o[2], o[3]);
   }
-}
-// dpre = d * (act > 0), to BF16 (the next backward conv's input) and optionally FP32.
-__global__ void k_relu_mask(const float *d, const __nv_bfloat16 *act, __nv_bfloat16 *out, int64_t n) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
-    out[e] = __float2bfloat16(__bfloat162float(act[e]) > 0.f ? d[e] : 0.f);
-}
-__global__ void k_add_f32(const float *src, float *dst, int64_t n) {
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x)
-    dst[e] += src[e];
 }
 
 // ---- gradients --------------------------------------------------------------------------------
@@ -435,17 +459,39 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const float *partial, i
   }
 }
 
+// The 16 channels of a voxel as floats.
+__device__ __forceinline__ void load_voxel(const __nv_bfloat16 *act, int64_t unit0, int nx, float *f) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(act) + unit0 + (int64_t)h * nx);
+    const __nv_bfloat162 *p2 = reinterpret_cast<const __nv_bfloat162 *>(&q);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float2 t = __bfloat1622float2(p2[c]);
+      f[8 * h + 2 * c] = t.x;
+      f[8 * h + 2 * c + 1] = t.y;
+    }
+  }
+}
+// Voxel index -> unit of its first half.
+__device__ __forceinline__ int64_t voxel_unit(int64_t v, int nx) {
+  const int64_t row = (uint64_t)v <= 0xFFFFFFFFull ? (int64_t)((uint32_t)v / (uint32_t)nx) : v / nx;
+  return act_unit(row, 0, (int)(v - row * nx), nx);
+}
+
 // Output projection (training path): out[v] = proj . act[v] + proj_b.
 __global__ void k_proj_fwd(const __nv_bfloat16 *act, const float *proj, float *out, int64_t nvox, int nx) {
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nvox; v += (int64_t)gridDim.x * blockDim.x) {
-    float r = proj[16];
+    float f[16], r = proj[16];
+    load_voxel(act, voxel_unit(v, nx), nx, f);
 #pragma unroll
-    for (int c = 0; c < 16; ++c) r = fmaf(proj[c], __bfloat162float(act[act_elem(v / nx, (int)(v % nx), c, nx)]), r);
+    for (int c = 0; c < 16; ++c) r = fmaf(proj[c], f[c], r);
     out[v] = r;
   }
 }
 // d act = proj * dOut (masked by act > 0, to BF16); per-block partials of
 // dproj[c] = sum act[v][c] dOut[v] and dproj_b = sum dOut[v] ([block][17]).
+// 16-byte units in and out (one element at a time: 56 us at 64^3, batch 4; 16 us here).
 __global__ void __launch_bounds__(256) k_proj_bwd(const __nv_bfloat16 *act, const float *proj, const float *dout,
                                                   __nv_bfloat16 *dact, float *partial, int64_t nvox, int nx) {
   __shared__ float red[17][256];
@@ -454,14 +500,25 @@ __global__ void __launch_bounds__(256) k_proj_bwd(const __nv_bfloat16 *act, cons
   for (int c = 0; c < 17; ++c) acc[c] = 0.f;
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nvox; v += (int64_t)gridDim.x * blockDim.x) {
     const float d = dout[v];
-    const int64_t row = v / nx;
-    const int x = (int)(v % nx);
+    const int64_t u = voxel_unit(v, nx);
+    float f[16];
+    load_voxel(act, u, nx, f);
 #pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      const int64_t e = act_elem(row, x, c, nx);
-      const float av = __bfloat162float(act[e]);
-      acc[c] = fmaf(av, d, acc[c]);
-      dact[e] = __float2bfloat16(av > 0.f ? proj[c] * d : 0.f);
+    for (int h = 0; h < 2; ++h) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float o[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const int c = 8 * h + 2 * k + j;
+          acc[c] = fmaf(f[c], d, acc[c]);
+          o[j] = f[c] > 0.f ? proj[c] * d : 0.f;
+        }
+        const __nv_bfloat162 b = __floats2bfloat162_rn(o[0], o[1]);
+        w[k] = *reinterpret_cast<const uint32_t *>(&b);
+      }
+      reinterpret_cast<uint4 *>(dact)[u + (int64_t)h * nx] = make_uint4(w[0], w[1], w[2], w[3]);
     }
     acc[16] += d;
   }
@@ -496,28 +553,57 @@ __global__ void __launch_bounds__(256) k_mse(const float *out, const float *tgt,
   if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
 }
 
+// Four floats at p, which need not be 16-byte aligned.
+__device__ __forceinline__ float4 load4(const float *p) {
+  if (((uintptr_t)p & 15) == 0) return __ldg(reinterpret_cast<const float4 *>(p));
+  return make_float4(__ldg(p), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3));
+}
+
 // Energy-norm loss of the HPCCG operator A (the 27-point generate_matrix
 // stencil: 27 on the diagonal, -1 for each neighbour inside the grid):
 // L = (1/n) d.(A d), d = target - out, per grid of the batch; dL/dout = -(2/n) A d.
+// A thread forms four voxels of a row (nx a multiple of 4): per (dz, dy) line it
+// loads the six differences around them once, out-of-grid ones as zeros.  99 -> 18 us
+// at 64^3, batch 4, against a voxel a thread and 54 loads one by one.
 __global__ void __launch_bounds__(256) k_energy(const float *out, const float *tgt, float *dout, float *partial,
                                                 int nx, int ny, int nz, int nb) {
   __shared__ float red[256];
   const int64_t n = (int64_t)nx * ny * nz * nb;
   const float scale = 2.f / (float)n;
   float s = 0.f;
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < n; v += (int64_t)gridDim.x * blockDim.x) {
-    const int x = (int)(v % nx), y = (int)((v / nx) % ny), z = (int)((v / ((int64_t)nx * ny)) % nz);
-    const int64_t b = v / ((int64_t)nx * ny * nz);
-    float ad = 0.f;
-    for (int t = 0; t < 27; ++t) {
-      const int xx = x + t % 3 - 1, yy = y + (t / 3) % 3 - 1, zz = z + t / 9 - 1;
-      if (xx < 0 || xx >= nx || yy < 0 || yy >= ny || zz < 0 || zz >= nz) continue;
-      const int64_t u = ((b * nz + zz) * ny + yy) * nx + xx;
-      const float du = tgt[u] - out[u];
-      ad += (t == 13 ? 27.f : -1.f) * du;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n / 4; q += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t v = 4 * q, row = (uint64_t)v <= 0xFFFFFFFFull ? (int64_t)((uint32_t)v / (uint32_t)nx) : v / nx;
+    int64_t b;
+    int y, z;
+    const int x = (int)(v - row * nx);
+    row_coords(row, ny, nz, &b, &z, &y);
+    float ad[4] = {0.f, 0.f, 0.f, 0.f}, dc[4];
+#pragma unroll
+    for (int li = 0; li < 9; ++li) {
+      const int dy = li % 3 - 1, dz = li / 3 - 1;
+      const bool line = (unsigned)(y + dy) < (unsigned)ny && (unsigned)(z + dz) < (unsigned)nz;
+      const int64_t u = v + ((int64_t)dz * ny + dy) * nx;
+      float d[6];
+      d[0] = line && x > 0 ? __ldg(tgt + u - 1) - __ldg(out + u - 1) : 0.f;
+      d[5] = line && x + 4 < nx ? __ldg(tgt + u + 4) - __ldg(out + u + 4) : 0.f;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 t4 = line ? load4(tgt + u) : zero, o4 = line ? load4(out + u) : zero;
+      d[1] = t4.x - o4.x;
+      d[2] = t4.y - o4.y;
+      d[3] = t4.z - o4.z;
+      d[4] = t4.w - o4.w;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (li == 4) dc[j] = d[j + 1];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) ad[j] = fmaf(li == 4 && k == 1 ? 27.f : -1.f, d[j + k], ad[j]);
+      }
     }
-    s += (tgt[v] - out[v]) * ad;
-    dout[v] = -scale * ad;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      s = fmaf(dc[j], ad[j], s);
+      dout[v + j] = -scale * ad[j];
+    }
   }
   red[threadIdx.x] = s;
   __syncthreads();

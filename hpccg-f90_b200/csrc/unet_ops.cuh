@@ -11,6 +11,7 @@ struct CcConvArgs {
   const float *W;                    // FP32 [27][16 nin][16]
   const float *bias;                 // [16] or null
   const float *proj;                 // [17] for kEpiProject
+  const __nv_bfloat16 *act;          // for kEpiMask
   int epi;
   void *out;
 };
@@ -23,6 +24,19 @@ struct DwArgs {
   float *partial;                    // [gridDim.x][27*cin + 1][16]
 };
 
+// Two FP32 numbers in a register pair, and their fused multiply-add.
+__device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(unsigned long long v, float &lo, float &hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ void fma_f32x2(unsigned long long &d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
 __global__ void k_pack_fwd(const float *W, int cin, int nin, __nv_bfloat16 *packed);
 __global__ void k_pack_bwd(const float *W, int cin, int g, __nv_bfloat16 *packed);
 __global__ void k_flip_fp32(const float *W, int cin, int g, float *Wf);
@@ -33,10 +47,9 @@ __global__ void k_conv3_in1x4(const float *in, const float *W, const float *bias
                               int nz, int nb, int relu);  // nx a multiple of 4
 __global__ void k_pool(const __nv_bfloat16 *in, __nv_bfloat16 *out, int nx, int ny, int nz, int nb);
 __global__ void k_upsample(const __nv_bfloat16 *in, __nv_bfloat16 *out, int nx, int ny, int nz, int nb);
-__global__ void k_pool_bwd(const float *dc, float *df, int nx, int ny, int nz, int nb);
-__global__ void k_up_bwd(const float *df, float *dc, int nx, int ny, int nz, int nb);
-__global__ void k_relu_mask(const float *d, const __nv_bfloat16 *act, __nv_bfloat16 *out, int64_t n);
-__global__ void k_add_f32(const float *src, float *dst, int64_t n);
+__global__ void k_pool_bwd(const float *dc, const float *skip, const __nv_bfloat16 *act, __nv_bfloat16 *out, int nx,
+                           int ny, int nz, int nb);
+__global__ void k_up_bwd(const float *df, const __nv_bfloat16 *act, __nv_bfloat16 *out, int nx, int ny, int nz, int nb);
 __global__ void k_reduce_partials(const float *partial, int nblocks, int n, float *grad, int accumulate);
 __global__ void k_proj_fwd(const __nv_bfloat16 *act, const float *proj, float *out, int64_t nvox, int nx);
 __global__ void k_proj_bwd(const __nv_bfloat16 *act, const float *proj, const float *dout, __nv_bfloat16 *dact,

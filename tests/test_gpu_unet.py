@@ -241,6 +241,31 @@ def test_gradients_ragged_shapes(env, nx, ny, nz, nb):
         assert err <= 6e-2, (l, err)
 
 
+@pytest.mark.parametrize("nx,ny,nz,nb", [(8, 8, 8, 1), (40, 24, 8, 3), (72, 40, 16, 1), (64, 16, 16, 2)])
+def test_input_layer_and_energy_gradients_edges(env, nx, ny, nz, nb):
+    """The energy loss and the first layer's and the projection's gradients on grids with partial
+    row tiles and x blocks, target and input not 16-byte aligned.  Loss and projection read BF16
+    activations, the first layer's gradient has come through all layers: the bars of the 16^3 test."""
+    torch, hp = env
+    net, p = _net_and_params(hp, seed=5)
+    net.set_loss(1)
+    rng = np.random.default_rng(ny)
+    r = rng.normal(0, 1, (nb, nz, ny, nx))
+    t = rng.normal(0, 0.05, (nb, nz, ny, nx))
+    buf = torch.zeros(2 * r.size + 2, dtype=torch.float32, device="cuda")
+    din, dt = buf[1 : r.size + 1], buf[r.size + 1 : 2 * r.size + 1]
+    din.copy_(torch.from_numpy(r.astype(np.float32)).ravel())
+    dt.copy_(torch.from_numpy(t.astype(np.float32)).ravel())
+    loss_ref, g_ref = uo.loss_grad(p, r, t, kind=1)
+    loss, g = net.loss_grad(din, dt, nx, ny, nz, nb, want_grad=True)
+    assert loss == pytest.approx(loss_ref, rel=5e-2)
+    off, n = uo.offsets()
+    for l in (0, 13):
+        a, b = off[l], (off[l + 1] if l < 13 else n)
+        err = np.linalg.norm(g[a:b] - g_ref[a:b]) / (np.linalg.norm(g_ref[a:b]) + 1e-30)
+        assert err <= 6e-2, (l, err)
+
+
 def test_trained_network_reduces_fcg_iterations(env):
     """What the trained network gains: FCG iterations to FP64 rel-res 1e-8 on
     held-out Gaussian-random-field right-hand sides, against plain CG through
