@@ -169,6 +169,7 @@ static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, c
     a.act = act;
     a.out = out;
     a.err = u->d_err;
+    a.chained = true;
     return launch_conv3_win(nin, epi, a, u->num_sms, u->stream);
   }
   if (in_f32 && (epi == kEpiBiasRelu || epi == kEpiBias)) {  // the 1-channel input layer
@@ -198,6 +199,7 @@ static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, c
   a.act = act;
   a.epi = epi;
   a.out = out;
+  a.chained = true;
   return launch_conv3_cc(a, u->num_sms, u->stream);
 }
 
@@ -207,31 +209,37 @@ static int conv(hpccg_unet *u, int layer, int level, const __nv_bfloat16 *in0, c
     if (rc_) return rc_;         \
   } while (0)
 
+// A CUDA-core kernel of the chain, 256 threads a block.
+template <typename... P, typename... A>
+static int run(hpccg_unet *u, void (*kern)(P...), int grid, A... args) {
+  HPCCG_CUDA(launch_chained(kern, grid, 256, 0, u->stream, true, args...));
+  return HPCCG_OK;
+}
+
 // Forward pass.  train: store c1 and write the projection to u->out_train.
 static int forward(hpccg_unet *u, const float *in, float *out, bool train) {
   const Level *L = u->L;
   UNET_TRY(conv(u, 0, 0, nullptr, nullptr, in, kEpiBiasRelu, u->e1a));
   UNET_TRY(conv(u, 1, 0, u->e1a, nullptr, nullptr, kEpiBiasRelu, u->e1b));
-  k_pool<<<grid1d(u, L[1].nvox * 2), 256, 0, u->stream>>>(u->e1b, u->d1, L[0].nx, L[0].ny, L[0].nz, u->nb);
+  UNET_TRY(run(u, k_pool, grid1d(u, L[1].nvox * 2), u->e1b, u->d1, L[0].nx, L[0].ny, L[0].nz, u->nb));
   UNET_TRY(conv(u, 2, 1, u->d1, nullptr, nullptr, kEpiBiasRelu, u->e2a));
   UNET_TRY(conv(u, 3, 1, u->e2a, nullptr, nullptr, kEpiBiasRelu, u->e2b));
-  k_pool<<<grid1d(u, L[2].nvox * 2), 256, 0, u->stream>>>(u->e2b, u->d2, L[1].nx, L[1].ny, L[1].nz, u->nb);
+  UNET_TRY(run(u, k_pool, grid1d(u, L[2].nvox * 2), u->e2b, u->d2, L[1].nx, L[1].ny, L[1].nz, u->nb));
   UNET_TRY(conv(u, 4, 2, u->d2, nullptr, nullptr, kEpiBiasRelu, u->e3a));
   UNET_TRY(conv(u, 5, 2, u->e3a, nullptr, nullptr, kEpiBiasRelu, u->e3b));
-  k_pool<<<grid1d(u, L[3].nvox * 2), 256, 0, u->stream>>>(u->e3b, u->d3, L[2].nx, L[2].ny, L[2].nz, u->nb);
+  UNET_TRY(run(u, k_pool, grid1d(u, L[3].nvox * 2), u->e3b, u->d3, L[2].nx, L[2].ny, L[2].nz, u->nb));
   UNET_TRY(conv(u, 6, 3, u->d3, nullptr, nullptr, kEpiBiasRelu, u->e4a));
   UNET_TRY(conv(u, 7, 3, u->e4a, nullptr, nullptr, kEpiBiasRelu, u->e4b));
-  k_upsample<<<grid1d(u, L[2].nvox / 4), 256, 0, u->stream>>>(u->e4b, u->u3, L[2].nx, L[2].ny, L[2].nz, u->nb);
+  UNET_TRY(run(u, k_upsample, grid1d(u, L[2].nvox / 4), u->e4b, u->u3, L[2].nx, L[2].ny, L[2].nz, u->nb));
   UNET_TRY(conv(u, 8, 2, u->e3b, u->u3, nullptr, kEpiBiasRelu, u->c3a));
   UNET_TRY(conv(u, 9, 2, u->c3a, nullptr, nullptr, kEpiBiasRelu, u->c3b));
-  k_upsample<<<grid1d(u, L[1].nvox / 4), 256, 0, u->stream>>>(u->c3b, u->u2, L[1].nx, L[1].ny, L[1].nz, u->nb);
+  UNET_TRY(run(u, k_upsample, grid1d(u, L[1].nvox / 4), u->c3b, u->u2, L[1].nx, L[1].ny, L[1].nz, u->nb));
   UNET_TRY(conv(u, 10, 1, u->e2b, u->u2, nullptr, kEpiBiasRelu, u->c2a));
   UNET_TRY(conv(u, 11, 1, u->c2a, nullptr, nullptr, kEpiBiasRelu, u->c2b));
-  k_upsample<<<grid1d(u, L[0].nvox / 4), 256, 0, u->stream>>>(u->c2b, u->u1, L[0].nx, L[0].ny, L[0].nz, u->nb);
+  UNET_TRY(run(u, k_upsample, grid1d(u, L[0].nvox / 4), u->c2b, u->u1, L[0].nx, L[0].ny, L[0].nz, u->nb));
   if (train) {
     UNET_TRY(conv(u, 12, 0, u->e1b, u->u1, nullptr, kEpiBiasRelu, u->c1));
-    k_proj_fwd<<<grid1d(u, L[0].nvox), 256, 0, u->stream>>>(u->c1, u->params + u->off[kNumLayers], out, L[0].nvox,
-                                                           L[0].nx);
+    UNET_TRY(run(u, k_proj_fwd, grid1d(u, L[0].nvox), u->c1, u->params + u->off[kNumLayers], out, L[0].nvox, L[0].nx));
   } else {
     UNET_TRY(conv(u, 12, 0, u->e1b, u->u1, nullptr, kEpiProject, out));
   }
@@ -258,7 +266,7 @@ static int weight_grad(hpccg_unet *u, int layer, int level, const __nv_bfloat16 
   int blocks = 0;
   UNET_TRY(launch_dW(a, u->partial_blocks, u->d_err, u->num_sms, u->stream, &blocks));
   const int n = (27 * d.cin + 1) * 16;
-  k_reduce_partials<<<(n + 31) / 32, 256, 0, u->stream>>>(u->partial, blocks, n, u->grads + u->off[layer], 1);
+  UNET_TRY(run(u, k_reduce_partials, (n + 31) / 32, u->partial, blocks, n, u->grads + u->off[layer], 1));
   HPCCG_CUDA(cudaGetLastError());
   return HPCCG_OK;
 }
@@ -268,57 +276,56 @@ static int weight_grad(hpccg_unet *u, int layer, int level, const __nv_bfloat16 
 static int backward(hpccg_unet *u, const float *in) {
   const Level *L = u->L;
   const int nb = u->nb;
-  cudaStream_t s = u->stream;
   auto up_bwd = [&](int l, const __nv_bfloat16 *act) {  // gt[l - 1] -> pre[l]
-    k_up_bwd<<<grid1d(u, L[l].nvox * 2), 256, 0, s>>>(u->gt[l - 1], act, u->pre[l], L[l - 1].nx, L[l - 1].ny,
-                                                      L[l - 1].nz, nb);
+    return run(u, k_up_bwd, grid1d(u, L[l].nvox * 2), u->gt[l - 1], act, u->pre[l], L[l - 1].nx, L[l - 1].ny,
+               L[l - 1].nz, nb);
   };
   auto pool_bwd = [&](int l, const __nv_bfloat16 *act) {  // gt[l + 1], gs[l] -> pre[l]
-    k_pool_bwd<<<grid1d(u, L[l].nvox * 2), 256, 0, s>>>(u->gt[l + 1], u->gs[l], act, u->pre[l], L[l].nx, L[l].ny,
-                                                        L[l].nz, nb);
+    return run(u, k_pool_bwd, grid1d(u, L[l].nvox * 2), u->gt[l + 1], u->gs[l], act, u->pre[l], L[l].nx, L[l].ny,
+               L[l].nz, nb);
   };
   // projection and dec1a (level 0)
   const int pb = (int)std::min<int64_t>(u->num_sms * 4, (L[0].nvox + 255) / 256);
-  k_proj_bwd<<<pb, 256, 0, s>>>(u->c1, u->params + u->off[kNumLayers], u->dout, u->pre[0], u->partial, L[0].nvox,
-                                L[0].nx);
-  k_reduce_partials<<<1, 256, 0, s>>>(u->partial, pb, 17, u->grads + u->off[kNumLayers], 1);
+  UNET_TRY(run(u, k_proj_bwd, pb, u->c1, u->params + u->off[kNumLayers], u->dout, u->pre[0], u->partial, L[0].nvox,
+               L[0].nx));
+  UNET_TRY(run(u, k_reduce_partials, 1, u->partial, pb, 17, u->grads + u->off[kNumLayers], 1));
   UNET_TRY(weight_grad(u, 12, 0, u->e1b, u->u1, nullptr, u->pre[0]));
   UNET_TRY(conv(u, 12, 0, u->pre[0], nullptr, nullptr, kEpiRawF32, u->gs[0], 0));  // d e1b (skip)
   UNET_TRY(conv(u, 12, 0, u->pre[0], nullptr, nullptr, kEpiRawF32, u->gt[0], 1));  // d u1
   // dec2b, dec2a (level 1)
-  up_bwd(1, u->c2b);
+  UNET_TRY(up_bwd(1, u->c2b));
   UNET_TRY(weight_grad(u, 11, 1, u->c2a, nullptr, nullptr, u->pre[1]));
   UNET_TRY(conv(u, 11, 1, u->pre[1], nullptr, nullptr, kEpiMask, u->pre2[1], 0, u->c2a));
   UNET_TRY(weight_grad(u, 10, 1, u->e2b, u->u2, nullptr, u->pre2[1]));
   UNET_TRY(conv(u, 10, 1, u->pre2[1], nullptr, nullptr, kEpiRawF32, u->gs[1], 0));  // d e2b (skip)
   UNET_TRY(conv(u, 10, 1, u->pre2[1], nullptr, nullptr, kEpiRawF32, u->gt[1], 1));  // d u2
   // dec3b, dec3a (level 2)
-  up_bwd(2, u->c3b);
+  UNET_TRY(up_bwd(2, u->c3b));
   UNET_TRY(weight_grad(u, 9, 2, u->c3a, nullptr, nullptr, u->pre[2]));
   UNET_TRY(conv(u, 9, 2, u->pre[2], nullptr, nullptr, kEpiMask, u->pre2[2], 0, u->c3a));
   UNET_TRY(weight_grad(u, 8, 2, u->e3b, u->u3, nullptr, u->pre2[2]));
   UNET_TRY(conv(u, 8, 2, u->pre2[2], nullptr, nullptr, kEpiRawF32, u->gs[2], 0));  // d e3b (skip)
   UNET_TRY(conv(u, 8, 2, u->pre2[2], nullptr, nullptr, kEpiRawF32, u->gt[2], 1));  // d u3
   // enc4b, enc4a (level 3)
-  up_bwd(3, u->e4b);
+  UNET_TRY(up_bwd(3, u->e4b));
   UNET_TRY(weight_grad(u, 7, 3, u->e4a, nullptr, nullptr, u->pre[3]));
   UNET_TRY(conv(u, 7, 3, u->pre[3], nullptr, nullptr, kEpiMask, u->pre2[3], 0, u->e4a));
   UNET_TRY(weight_grad(u, 6, 3, u->d3, nullptr, nullptr, u->pre2[3]));
   UNET_TRY(conv(u, 6, 3, u->pre2[3], nullptr, nullptr, kEpiRawF32, u->gt[3], 0));  // d d3
   // enc3b, enc3a (level 2)
-  pool_bwd(2, u->e3b);
+  UNET_TRY(pool_bwd(2, u->e3b));
   UNET_TRY(weight_grad(u, 5, 2, u->e3a, nullptr, nullptr, u->pre[2]));
   UNET_TRY(conv(u, 5, 2, u->pre[2], nullptr, nullptr, kEpiMask, u->pre2[2], 0, u->e3a));
   UNET_TRY(weight_grad(u, 4, 2, u->d2, nullptr, nullptr, u->pre2[2]));
   UNET_TRY(conv(u, 4, 2, u->pre2[2], nullptr, nullptr, kEpiRawF32, u->gt[2], 0));  // d d2
   // enc2b, enc2a (level 1)
-  pool_bwd(1, u->e2b);
+  UNET_TRY(pool_bwd(1, u->e2b));
   UNET_TRY(weight_grad(u, 3, 1, u->e2a, nullptr, nullptr, u->pre[1]));
   UNET_TRY(conv(u, 3, 1, u->pre[1], nullptr, nullptr, kEpiMask, u->pre2[1], 0, u->e2a));
   UNET_TRY(weight_grad(u, 2, 1, u->d1, nullptr, nullptr, u->pre2[1]));
   UNET_TRY(conv(u, 2, 1, u->pre2[1], nullptr, nullptr, kEpiRawF32, u->gt[1], 0));  // d d1
   // enc1b, enc1a (level 0)
-  pool_bwd(0, u->e1b);
+  UNET_TRY(pool_bwd(0, u->e1b));
   UNET_TRY(weight_grad(u, 1, 0, u->e1a, nullptr, nullptr, u->pre[0]));
   UNET_TRY(conv(u, 1, 0, u->pre[0], nullptr, nullptr, kEpiMask, u->pre2[0], 0, u->e1a));
   UNET_TRY(weight_grad(u, 0, 0, nullptr, nullptr, in, u->pre2[0]));
@@ -474,9 +481,9 @@ extern "C" int hpccg_unet_loss_grad(hpccg_unet *u, int32_t nx, int32_t ny, int32
   const int64_t n = u->L[0].nvox;
   const int mb = std::min(u->num_sms * 8, grid1d(u, u->loss_kind == 1 ? n / 4 : n));
   if (u->loss_kind == 1)
-    k_energy<<<mb, 256, 0, u->stream>>>(u->out_train, d_target, u->dout, u->loss_partial, nx, ny, nz, nb);
+    UNET_TRY(run(u, k_energy, mb, u->out_train, d_target, u->dout, u->loss_partial, nx, ny, nz, nb));
   else
-    k_mse<<<mb, 256, 0, u->stream>>>(u->out_train, d_target, u->dout, u->loss_partial, n);
+    UNET_TRY(run(u, k_mse, mb, u->out_train, d_target, u->dout, u->loss_partial, n));
   if ((rc = backward(u, d_in))) return rc;
   // read after the backward pass: nothing on the host waits between the two
   std::vector<float> lp(mb);
@@ -589,6 +596,7 @@ extern "C" int hpccg_unet_conv3_layer(int32_t nx, int32_t ny, int32_t nz, int32_
     a.proj = d_proj;
     a.act = nullptr;
     a.out = d_out;
+    a.chained = false;
     a.err = d_err;
     rc = path == 2 ? launch_conv3_brick(nin, epi, a, sms, 0) : launch_conv3_win(nin, epi, a, sms, 0);
     if (cudaDeviceSynchronize() != cudaSuccess) rc = set_cuda_error(cudaGetLastError(), "conv3 tc", __FILE__, __LINE__);
@@ -608,6 +616,7 @@ extern "C" int hpccg_unet_conv3_layer(int32_t nx, int32_t ny, int32_t nz, int32_
     a.act = nullptr;
     a.epi = epi;
     a.out = d_out;
+    a.chained = false;
     rc = launch_conv3_cc(a, sms, 0);
     if (cudaDeviceSynchronize() != cudaSuccess) rc = set_cuda_error(cudaGetLastError(), "conv3 cc", __FILE__, __LINE__);
   }

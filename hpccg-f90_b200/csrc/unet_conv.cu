@@ -321,6 +321,7 @@ __global__ void __launch_bounds__(kIn1Threads) k_conv3_in1_tc(const float *in, c
   __syncthreads();  // B, the bias, the first tile's lines, the barriers and the TMEM slot
   tc_fence_after();
   const uint32_t tmem = slot;
+  chain_release();  // the TMEM is allocated
   constexpr uint32_t idesc = idesc_bf16(128, 16);
   const uint64_t bd = smem_desc(sB, 256, 128);
   // the epilogue of tile D (buffer buf, its use u of that buffer): bias, ReLU, BF16 stores

@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
     }
     mbar_init(&drain, 1);
     fence_mbar_init();
+    chain_wait();
     for (; fetched < p.slots && fu < p.nunits; ++fetched) fetch(fetched);  // under the weights' set-up
   }
   if (warp == 1) {
@@ -191,6 +192,8 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = slot;
+  chain_wait();
+  chain_release();  // the TMEM is allocated
 
   if (warp == 0) {
     if (lane == 0) {
@@ -457,8 +460,7 @@ static int launch_win(const WinArgs &w, int num_sms, cudaStream_t s) {
   const int smem = win_weight_bytes(NIN) + w.p.slots * NIN * w.p.input_bytes + kWinPad + (EPI == kEpiProject ? kWinProjBytes : 0);
   // the attribute is per device: set every time
   HPCCG_CUDA(cudaFuncSetAttribute(k_conv3_win<NIN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, kWinSmem));
-  k_conv3_win<NIN, EPI><<<std::min(w.p.nunits, num_sms), kWinThreads, smem, s>>>(w);
-  HPCCG_CUDA(cudaGetLastError());
+  HPCCG_CUDA(launch_chained(k_conv3_win<NIN, EPI>, std::min(w.p.nunits, num_sms), kWinThreads, smem, s, w.a.chained, w));
   return HPCCG_OK;
 }
 

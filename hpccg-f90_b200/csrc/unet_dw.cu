@@ -109,6 +109,8 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = slot;
+  chain_wait();
+  chain_release();  // the TMEM is allocated
   const int ksteps = a.kx / 16, chunk = max(1, kDwChain / ksteps);  // rows between two drains
   auto unit = [&](int u, int &b, int &z, int &ya, int &yb, int &x0) {
     x0 = (u % a.nxb) * a.kx;
@@ -262,6 +264,8 @@ __global__ void __launch_bounds__(kDwInThreads, kDwInPerSm) k_dW_in1(DwArgs a, i
   const int64_t nunit = (int64_t)nxb * nyb * nz * a.nb;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5, xh = warp / 3, dzi = warp % 3;
   const int h = lane & 1, r = lane >> 1;
+  chain_wait();
+  chain_release();
   unsigned long long acc[9][4], bs[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
@@ -380,8 +384,7 @@ int launch_dW(const DwArgs &a, int max_blocks, int *err, int num_sms, cudaStream
     const int64_t units = (int64_t)((a.ny + kDwInRows - 1) / kDwInRows) * a.nz * a.nb * nxb;
     // its partials are 1/30 of a 32-channel layer's, which max_blocks counts
     *blocks = (int)std::min<int64_t>(std::min(30 * max_blocks, kDwInPerSm * num_sms), units);
-    k_dW_in1<<<*blocks, kDwInThreads, 0, s>>>(a, xb);
-    HPCCG_CUDA(cudaGetLastError());
+    HPCCG_CUDA(launch_chained(k_dW_in1, *blocks, kDwInThreads, 0, s, true, a, xb));
     return HPCCG_OK;
   }
   DwTcArgs t{};
@@ -408,8 +411,7 @@ int launch_dW(const DwArgs &a, int max_blocks, int *err, int num_sms, cudaStream
   auto kern = nin == 2 ? k_dW_tc<2> : k_dW_tc<1>;
   // the attribute is per device: set every time, to the most any width needs
   HPCCG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_smem_bytes(nin, kDwMaxX)));
-  kern<<<*blocks, kDwThreads, smem, s>>>(t);
-  HPCCG_CUDA(cudaGetLastError());
+  HPCCG_CUDA(launch_chained(kern, *blocks, kDwThreads, smem, s, true, t));
   return HPCCG_OK;
 }
 

@@ -86,6 +86,8 @@ __global__ void __launch_bounds__(kCcThreads, cc_blocks<V, CO>()) k_conv3_cc(CcC
   const int nx = a.nx, ny = a.ny, nz = a.nz, cin = 16 * a.nin;
   for (int e = threadIdx.x; e < 27 * cin * 4; e += blockDim.x)
     reinterpret_cast<float4 *>(cc_w)[e] = __ldg(reinterpret_cast<const float4 *>(a.W) + e);
+  chain_wait();
+  chain_release();
   __syncthreads();
   constexpr int NG = 16 / CO;
   const int nyg = (ny + V - 1) / V;
@@ -180,15 +182,19 @@ __global__ void __launch_bounds__(kCcThreads, cc_blocks<V, CO>()) k_conv3_cc(CcC
 
 template <int V, int CO>
 static int launch_cc(const CcConvArgs &a, int num_sms, cudaStream_t s) {
-  const int smem = 27 * 16 * a.nin * 16 * (int)sizeof(float);
-  // the attribute is per device: set every time
-  HPCCG_CUDA(cudaFuncSetAttribute(k_conv3_cc<V, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  27 * 32 * 16 * (int)sizeof(float)));
   const int64_t threads = (int64_t)a.nx * ((a.ny + V - 1) / V) * a.nz * a.nb * (16 / CO);
+  constexpr int kBlocks = cc_blocks<V, CO>();
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((threads + kCcThreads - 1) / kCcThreads,
-                                                          (int64_t)num_sms * cc_blocks<V, CO>()));
-  k_conv3_cc<V, CO><<<grid, kCcThreads, smem, s>>>(a);
-  HPCCG_CUDA(cudaGetLastError());
+                                                               (int64_t)num_sms * kBlocks));
+  // The blocks of a chained launch start where the predecessor's end first and would
+  // pile up there: shared memory is padded so that no SM takes more than its share
+  // (72^3 forward: plain launches 779 us, unpadded 886, padded 753; 88^3 1237, 1243, 1155).
+  const int per_sm = (grid + num_sms - 1) / num_sms;
+  int smem = 27 * 16 * a.nin * 16 * (int)sizeof(float);
+  if (per_sm < kBlocks) smem = std::max(smem, 228 * 1024 / (per_sm + 1) - 1024 + 128);
+  // the attribute is per device: set every time, to the most any launch needs
+  HPCCG_CUDA(cudaFuncSetAttribute(k_conv3_cc<V, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 114 * 1024));
+  HPCCG_CUDA(launch_chained(k_conv3_cc<V, CO>, grid, kCcThreads, smem, s, a.chained, a));
   return HPCCG_OK;
 }
 
@@ -213,6 +219,8 @@ __device__ __forceinline__ void conv3_in1_body(const float *in, const float *W, 
                                                __nv_bfloat16 *out, int nx, int ny, int nz, int nb, int relu) {
   __shared__ __align__(16) float sw[27 * 16 + 16];
   for (int e = threadIdx.x; e < 27 * 16 + 16; e += blockDim.x) sw[e] = e < 27 * 16 ? W[e] : bias[e - 27 * 16];
+  chain_wait();
+  chain_release();
   __syncthreads();
   const int64_t ngroups = (int64_t)nx * ny * nz * nb / V;
   for (int64_t gi = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; gi < ngroups;
@@ -320,6 +328,8 @@ __device__ __forceinline__ void row_coords(int64_t row, int ny, int nz, int64_t 
 
 // 2x2x2 average pooling, one thread per coarse 16-byte unit (8 channels).
 __global__ void k_pool(const __nv_bfloat16 *in, __nv_bfloat16 *out, int nx, int ny, int nz, int nb) {
+  chain_wait();
+  chain_release();
   const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
   const int64_t n = (int64_t)cx * cy * cz * nb * 2;
   const uint4 *src = reinterpret_cast<const uint4 *>(in);
@@ -352,6 +362,8 @@ __global__ void k_pool(const __nv_bfloat16 *in, __nv_bfloat16 *out, int nx, int 
 // thread per coarse 16-byte unit: one load, and its eight fine copies as two
 // adjacent units in each of the four fine rows (a warp writes 1 KB runs).
 __global__ void k_upsample(const __nv_bfloat16 *in, __nv_bfloat16 *out, int nx, int ny, int nz, int nb) {
+  chain_wait();
+  chain_release();
   const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
   const int64_t n = (int64_t)cx * cy * cz * nb * 2;
   const uint4 *src = reinterpret_cast<const uint4 *>(in);
@@ -378,6 +390,8 @@ __global__ void k_upsample(const __nv_bfloat16 *in, __nv_bfloat16 *out, int nx, 
 // 144 us at 64^3, batch 4; 22 us here.
 __global__ void k_pool_bwd(const float *dc, const float *skip, const __nv_bfloat16 *act, __nv_bfloat16 *out, int nx,
                            int ny, int nz, int nb) {
+  chain_wait();
+  chain_release();
   const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
   const int64_t n = (int64_t)nx * ny * nz * nb * 2;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
@@ -405,6 +419,8 @@ __global__ void k_pool_bwd(const float *dc, const float *skip, const __nv_bfloat
 // sum of the 8 fine children : 0 in BF16.  One thread per 16-byte unit of out.
 __global__ void k_up_bwd(const float *df, const __nv_bfloat16 *act, __nv_bfloat16 *out, int nx, int ny, int nz,
                          int nb) {
+  chain_wait();
+  chain_release();
   const int cx = nx / 2, cy = ny / 2, cz = nz / 2;
   const int64_t n = (int64_t)cx * cy * cz * nb * 2;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
@@ -446,6 +462,8 @@ __global__ void k_up_bwd(const float *df, const __nv_bfloat16 *act, __nv_bfloat1
 // (One thread per k summing every partial: 14.8 against 4 us a layer.)
 __global__ void __launch_bounds__(256) k_reduce_partials(const float *partial, int nblocks, int n, float *grad,
                                                          int accumulate) {
+  chain_wait();
+  chain_release();
   __shared__ double s[8][32];
   const int c = threadIdx.x & 31, r = threadIdx.x >> 5, k = blockIdx.x * 32 + c;
   double v = 0.0;
@@ -481,6 +499,8 @@ __device__ __forceinline__ int64_t voxel_unit(int64_t v, int nx) {
 
 // Output projection (training path): out[v] = proj . act[v] + proj_b.
 __global__ void k_proj_fwd(const __nv_bfloat16 *act, const float *proj, float *out, int64_t nvox, int nx) {
+  chain_wait();
+  chain_release();
   for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < nvox; v += (int64_t)gridDim.x * blockDim.x) {
     float f[16], r = proj[16];
     load_voxel(act, voxel_unit(v, nx), nx, f);
@@ -494,6 +514,8 @@ __global__ void k_proj_fwd(const __nv_bfloat16 *act, const float *proj, float *o
 // 16-byte units in and out (one element at a time: 56 us at 64^3, batch 4; 16 us here).
 __global__ void __launch_bounds__(256) k_proj_bwd(const __nv_bfloat16 *act, const float *proj, const float *dout,
                                                   __nv_bfloat16 *dact, float *partial, int64_t nvox, int nx) {
+  chain_wait();
+  chain_release();
   __shared__ float red[17][256];
   float acc[17];
 #pragma unroll
@@ -536,6 +558,8 @@ __global__ void __launch_bounds__(256) k_proj_bwd(const __nv_bfloat16 *act, cons
 // Mean squared error over n values and dL/dout; per-block loss partials.
 __global__ void __launch_bounds__(256) k_mse(const float *out, const float *tgt, float *dout, float *partial,
                                              int64_t n) {
+  chain_wait();
+  chain_release();
   __shared__ float red[256];
   float s = 0.f;
   const float scale = 2.f / (float)n;
@@ -567,6 +591,8 @@ __device__ __forceinline__ float4 load4(const float *p) {
 // at 64^3, batch 4, against a voxel a thread and 54 loads one by one.
 __global__ void __launch_bounds__(256) k_energy(const float *out, const float *tgt, float *dout, float *partial,
                                                 int nx, int ny, int nz, int nb) {
+  chain_wait();
+  chain_release();
   __shared__ float red[256];
   const int64_t n = (int64_t)nx * ny * nz * nb;
   const float scale = 2.f / (float)n;

@@ -14,6 +14,7 @@ struct CcConvArgs {
   const __nv_bfloat16 *act;          // for kEpiMask
   int epi;
   void *out;
+  bool chained;                      // launch_chained
 };
 
 struct DwArgs {
