@@ -121,6 +121,8 @@ struct hpccg_ctx {
   // SpMV selection
   int spmv_kind = HPCCG_SPMV_AUTO;
   int spmv_param = 0;
+  // hpccg_gpu_solve_mixed_fcg: its vectors (kept up to kMfcgKeepBytes), scalars, and their copy on the host
+  void *mfcg_vec = nullptr, *mfcg_st = nullptr, *mfcg_host = nullptr;
   bool mixed_fused_off = false;  // hpccg_gpu_set_mixed_fused(ctx, 0)
   bool spmv_tuned = false;
   // CG graph

@@ -258,9 +258,10 @@ extern "C" void hpccg_gpu_destroy(hpccg_ctx *c) {
   if (c->cg_exec) cudaGraphExecDestroy(c->cg_exec);
   if (c->cg_graph) cudaGraphDestroy(c->cg_graph);
   void *bufs[] = {c->d_rowptr, c->d_col, c->d_val, c->d_ell_col, c->d_ell_val, c->d_r, c->d_p,
-                  c->d_Ap, c->d_x, c->d_b, c->d_partials, c->d_counter, c->d_state, c->d_hist, c->d_p2, c->d_slots};
+                  c->d_Ap, c->d_x, c->d_b, c->d_partials, c->d_counter, c->d_state, c->d_hist, c->d_p2, c->d_slots, c->mfcg_vec, c->mfcg_st};
   for (void *p : bufs)
     if (p) cudaFree(p);
+  if (c->mfcg_host) cudaFreeHost(c->mfcg_host);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->solve0) cudaEventDestroy(c->solve0);

@@ -15,8 +15,13 @@
 // It stops at ||r_in|| <= max(1e-5, 0.5 rel_tol ||b|| / ||r||) (the inner
 // start is scaled to norm 1), the adaptive target of hpccg_gpu_solve_mixed.
 //
-// The loop is host-driven: each inner iteration reads its scalars back (the
-// network application, about 3 ms at 256^3, dominates the time anyway).
+// The loop is host-driven, one synchronisation per inner iteration: the kernels
+// form beta, alpha and the next s themselves, and the last one leaves a copy of
+// the scalars in host memory, from which the host decides whether to go on.  r.z <= 0
+// is found on the device too: the rest of that iteration does nothing, and the
+// host launches it again as plain CG.  At 128^3 an iteration is the network's 407
+// us and about 60 us besides; reading the scalars twice an iteration and writing them
+// twice cost 30 us more, allocating the vectors in each solve 1 to 2.5 ms a solve.
 #include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -33,17 +38,20 @@ namespace hpccg {
 
 struct MfcgState {
   double rr64, bb;      // FP64 residual and right-hand side norms squared
-  double rz;            // r.z of the current direction (set by the host)
+  double rz;            // r.z of the current direction
   double rznew, rzold;  // r.z and r.z_old of the latest preconditioner application
   double pAp, rr, alpha, beta, s, scale;
+  int neg;  // the network lost positivity (r.z <= 0): nothing is updated
 };
+// Vectors larger than this are given back after the solve.
+constexpr size_t kMfcgKeepBytes = (size_t)256 << 20;
 
 struct MfcgArgs {
   int n;
   double *x, *r64;
   const double *b;
   float *r, *p, *Ap, *z, *zold, *d, *nn_in, *nn_out;
-  MfcgState *st;
+  MfcgState *st, *host;  // host: the copy that the host reads after a synchronisation
   Reduction red;
   StencilGeom geom;
   PlaneMap pm;  // the FP32 walk's map (four or one column per thread)
@@ -93,7 +101,7 @@ __global__ void k_mfcg_nn_in(MfcgArgs g) {
 // z = s * net(r/s) or z = r; r.z and r.z_old, both reduced in a fixed order
 // (r.z_old's block partials sit in the upper half of the scratch)
 constexpr int kHalf = kMaxPartials / 2;
-__global__ void __launch_bounds__(kBlock) k_mfcg_zdots(MfcgArgs g, int use_net) {
+__global__ void __launch_bounds__(kBlock) k_mfcg_zdots(MfcgArgs g, int use_net, int restart) {
   __shared__ double smem[32];
   const float s = (float)g.st->s;
   double a = 0.0, b = 0.0;
@@ -114,14 +122,22 @@ __global__ void __launch_bounds__(kBlock) k_mfcg_zdots(MfcgArgs g, int use_net) 
       vb = __dadd_rn(vb, ((volatile double *)g.red.partials)[kHalf + i]);
     vb = block_sum<kBlock>(vb, smem);
     if (threadIdx.x == 0) {
-      g.st->rznew = va;
-      g.st->rzold = vb;
+      MfcgState *st = g.st;
+      st->rznew = va;
+      st->rzold = vb;
+      st->neg = use_net && !(va > 0.0);
+      if (!st->neg) {
+        st->beta = restart ? 0.0 : (va - vb) / st->rz;  // Polak-Ribiere
+        st->rz = va;
+      }
+      *g.host = *st;
     }
   }
 }
 
 // p = z + beta p (restart: p = z); z_old = z
 __global__ void k_mfcg_update_p(MfcgArgs g, int restart) {
+  if (g.st->neg) return;
   const float beta = restart ? 0.f : (float)g.st->beta;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x) {
     const float zi = g.z[i];
@@ -145,6 +161,7 @@ struct EpiAp32 {
 template <bool W4>
 __global__ void __launch_bounds__(kBlock) k_mfcg_spmv(MfcgArgs g) {
   __shared__ double smem[32];
+  if (g.st->neg) return;
   EpiAp32 epi{g.Ap};
   double part;
   if constexpr (W4)
@@ -161,9 +178,10 @@ __global__ void __launch_bounds__(kBlock) k_mfcg_spmv(MfcgArgs g) {
   }
 }
 
-// d += alpha p, r -= alpha Ap, r.r
+// d += alpha p, r -= alpha Ap, r.r; the next iteration's s, the rms of r
 __global__ void __launch_bounds__(kBlock) k_mfcg_update(MfcgArgs g) {
   __shared__ double smem[32];
+  if (g.st->neg) return;
   const float alpha = (float)g.st->alpha;
   double part = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.n; i += gridDim.x * blockDim.x) {
@@ -175,7 +193,11 @@ __global__ void __launch_bounds__(kBlock) k_mfcg_update(MfcgArgs g) {
   const double tot = block_sum<kBlock>(part, smem);
   if (arrive_last(g.red, tot)) {
     const double v = finish_sum<kBlock>(g.red, smem);
-    if (threadIdx.x == 0) g.st->rr = v;
+    if (threadIdx.x == 0) {
+      g.st->rr = v;
+      g.st->s = sqrt(v) / sqrt((double)g.n);
+      *g.host = *g.st;
+    }
   }
 }
 
@@ -201,16 +223,17 @@ extern "C" int hpccg_gpu_solve_mixed_fcg(hpccg_ctx *c, hpccg_unet *u, int32_t nx
   if (rc) return rc;
   const int n = c->nrow;
   const size_t v4 = sizeof(float) * (size_t)c->npad, bytes = sizeof(double) * (size_t)n;
-  float *f32 = nullptr;
-  MfcgState *st = nullptr;
-  if (cudaMalloc(&f32, 8 * v4) != cudaSuccess || cudaMalloc(&st, sizeof(MfcgState)) != cudaSuccess) {
+  float *f32 = static_cast<float *>(c->mfcg_vec);
+  if (!c->mfcg_st && cudaMalloc(&c->mfcg_st, sizeof(MfcgState)) != cudaSuccess) c->mfcg_st = nullptr;
+  if (!c->mfcg_host && cudaMallocHost(&c->mfcg_host, sizeof(MfcgState)) != cudaSuccess) c->mfcg_host = nullptr;
+  if (!c->mfcg_st || !c->mfcg_host || (!f32 && cudaMalloc(&f32, 8 * v4) != cudaSuccess)) {
     cudaGetLastError();
-    cudaFree(f32);
     return HPCCG_ERR_OOM;
   }
+  MfcgState *st = static_cast<MfcgState *>(c->mfcg_st);
+  if (8 * v4 <= kMfcgKeepBytes) c->mfcg_vec = f32;
   auto cleanup = [&]() {
-    cudaFree(f32);
-    cudaFree(st);
+    if (!c->mfcg_vec) cudaFree(f32);
   };
   cudaStream_t s = c->stream;
   MfcgArgs g;
@@ -222,6 +245,7 @@ extern "C" int hpccg_gpu_solve_mixed_fcg(hpccg_ctx *c, hpccg_unet *u, int32_t nx
   for (int k = 0; k < 8; ++k) f[k] = f32 + (size_t)k * c->npad;
   g.r = f[0], g.p = f[1], g.Ap = f[2], g.z = f[3], g.zold = f[4], g.d = f[5], g.nn_in = f[6], g.nn_out = f[7];
   g.st = st;
+  g.host = static_cast<MfcgState *>(c->mfcg_host);
   g.red = reduction_of(c);
   g.geom = StencilGeom{nx, ny, nz};
   const PlaneMap q4 = boxw_map(4, nx, ny, nz, (int64_t)c->num_sms * 4 * kBlock);
@@ -267,44 +291,41 @@ extern "C" int hpccg_gpu_solve_mixed_fcg(hpccg_ctx *c, hpccg_unet *u, int32_t nx
     ++outer;
     const double target = std::max(1e-5, 0.5 * rel_tol * bnorm / rnorm);
     h.scale = rnorm;
+    h.s = 1.0 / sqrt((double)n);  // rms of the inner residual, whose norm starts at 1
     if ((rc = write_state())) break;
     k_mfcg_start<<<c->grid, kBlock, 0, s>>>(g);
     bool use_net = u != nullptr, restart = true;
     double rin = 1.0, best = 1.0;
     int since_best = 0;
-    for (int k = 0; k < max_inner && rin > target; ++k) {
-      h.s = rin / sqrt((double)n);  // rms of the inner residual
-      if ((rc = write_state())) break;
-      if (use_net) {
-        k_mfcg_nn_in<<<c->grid, kBlock, 0, s>>>(g);
-        if ((rc = hpccg_unet_forward_on(u, nx, ny, nz, g.nn_in, g.nn_out, s))) break;
-        ++applies;
-      }
-      k_mfcg_zdots<<<c->grid, kBlock, 0, s>>>(g, use_net ? 1 : 0);
-      if ((rc = read_state())) break;
-      if (use_net && !(h.rznew > 0.0)) {  // the network lost positivity on this residual: plain CG
-        use_net = false;
-        fallback = 1;
-        restart = true;
-        k_mfcg_zdots<<<c->grid, kBlock, 0, s>>>(g, 0);
-        if ((rc = read_state())) break;
-      }
-      h.beta = restart ? 0.0 : (h.rznew - h.rzold) / h.rz;  // Polak-Ribiere
-      h.rz = h.rznew;
-      if ((rc = write_state())) break;
+    // z, the direction, A p and the update; the scalars as they then are
+    auto step = [&](bool net) -> int {
+      k_mfcg_zdots<<<c->grid, kBlock, 0, s>>>(g, net ? 1 : 0, restart ? 1 : 0);
       k_mfcg_update_p<<<c->grid, kBlock, 0, s>>>(g, restart ? 1 : 0);
-      restart = false;
       if (w4)
         k_mfcg_spmv<true><<<sgrid, kBlock, 0, s>>>(g);
       else
         k_mfcg_spmv<false><<<sgrid, kBlock, 0, s>>>(g);
       k_mfcg_update<<<c->grid, kBlock, 0, s>>>(g);
-      const cudaError_t le = cudaGetLastError();
-      if (le != cudaSuccess) {
-        rc = set_cuda_error(le, "mixed fcg inner", __FILE__, __LINE__);
-        break;
+      cudaError_t e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+      if (e != cudaSuccess) return set_cuda_error(e, "mixed fcg inner", __FILE__, __LINE__);
+      h = *g.host;
+      return HPCCG_OK;
+    };
+    for (int k = 0; k < max_inner && rin > target; ++k) {
+      if (use_net) {
+        k_mfcg_nn_in<<<c->grid, kBlock, 0, s>>>(g);
+        if ((rc = hpccg_unet_forward_on(u, nx, ny, nz, g.nn_in, g.nn_out, s))) break;
+        ++applies;
       }
-      if ((rc = read_state())) break;
+      if ((rc = step(use_net))) break;
+      if (h.neg) {  // the network lost positivity on this residual: plain CG
+        use_net = false;
+        fallback = 1;
+        restart = true;
+        if ((rc = step(false))) break;
+      }
+      restart = false;
       ++inner_total;
       if (!(h.pAp > 0.0) || !isfinite(h.rr)) {
         status = HPCCG_ERR_BREAKDOWN;

@@ -266,6 +266,34 @@ def test_input_layer_and_energy_gradients_edges(env, nx, ny, nz, nb):
         assert err <= 6e-2, (l, err)
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(16, 16, 16), (24, 16, 40), (64, 32, 16)])
+def test_mixed_fcg_without_positivity_is_plain_cg(env, nx, ny, nz):
+    """One outer cycle with a network and with its negative: r.z > 0 holds for one of them
+    at most, and the other gives way to plain CG before it has changed anything, so that
+    its result is the plain solver's bit for bit."""
+    torch, hp = env
+    from hpccg_b200 import learned
+
+    M = hp.Matrix.generated(nx, ny, nz)
+    rng = np.random.default_rng(nx)
+    b = torch.from_numpy(rng.normal(0, 1, nx * ny * nz)).cuda()
+    x0 = torch.zeros_like(b)
+    plain, st = learned.solve_mixed_fcg(M, None, (nx, ny, nz), b, x0, rel_tol=1e-12, max_outer=1)
+    assert st == hp.HPCCG_ERR_NOT_CONVERGED and plain.fallback == 0 and plain.nn_applies == 0
+    net, p = _net_and_params(hp, seed=4)
+    same = 0
+    for sign in (1.0, -1.0):
+        q = p.copy()
+        q[-17:] *= sign
+        net.set_params(q.astype(np.float32))
+        x = torch.zeros_like(b)
+        info, _ = learned.solve_mixed_fcg(M, net, (nx, ny, nz), b, x, rel_tol=1e-12, max_outer=1)
+        if info.fallback and info.nn_applies == 1:
+            assert info.inner_iters == plain.inner_iters and torch.equal(x, x0)
+            same += 1
+    assert same >= 1
+
+
 def test_trained_network_reduces_fcg_iterations(env):
     """What the trained network gains: FCG iterations to FP64 rel-res 1e-8 on
     held-out Gaussian-random-field right-hand sides, against plain CG through
