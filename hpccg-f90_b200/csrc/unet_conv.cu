@@ -6,6 +6,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "unet_conv.cuh"
 
@@ -216,95 +217,39 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv3_brick(ConvArgs a) {
 // An im2col GEMM per tile of 128 voxels of one x row: A[m][k] = in(x0+m+dx, y+dy, z+dz)
 // in BF16 for tap k = (dz+1)*9 + (dy+1)*3 + (dx+1) (k = 27..31 zero), B[c][k] = W[k][c];
 // two MMAs (M = 128, N = 16, K = 16) into a 16-column FP32 accumulator.  A CTA walks a
-// contiguous range of tiles.  The tile's nine input lines (dz, dy), x0-1 .. x0+128 with
-// zeros outside the grid, are staged once in shared memory: each thread loads one element
-// of every line a tile ahead into registers and stores them while the current tile is
-// built.  Thread m then reads its voxel's 27 taps from the staged lines into its A row;
-// thread 0 issues the tile's MMAs; every warp drains its TMEM lane quarter of the PREVIOUS
-// tile (bias, ReLU, BF16 stores), so a tile's MMAs run while the next tile is built.  The
-// staged lines, A and the accumulator are double-buffered: one barrier per tile.
+// contiguous range of tiles, y innermost: thread m keeps its voxel's 27 taps in
+// registers, and from one tile to the next takes over two of the three rows of each
+// z plane and forms the third from one load per plane, a tile ahead, and its
+// neighbours' lanes (the lanes at a warp's ends load their outer neighbour).  It
+// writes the taps to its A row; thread 0 issues the tile's MMAs; every warp drains
+// its TMEM lane quarter of the PREVIOUS tile (bias, ReLU, BF16 stores), so a tile's
+// MMAs run while the next tile is built.  A and the accumulator are double-buffered:
+// one barrier per tile.  Against nine lines per tile staged in shared memory and 27
+// reads of them a thread: 282 -> 202 us at 256^3 (2.7 TB/s of stores), 46 -> 34 at
+// 128^3.  Bound by instruction issue, 250 a warp and tile; with 5, 7 or 8 CTAs an SM 205,
+// 234 and 278 us.
 constexpr int kIn1Threads = 128;
 constexpr int kIn1ABytes = 4 * 128 * 16;  // [4 K chunks of 8 taps][128 rows][8 BF16]
 constexpr int kIn1BBytes = 4 * 16 * 16;   // [4 K chunks][16 output channels][8 BF16]
-constexpr int kIn1Line = 132;             // a staged line: x0-1+i at [i], i < 130
+constexpr int kIn1PerSm = 6;
 
-// tile coordinates in tile order: row = (b*nz + z)*ny + y, x block xb (tile = row*tx + xb)
-struct In1Tile {
-  int row, xb, y, z;
-  __device__ __forceinline__ void at(int t, int tx, int ny, int nz) {
-    row = t / tx;
-    xb = t - row * tx;
-    const int yz = row / ny;
-    y = row - yz * ny;
-    z = yz % nz;
-  }
-  __device__ __forceinline__ void next(int tx, int ny, int nz) {
-    if (++xb == tx) {
-      xb = 0;
-      ++row;
-      if (++y == ny) {
-        y = 0;
-        if (++z == nz) z = 0;
-      }
-    }
-  }
-};
-
-__global__ void __launch_bounds__(kIn1Threads) k_conv3_in1_tc(const float *in, const float *W, const float *bias,
-                                                              __nv_bfloat16 *out, int nx, int ny, int nz, int nb,
-                                                              int relu, int *err) {
+__global__ void __launch_bounds__(kIn1Threads, kIn1PerSm) k_conv3_in1_tc(const float *in, const float *W,
+                                                                         const float *bias, __nv_bfloat16 *out,
+                                                                         int nx, int ny, int nz, int nb, int relu,
+                                                                         int *err) {
   __shared__ __align__(1024) uint8_t sA[2][kIn1ABytes];
   __shared__ __align__(128) uint8_t sB[kIn1BBytes];
-  __shared__ __align__(16) float sL[2][9 * kIn1Line];
   __shared__ __align__(16) float sBias[16];
   __shared__ uint64_t done[2], fin;
   __shared__ uint32_t slot;
   __shared__ int s_fail;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int e = tid; e < 32 * 16; e += kIn1Threads) {  // B element (k, c): chunk k/8, row c, position k%8
     const int k = e / 16, c = e % 16;
     reinterpret_cast<__nv_bfloat16 *>(sB)[((k >> 3) * 16 + c) * 8 + (k & 7)] =
         __float2bfloat16(k < 27 ? W[k * 16 + c] : 0.f);
   }
   if (tid < 16) sBias[tid] = bias[tid];
-  // tile t = ((b*nz + z)*ny + y)*tx + x-block; 32-bit indices (a grid has fewer than 2^31 tiles)
-  const int tx = nx / 128;
-  const int ntiles = tx * ny * nz * nb;
-  const int t_lo = (int)((int64_t)blockIdx.x * ntiles / gridDim.x);
-  const int t_hi = (int)((int64_t)(blockIdx.x + 1) * ntiles / gridDim.x);
-  // this thread's element of each staged line (x0 + tid), and for threads 0..8 / 32..40
-  // the left / right halo element (x0 - 1 / x0 + 128) of line hl
-  const int hl = tid < 9 ? tid : (tid >= 32 && tid < 41 ? tid - 32 : -1);
-  const int hx = tid < 32 ? -1 : 128;
-  float ld[9], lh = 0.f;
-  In1Tile L, D;  // the next tile to load, the next tile to drain
-  L.at(t_lo, tx, ny, nz);
-  D = L;
-  auto load = [&](bool live) {
-    const int x0 = L.xb * 128;
-#pragma unroll
-    for (int l = 0; l < 9; ++l) {
-      const int dz = l / 3 - 1, dy = l % 3 - 1;
-      const bool ok = live && (unsigned)(L.z + dz) < (unsigned)nz && (unsigned)(L.y + dy) < (unsigned)ny;
-      ld[l] = ok ? __ldg(in + (int64_t)(L.row + dz * ny + dy) * nx + x0 + tid) : 0.f;
-    }
-    if (hl >= 0) {
-      const int dz = hl / 3 - 1, dy = hl % 3 - 1, xh = x0 + hx;
-      const bool ok = live && (unsigned)(L.z + dz) < (unsigned)nz && (unsigned)(L.y + dy) < (unsigned)ny &&
-                      (unsigned)xh < (unsigned)nx;
-      lh = ok ? __ldg(in + (int64_t)(L.row + dz * ny + dy) * nx + xh) : 0.f;
-    }
-    L.next(tx, ny, nz);
-  };
-  auto stage = [&](int sb) {
-    float *s = sL[sb];
-#pragma unroll
-    for (int l = 0; l < 9; ++l) s[l * kIn1Line + tid + 1] = ld[l];
-    if (hl >= 0) s[hl * kIn1Line + hx + 1] = lh;
-  };
-  load(t_lo < t_hi);
-  stage(0);
-  load(t_lo + 1 < t_hi);
   if (tid == 0) {
     mbar_init(&done[0], 1);
     mbar_init(&done[1], 1);
@@ -318,70 +263,111 @@ __global__ void __launch_bounds__(kIn1Threads) k_conv3_in1_tc(const float *in, c
   }
   fence_proxy_async_smem();
   tc_fence_before();
-  __syncthreads();  // B, the bias, the first tile's lines, the barriers and the TMEM slot
+  __syncthreads();  // B, the bias, the barriers and the TMEM slot
   tc_fence_after();
   const uint32_t tmem = slot;
   chain_release();  // the TMEM is allocated
   constexpr uint32_t idesc = idesc_bf16(128, 16);
   const uint64_t bd = smem_desc(sB, 256, 128);
-  // the epilogue of tile D (buffer buf, its use u of that buffer): bias, ReLU, BF16 stores
-  auto drain = [&](int buf, uint32_t use) {
+
+  // tile t = ((b*nz + z)*tx + xb)*ny + y; 32-bit indices (a grid has fewer than 2^31 tiles)
+  const int tx = nx / 128, ntiles = tx * ny * nz * nb;
+  int t = (int)((int64_t)blockIdx.x * ntiles / gridDim.x);
+  const int t_hi = (int)((int64_t)(blockIdx.x + 1) * ntiles / gridDim.x);
+  const int64_t plane_step = (int64_t)nx * ny;
+  int y = t % ny;
+  const float *src;  // row y, this thread's voxel
+  uint4 *dst;        // its first unit of the output
+  bool ok[3], edge[3];
+  auto column = [&]() {  // what a column of tiles shares
+    const int col = t / ny, plane = col / tx, xb = col - plane * tx, z = plane % nz, x = xb * 128 + tid;
+    src = in + (int64_t)plane * plane_step + (int64_t)y * nx + x;
+    dst = reinterpret_cast<uint4 *>(out) + act_unit((int64_t)plane * ny + y, 0, x, nx);
+    const bool has = lane == 0 ? x > 0 : lane == 31 && x + 1 < nx;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      ok[p] = (unsigned)(z + p - 1) < (unsigned)nz;
+      edge[p] = ok[p] && has;
+    }
+  };
+  const int xe = lane ? 1 : -1;
+  // row y + dy of the three planes: this thread's element and, at a warp's ends, its outer neighbour's
+  float c[3], e[3];
+  auto load = [&](int dy) {
+    const bool row = (unsigned)(y + dy) < (unsigned)ny;
+    const float *q = src + (int64_t)dy * nx - plane_step;
+#pragma unroll
+    for (int p = 0; p < 3; ++p, q += plane_step) {
+      c[p] = row && ok[p] ? __ldg(q) : 0.f;
+      e[p] = row && edge[p] ? __ldg(q + xe) : 0.f;
+    }
+  };
+  // the taps (x-1, x, x+1) of the loaded rows: BF16 in the low half of v[plane][slot][dx]
+  uint32_t v[3][3][3];
+  const uint32_t left = lane == 0 ? 0x0076u : 0x0010u, right = lane == 31 ? 0x0076u : 0x0010u;  // neighbour's | own outer
+  auto taps = [&](int slot_) {
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+      const __nv_bfloat162 h = __floats2bfloat162_rn(c[p], e[p]);
+      const uint32_t m = *reinterpret_cast<const uint32_t *>(&h);
+      v[p][slot_][0] = __byte_perm(__shfl_up_sync(0xffffffffu, m, 1), m, left);
+      v[p][slot_][1] = m;
+      v[p][slot_][2] = __byte_perm(__shfl_down_sync(0xffffffffu, m, 1), m, right);
+    }
+  };
+  // bias, ReLU and stores of a tile: accumulator buf in its use-th use
+  auto drain = [&](uint4 *o, int buf, uint32_t use) {
     if (!mbar_wait(&done[buf], use & 1u, err, 31)) s_fail = 1;
     tc_fence_after();
-    float v[16];
-    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * 16), v);
+    float a[16];
+    tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * 16), a);
     tc_fence_before();
-    const int x = D.xb * 128 + tid;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const float4 b0 = *reinterpret_cast<const float4 *>(sBias + 8 * h);
-      const float4 b1 = *reinterpret_cast<const float4 *>(sBias + 8 * h + 4);
-      const float bc[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
       uint32_t w[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float lo = v[8 * h + 2 * c] + bc[2 * c], hi = v[8 * h + 2 * c + 1] + bc[2 * c + 1];
+      for (int k = 0; k < 2; ++k) {
+        const float4 b = reinterpret_cast<const float4 *>(sBias)[2 * h + k];
+        __nv_bfloat162 p0 = __floats2bfloat162_rn(a[8 * h + 4 * k] + b.x, a[8 * h + 4 * k + 1] + b.y);
+        __nv_bfloat162 p1 = __floats2bfloat162_rn(a[8 * h + 4 * k + 2] + b.z, a[8 * h + 4 * k + 3] + b.w);
         if (relu) {
-          lo = fmaxf(lo, 0.f);
-          hi = fmaxf(hi, 0.f);
+          p0 = __hmax2(p0, __float2bfloat162_rn(0.f));
+          p1 = __hmax2(p1, __float2bfloat162_rn(0.f));
         }
-        const __nv_bfloat162 pr = __floats2bfloat162_rn(lo, hi);
-        w[c] = *reinterpret_cast<const uint32_t *>(&pr);
+        w[2 * k] = *reinterpret_cast<const uint32_t *>(&p0);
+        w[2 * k + 1] = *reinterpret_cast<const uint32_t *>(&p1);
       }
-      *reinterpret_cast<uint4 *>(out + act_unit(D.row, h, x, nx) * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+      o[(int64_t)h * nx] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    D.next(tx, ny, nz);
   };
   int it = 0;
-  for (int t = t_lo; t < t_hi; ++t, ++it) {
+  uint4 *prev = nullptr;  // the tile whose MMAs run
+  uint8_t *const arow = sA[0] + (tid >> 3) * 128 + (tid & 7) * 16;
+  // One tile; rows y-1, y, y+1 are in slots R, R+1, R+2 (mod 3).  False: the range's last, or a wait ran out.
+  auto step = [&](auto rot) -> bool {
+    constexpr int R = decltype(rot)::value;
     const int buf = it & 1;
-    // this thread's voxel: 27 taps from the staged lines
-    const float *s = sL[buf] + tid;
-    float v[32];
+    load(2);  // the next tile's new row, in flight until the end of this one
 #pragma unroll
-    for (int l = 0; l < 9; ++l)
-#pragma unroll
-      for (int dx = 0; dx < 3; ++dx) v[l * 3 + dx] = s[l * kIn1Line + dx];
-#pragma unroll
-    for (int k = 27; k < 32; ++k) v[k] = 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
+    for (int k = 0; k < 4; ++k) {
       uint32_t w[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const __nv_bfloat162 pr = __floats2bfloat162_rn(v[8 * c + 2 * j], v[8 * c + 2 * j + 1]);
-        w[j] = *reinterpret_cast<const uint32_t *>(&pr);
+        const int i = 8 * k + 2 * j;
+        if (i > 26)
+          w[j] = 0;
+        else if (i == 26)
+          w[j] = v[2][(R + 2) % 3][2] & 0xffffu;
+        else
+          w[j] = __byte_perm(v[i / 9][(R + i / 3) % 3][i % 3], v[(i + 1) / 9][(R + (i + 1) / 3) % 3][(i + 1) % 3], 0x5410);
       }
-      *reinterpret_cast<uint4 *>(sA[buf] + c * 2048 + (tid >> 3) * 128 + (tid & 7) * 16) =
-          make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4 *>(arow + buf * kIn1ABytes + k * 2048) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    stage(buf ^ 1);        // tile t+1's lines: that buffer was last read before the previous barrier
-    load(t + 2 < t_hi);    // tile t+2's elements, in flight until the next iteration's stage
     fence_proxy_async_smem();  // the A rows -> tensor-core proxy
     tc_fence_before();
-    __syncthreads();  // A and the next lines written; the drain of this buffer's last tile is done
+    __syncthreads();  // A written; the drain of this buffer's last tile is done
     tc_fence_after();
-    if (s_fail) break;  // read by every thread after the same barrier
+    if (s_fail) return false;  // read by every thread after the same barrier
     if (tid == 0) {
       const uint64_t ad = smem_desc(sA[buf], 2048, 128);
       const uint32_t d = tmem + (uint32_t)(buf * 16);
@@ -389,9 +375,37 @@ __global__ void __launch_bounds__(kIn1Threads) k_conv3_in1_tc(const float *in, c
       mma_bf16(d, ad + (uint64_t)(4096 >> 4), bd + (uint64_t)(512 >> 4), idesc, 1u);
       mma_commit(&done[buf]);
     }
-    if (it > 0) drain(buf ^ 1, (uint32_t)((it - 1) >> 1));
+    if (it > 0) drain(prev, buf ^ 1, (uint32_t)((it - 1) >> 1));
+    prev = dst;
+    ++it;
+    if (++t >= t_hi) return false;
+    src += nx;
+    dst += 2 * nx;
+    if (++y < ny) {
+      taps(R);  // the oldest row's slot
+    } else {
+      y = 0;
+      column();
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        load(r - 1);
+        taps((R + 1 + r) % 3);
+      }
+    }
+    return true;
+  };
+  if (t < t_hi) {
+    column();
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      load(r - 1);
+      taps(r);
+    }
+    while (step(std::integral_constant<int, 0>()) && step(std::integral_constant<int, 1>()) &&
+           step(std::integral_constant<int, 2>())) {
+    }
   }
-  if (it > 0 && !s_fail) drain((it - 1) & 1, (uint32_t)((it - 1) >> 1));
+  if (it > 0 && !s_fail) drain(prev, (it - 1) & 1, (uint32_t)((it - 1) >> 1));
   if (tid == 0) {  // every MMA this thread issued has completed before TMEM is freed
     mma_commit(&fin);
     mbar_wait(&fin, 0, err, 32);
@@ -409,7 +423,7 @@ int launch_conv3_in1_tc(const float *in, const float *W, const float *bias, __nv
   if (nx % 128 || ny < 1 || nz < 1 || nb < 1) return HPCCG_ERR_UNSUPPORTED;
   const int64_t ntiles = (int64_t)(nx / 128) * ny * nz * nb;
   if (ntiles >= ((int64_t)1 << 31)) return HPCCG_ERR_TOO_LARGE;
-  const int grid = (int)std::min<int64_t>(ntiles, (int64_t)num_sms * 8);
+  const int grid = (int)std::min<int64_t>(ntiles, (int64_t)num_sms * kIn1PerSm);
   k_conv3_in1_tc<<<grid, kIn1Threads, 0, s>>>(in, W, bias, out, nx, ny, nz, nb, relu, err);
   HPCCG_CUDA(cudaGetLastError());
   return HPCCG_OK;

@@ -108,6 +108,23 @@ def test_input_layer_tc_and_cc(env, nx, ny, nz, nb, epi):
         assert np.all(np.abs(got - want) <= tol), (path, np.abs(got - want).max(), scale)
 
 
+@pytest.mark.parametrize("nx,ny,nz,nb", [(128, 1, 1900, 1), (128, 7, 200, 2), (384, 37, 29, 1)])
+def test_input_layer_tc_column_changes(env, nx, ny, nz, nb):
+    """More tiles than CTAs, so that a CTA's range crosses columns of tiles (every tile with ny = 1),
+    planes, x blocks and grids of the batch: the bar of test_input_layer_tc_and_cc."""
+    torch, hp = env
+    rng = np.random.default_rng(nz)
+    x = rng.normal(0, 1, (nb, nz, ny, nx)).astype(np.float32)
+    W = rng.normal(0, 0.2, (27, 1, 16)).astype(np.float32)
+    b = rng.normal(0, 0.1, 16).astype(np.float32)
+    want = uo.conv3(uo.bf16_round(x)[..., None].astype(np.float64), uo.bf16_round(W).astype(np.float64)) + b
+    out = torch.full((nb, nz, ny, 2, nx, 8), float("nan"), dtype=torch.bfloat16, device="cuda")
+    hp.conv3_layer(torch.from_numpy(x).cuda(), None, torch.from_numpy(W).cuda(), torch.from_numpy(b).cuda(), None, 1, 0,
+                   out, nx, ny, nz, nb, nin=0)
+    got = from_planar(out.float().cpu().numpy().astype(np.float64))
+    assert np.all(np.abs(got - want) <= 1e-3 * np.abs(want).max() + 2.0 ** -8 * np.abs(want))
+
+
 @pytest.mark.parametrize("nx,ny,nz,nb", [(128, 9, 1, 1), (128, 1, 3, 1), (384, 10, 2, 1), (64, 18, 5, 1), (32, 12, 9, 2),
                                          (16, 8, 17, 1), (8, 16, 9, 2)])
 @pytest.mark.parametrize("nin", [1, 2])
