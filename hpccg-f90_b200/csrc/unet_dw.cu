@@ -40,9 +40,10 @@ using namespace tc;
 //
 // Against the CUDA-core kernel it replaces (one thread per (tap, ci), each
 // re-reading its input voxel from global memory): the 13 layers of a 64^3,
-// batch 4 training step 25.7 -> 0.62 ms (a 16-channel layer at 64^3, batch 4:
-// 6.24 -> 0.12 ms), of which the MMAs are about a third and start-up, drain and
-// the first copies of each unit the rest.
+// batch 4 training step 25.7 -> 0.29 ms (the 1-channel layer's 0.05 included).
+// Issued by a branch for one lane the MMAs took 0.09 ms more: the gradient of
+// that step 1.15 -> 1.05 ms, of 64^3 641 -> 610 us, of 32^3 493 -> 465.  Bound by
+// the MMAs, then by start-up, drain and the first copies of each unit.
 constexpr int kDwThreads = 192;  // producer warp, MMA warp, four draining warps
 constexpr int kDwRows = 8;   // y rows per unit
 constexpr int kDwSlots = 4;  // X slabs in flight
@@ -79,7 +80,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__
   __shared__ uint32_t slot;
   constexpr int P = dw_planes(NIN);
   const ConvGeom &g = a.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int ps = dw_plane_bytes(a.kx), slab = P * ps, dyb = dw_dy_bytes(a.kx);
   uint8_t *sY = smem, *sX = smem + 2 * dyb;
   for (int s = 0; s < kDwSlots; ++s) {  // the ones planes: written once, no copy touches them
@@ -148,42 +149,48 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__
       for (uint32_t j = uc > 2u ? uc - 2 : 0; j < uc; ++j) mbar_wait(&fully[j & 1], (j >> 1) & 1, a.err, 44);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = idesc_bf16_mn(128, 48);
-      uint32_t sc = 0, uc = 0, cc = 0;  // rows, units, chunks of rows
-      int in_chunk = 0;
-      bool ok = true;
-      for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x, ++uc) {
-        int b, z, ya, yb, x0;
-        unit(u, b, z, ya, yb, x0);
-        if (!(ok = mbar_wait(&fully[uc & 1], (uc >> 1) & 1, a.err, 45))) break;
-        for (int y = ya; y < yb; ++y, ++sc) {
-          const int s = sc % kDwSlots;
-          if (in_chunk == 0 && cc >= 2 && !(ok = mbar_wait(&acc_empty[cc & 1], ((cc >> 1) - 1) & 1, a.err, 48))) break;
-          if (!(ok = mbar_wait(&fullx[s], (sc / kDwSlots) & 1, a.err, 46))) break;
-          tc_fence_after();
-          const uint32_t d = tmem + 256 * (cc & 1);
-          // MN-major: lbo = distance of 8-voxel groups (K), sbo = of 8-channel groups
-          uint64_t ad = smem_desc(sX + s * slab, 128, ps);
-          uint64_t bd = smem_desc(sY + (uc & 1) * dyb + (y - ya) * 2 * a.kx * 16, 128, a.kx * 16);
-          for (int k = 0; k < ksteps; ++k, ad += 16, bd += 16)
+    // the whole warp walks the rows; one lane issues (a branch for one lane takes ~70 cycles an
+    // MMA to issue, more than the 46 that it runs)
+    const uint32_t leader = elect_one();
+    constexpr uint32_t idesc = idesc_bf16_mn(128, 48);
+    // MN-major: lbo = distance of 8-voxel groups (K), sbo = of 8-channel groups
+    const uint64_t ad0 = smem_desc(sX, 128, ps), bd0 = smem_desc(sY, 128, a.kx * 16);
+    const uint32_t slab16 = slab >> 4, dyb16 = dyb >> 4, dyrow16 = 2 * a.kx;
+    uint32_t uc = 0, cc = 0, sl = 0, par = 0;  // units, chunks of rows; X ring
+    int in_chunk = 0;
+    bool ok = true;
+    for (int u = blockIdx.x; u < a.nunits && ok; u += gridDim.x, ++uc) {
+      int b, z, ya, yb, x0;
+      unit(u, b, z, ya, yb, x0);
+      if (!(ok = mbar_wait(&fully[uc & 1], (uc >> 1) & 1, a.err, 45))) break;
+      uint64_t brow = bd0 + (uint64_t)((uc & 1) * dyb16);
+      for (int y = ya; y < yb; ++y, brow += dyrow16) {
+        if (in_chunk == 0 && cc >= 2 && !(ok = mbar_wait(&acc_empty[cc & 1], ((cc >> 1) - 1) & 1, a.err, 48))) break;
+        if (!(ok = mbar_wait(&fullx[sl], par, a.err, 46))) break;
+        tc_fence_after();
+        const uint32_t d = tmem + 256 * (cc & 1);
+        uint64_t ad = ad0 + (uint64_t)(sl * slab16), bd = brow;
+        uint32_t more = in_chunk > 0;
+        for (int k = 0; k < ksteps; ++k, ad += 16, bd += 16, more = 1)
 #pragma unroll
-            for (int dx = 0; dx < 3; ++dx)
-              mma_bf16(d + 48 * dx, ad + dx, bd, idesc, in_chunk > 0 || k > 0 ? 1u : 0u);
-          mma_commit(&emptyx[s]);
-          if (++in_chunk == chunk) {
-            mma_commit(&acc_full[cc & 1]);
-            in_chunk = 0;
-            ++cc;
-          }
+          for (int dx = 0; dx < 3; ++dx) mma_bf16_warp(d + 48 * dx, ad + dx, bd, idesc, more, leader);
+        mma_commit_warp(&emptyx[sl], leader);
+        if (++sl == kDwSlots) {
+          sl = 0;
+          par ^= 1;
         }
-        if (!ok) break;
-        mma_commit(&emptyy[uc & 1]);
+        if (++in_chunk == chunk) {
+          mma_commit_warp(&acc_full[cc & 1], leader);
+          in_chunk = 0;
+          ++cc;
+        }
       }
-      if (ok && in_chunk) mma_commit(&acc_full[cc & 1]);
-      mma_commit(&drain);
-      mbar_wait(&drain, 0, a.err, 47);
+      if (!ok) break;
+      mma_commit_warp(&emptyy[uc & 1], leader);
     }
+    if (ok && in_chunk) mma_commit_warp(&acc_full[cc & 1], leader);
+    mma_commit_warp(&drain, leader);
+    mbar_wait(&drain, 0, a.err, 47);
   } else {
     int rows = 0;
     for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
