@@ -23,6 +23,7 @@
 
 #include <algorithm>
 #include <type_traits>
+#include <map>
 #include <vector>
 
 #include "hpccg_internal.cuh"
@@ -58,6 +59,13 @@ struct BatchArgs {
   const int4 *pieces;       // (system, first row, end row, -) of each block of k_batch_r32
   const int *piece0;        // nsys+1 prefix
   float *p32b;              // the second p buffer
+  // box walks of stored batches (null: not in use)
+  const int4 *btiles;       // (system, first column, z0, z1) of each block of k_batch_box
+  const int4 *bdims;        // (nx, ny, nz, first row) per system
+  const int2 *bgroup;       // (first box, boxes) per system
+  const uint16_t *bcode;    // each row's box in its system's group
+  const double *box64;
+  const float *box_lp;
   double *part;             // one partial per chunk (per block in the tiled iteration)
   unsigned *counter;        // [0] blocks of a phase that have arrived, [1 + s] partials of system s that have
   BatchSys *sys;
@@ -76,7 +84,7 @@ __device__ __forceinline__ double row_fp64(const BatchArgs &g, int i, int sys, c
     return stencil_row<double>(i - d.w, StencilGeom{d.x, d.y, d.z}, x + d.w);
   }
   double s = 0.0;
-  if (g.code) {  // row patterns: the same terms and order (32 systems, edges 16 to 64: 141 -> 74 us a phase)
+  if (g.code) {  // row patterns: the same terms and order (32 systems, edges 16 to 64: 141 -> 68 us a phase)
     const PatEntry64 *t = g.pat + (size_t)g.code[i] * kPatW;
 #pragma unroll
     for (int k = 0; k < 27; ++k) {
@@ -445,6 +453,64 @@ __global__ void __launch_bounds__(256, 4) k_batch_walk64(BatchArgs g, int all) {
     walk(g.x, WalkResidual{g.b + w.d.w, g.r + w.d.w});
   else
     walk(g.p, WalkStore{g.Ap + w.d.w});
+}
+
+// ---- box walks of stored batches on known grids -------------------------------------
+// A p, r = b - A x (FP64) or A p of the inner solves (FP32) where every row is a
+// pattern of its system's grid: a block walks up to 256 columns of one system along z
+// with that grid's boxes in shared memory (box_walk), instead of 27 table entries and 27
+// gathers a row.  Sums and bits are those of the ELL rows.  32 systems, edges 16 to
+// 64 (2.1M rows): the phase 68 -> 28 us and 8 for the dot product's own pass, bound by
+// the chain of additions of a row and its plane loads at 5 to 8 blocks an SM.
+template <typename Real, bool RES>
+__global__ void __launch_bounds__(256) k_batch_box(BatchArgs g, int all) {
+  constexpr bool kFp64 = sizeof(Real) == 8;
+  const int4 t = g.btiles[blockIdx.x];
+  if (!(kFp64 ? all || g.sys[t.x].active : g.sys[t.x].inner_active)) return;
+  const int4 d = g.bdims[t.x];
+  const int2 grp = g.bgroup[t.x];
+  const Real *table, *x;
+  if constexpr (kFp64) {
+    table = g.box64;
+    x = RES ? g.x : g.p;
+  } else {
+    table = g.box_lp;
+    x = g.p32;
+  }
+  const Real *local = box_table(table + (size_t)grp.x * kPatW, grp.y);
+  const int plane = d.x * d.y, c = t.y + threadIdx.x;
+  if (c >= plane) return;
+  const int iy = c / d.x, ix = c - iy * d.x;
+  const unsigned mask = stencil_mask(StencilGeom{d.x, d.y, d.z}, ix, iy);
+  const Real *xc = x + d.w + c;
+  box_walk<Real, 1>(c, t.z, t.w, d.x, plane, d.z, g.bcode + d.w, local,
+                    [&](int p, Real *v) {
+                      stencil_plane<Real>(xc + (int64_t)p * plane, d.x, mask, (unsigned)p < (unsigned)d.z, v);
+                      return true;
+                    },
+                    [&](int i, Real sum, Real) {
+                      if constexpr (!kFp64)
+                        g.Ap32[d.w + i] = sum;
+                      else if constexpr (RES)
+                        g.r[d.w + i] = __dsub_rn(g.b[d.w + i], sum);
+                      else
+                        g.Ap[d.w + i] = sum;
+                    });
+}
+
+// The patterns of the rows [0, n) belong to the grid `key`; *bad where one has another.
+__global__ void k_batch_box_owner(const uint16_t *code, int n, unsigned long long key, unsigned long long *owner,
+                                  int *bad) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    unsigned long long *o = owner + code[i];
+    unsigned long long have = *(volatile unsigned long long *)o;
+    if (have == 0) have = atomicCAS(o, 0ull, key);
+    if (have != 0 && have != key) *bad = 1;
+  }
+}
+__global__ void k_batch_box_code(const uint16_t *code, int n, const int4 *place, uint16_t *bcode) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    bcode[i] = (uint16_t)place[code[i]].w;
 }
 
 // The same for the FP32 inner solves, rows as 28 x - (plane box sums), the
@@ -939,6 +1005,10 @@ struct hpccg_batch {
   int spmv_kind = HPCCG_SPMV_ELL;
   RowPatterns pat;         // of the stacked matrix, looked for by the first stored-matrix solve
   bool pat_tried = false;
+  int4 *d_btiles = nullptr;  // box walks (null: not in use)
+  int2 *d_bgroup = nullptr;
+  uint16_t *bcode = nullptr;
+  int nbtiles = 0;
   int ntiles = 0;
   int tile_chunks = 0, blocks_per_sm = 0;  // schedule; 0 = not tuned yet
   bool tuned = false;
@@ -953,7 +1023,7 @@ static void batch_free(hpccg_batch *B) {
     if (e) cudaGraphExecDestroy(e);
   void *bufs[] = {B->col, B->val, B->val32, B->val16, B->x, B->b, B->r, B->p, B->Ap, B->r32, B->p32,
                   B->Ap32, B->d32, B->part, B->counter, B->sys, B->d_sys_chunk0, B->d_tiles, B->d_dims, B->d_walk,
-                  B->d_wtiles, B->d_pieces, B->d_wtile0, B->d_piece0, B->p32b};
+                  B->d_wtiles, B->d_pieces, B->d_wtile0, B->d_piece0, B->p32b, B->d_btiles, B->d_bgroup, B->bcode};
   for (void *q : bufs)
     if (q) cudaFree(q);
   free_patterns(&B->pat);
@@ -1201,6 +1271,14 @@ static BatchArgs batch_args(hpccg_batch *B, int precision) {
   g.sys = B->sys;
   g.dims = B->spmv_kind == HPCCG_SPMV_STENCIL ? B->d_dims : nullptr;
   g.walk = B->d_walk;
+  if (!g.dims && B->d_btiles) {
+    g.btiles = B->d_btiles;
+    g.bdims = B->d_dims;
+    g.bgroup = B->d_bgroup;
+    g.bcode = B->bcode;
+    g.box64 = B->pat.box64;
+    g.box_lp = precision == HPCCG_PREC_BF16 ? B->pat.box16 : B->pat.box32;
+  }
   if (g.dims && B->p32b) {
     g.wtiles = B->d_wtiles;
     g.wtile0 = B->d_wtile0;
@@ -1227,10 +1305,15 @@ static cudaError_t phase(hpccg_batch *B, const BatchArgs &g, cudaStream_t s) {
 static int walk_grid(const hpccg_batch *B) { return (int)((B->walk_total + 255) / 256); }
 
 // Ap = A p and alpha: one phase on the stored matrix, a column walk and a dot
-// phase on matrix-free rows.
+// phase on matrix-free rows and where the patterns have boxes.
 static cudaError_t launch_spmv_dot64(hpccg_batch *B, const BatchArgs &g, cudaStream_t s) {
   if (g.dims && g.walk && B->walk_total > 0) {
     k_batch_walk64<false><<<walk_grid(B), 256, 0, s>>>(g, 0);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? phase<PhDot64>(B, g, s) : e;
+  }
+  if (g.btiles) {
+    k_batch_box<double, false><<<B->nbtiles, 256, 0, s>>>(g, 0);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? phase<PhDot64>(B, g, s) : e;
   }
@@ -1249,8 +1332,12 @@ static cudaError_t launch_cg64_body(hpccg_batch *B, const BatchArgs &g, cudaStre
 // on matrix-free rows (11.2M rows: 205 -> 122 us).
 template <class Ph>
 static cudaError_t launch_residual64(hpccg_batch *B, const BatchArgs &g, cudaStream_t s, bool all) {
-  if (!(g.dims && g.walk && B->walk_total > 0)) return phase<Ph>(B, g, s);
-  k_batch_walk64<true><<<walk_grid(B), 256, 0, s>>>(g, all ? 1 : 0);
+  if (g.btiles)
+    k_batch_box<double, true><<<B->nbtiles, 256, 0, s>>>(g, all ? 1 : 0);
+  else if (g.dims && g.walk && B->walk_total > 0)
+    k_batch_walk64<true><<<walk_grid(B), 256, 0, s>>>(g, all ? 1 : 0);
+  else
+    return phase<Ph>(B, g, s);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? phase<PhSquare64<Ph>>(B, g, s) : e;
 }
@@ -1265,8 +1352,11 @@ static cudaError_t launch_inner_body(hpccg_batch *B, const BatchArgs &g, cudaStr
   k_batch_p32<<<grid_of(B), 256, 0, s>>>(g);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {
-    if (g.dims && g.walk && B->walk_total > 0) {
-      k_batch_walk32<<<walk_grid(B), 256, 0, s>>>(g);
+    if (g.btiles || (g.dims && g.walk && B->walk_total > 0)) {
+      if (g.btiles)
+        k_batch_box<float, false><<<B->nbtiles, 256, 0, s>>>(g, 0);
+      else
+        k_batch_walk32<<<walk_grid(B), 256, 0, s>>>(g);
       e = cudaGetLastError();
       if (e == cudaSuccess) e = phase<PhDotLp>(B, g, s);
     } else {
@@ -1613,6 +1703,98 @@ extern "C" int hpccg_batch_spmv(hpccg_batch *B, const double *d_x, double *d_y) 
   return HPCCG_OK;
 }
 
+// Box walks where the systems' grids are known, every pattern belongs to one (nx, ny)
+// and its entries lie at the neighbours, at most kPatLocal patterns to a grid.  Not for
+// small batches, where the phase's 27 gathers hide in the launches that a walk with its
+// own dot product doubles: 100 thousand rows 1.13 ms a solve with patterns, 1.14 with
+// boxes (FP32 1.29, 1.36), 336 thousand 1.69, 1.56, 980 thousand 2.65, 2.01.
+constexpr int kBoxRowsPerSm = 2048;
+static int batch_boxes(hpccg_batch *B) {
+  if (!B->pat.count || !B->d_dims || B->npad < kBoxRowsPerSm * B->num_sms) return HPCCG_OK;
+  const int count = B->pat.count;
+  for (const int4 &d : B->h_dims)
+    if (d.x < 3 || d.y < 3) return HPCCG_OK;  // narrower: neighbours' offsets coincide
+  void *scratch = nullptr;  // owners, then places; the flag behind them
+  const size_t place_bytes = sizeof(int4) * count;
+  if (cudaMalloc(&scratch, place_bytes + sizeof(int)) != cudaSuccess) {
+    cudaGetLastError();
+    return HPCCG_OK;  // without room for the boxes the patterns serve
+  }
+  unsigned long long *owner = static_cast<unsigned long long *>(scratch);
+  int4 *place = static_cast<int4 *>(scratch);
+  int *d_bad = reinterpret_cast<int *>(place + count), bad = 1;
+  std::vector<unsigned long long> own(count);
+  auto key = [](const int4 &d) { return (unsigned long long)(unsigned)d.x << 32 | (unsigned)d.y; };
+  cudaError_t e = cudaMemsetAsync(scratch, 0, place_bytes + sizeof(int), B->stream);
+  for (int s = 0; s < B->nsys && e == cudaSuccess; ++s) {
+    k_batch_box_owner<<<B->num_sms, 256, 0, B->stream>>>(B->pat.code + B->off[s], B->n[s], key(B->h_dims[s]), owner, d_bad);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(own.data(), owner, 8 * (size_t)count, cudaMemcpyDeviceToHost, B->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, B->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
+  int rc = HPCCG_OK;
+  if (e == cudaSuccess && !bad) {
+    std::vector<int> order(count);
+    for (int c = 0; c < count; ++c) order[c] = c;
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return own[a] < own[b]; });
+    std::vector<int4> pl(count, make_int4(0, 0, 0, 0));
+    std::map<unsigned long long, int2> groups;
+    for (int i = 0; i < count; ++i) {
+      const int c = order[i];
+      if (!own[c]) continue;  // a pattern of padding rows only
+      int2 &grp = groups.emplace(own[c], make_int2(i, 0)).first->second;
+      pl[c] = make_int4((int)(own[c] >> 32), (int)(own[c] & 0xffffffffu), i, grp.y++);
+      bad |= grp.y > kPatLocal;
+    }
+    std::vector<int2> sysgrp(B->nsys);
+    for (int s = 0; s < B->nsys; ++s) sysgrp[s] = groups[key(B->h_dims[s])];
+    if (!bad) {
+      e = cudaMemcpyAsync(place, pl.data(), place_bytes, cudaMemcpyHostToDevice, B->stream);
+      if (e == cudaSuccess) rc = pattern_boxes_placed(&B->pat, place, B->stream);
+      if (e == cudaSuccess && !rc && B->pat.boxes) {
+        // planes a block walks: the most that still give every SM five blocks (32
+        // systems, edges 16 to 64: 3.50 ms with 8, 3.63 with 16, 3.74 with 4; 64 systems,
+        // edges 30 to 78: 16.6 with 16, 17.1 with 8, 17.0 with 32)
+        std::vector<int4> tiles;
+        for (int zc : {16, 8, 4}) {
+          tiles.clear();
+          for (int s = 0; s < B->nsys; ++s) {
+            const int4 d = B->h_dims[s];
+            for (int z = 0; z < d.z; z += zc)
+              for (int c = 0; c < d.x * d.y; c += 256) tiles.push_back(make_int4(s, c, z, std::min(d.z, z + zc)));
+          }
+          if ((int)tiles.size() >= 5 * B->num_sms) break;
+        }
+        B->nbtiles = (int)tiles.size();
+        const size_t tb = sizeof(int4) * tiles.size(), gb = sizeof(int2) * B->nsys;
+        e = cudaMalloc(&B->bcode, sizeof(uint16_t) * B->npad);
+        if (e == cudaSuccess) e = cudaMalloc(&B->d_bgroup, gb);
+        if (e == cudaSuccess) e = cudaMalloc(&B->d_btiles, tb);
+        if (e == cudaErrorMemoryAllocation) {  // no room: the patterns serve
+          cudaGetLastError();
+          void *part[] = {B->bcode, B->d_bgroup};
+          for (void *q : part)
+            if (q) cudaFree(q);
+          B->bcode = nullptr;
+          B->d_bgroup = nullptr;
+          B->d_btiles = nullptr;
+          e = cudaSuccess;
+        } else if (e == cudaSuccess) {
+          k_batch_box_code<<<B->num_sms * 8, 256, 0, B->stream>>>(B->pat.code, B->npad, place, B->bcode);
+          e = cudaGetLastError();
+          if (e == cudaSuccess) e = cudaMemcpyAsync(B->d_bgroup, sysgrp.data(), gb, cudaMemcpyHostToDevice, B->stream);
+          if (e == cudaSuccess) e = cudaMemcpyAsync(B->d_btiles, tiles.data(), tb, cudaMemcpyHostToDevice, B->stream);
+          if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
+        }
+      }
+    }
+  }
+  cudaFree(scratch);
+  HPCCG_CUDA(e);
+  return rc;
+}
+
 // The solve of hpccg_batch_solve; b and x are copied in with `in` and the
 // solution out with `out` (device-to-device for device vectors, host-to-device
 // and device-to-host for host arrays).
@@ -1627,6 +1809,7 @@ static int batch_solve(hpccg_batch *B, const double *d_b, double *d_x, cudaMemcp
   if (B->spmv_kind != HPCCG_SPMV_STENCIL && !B->pat_tried) {
     B->pat_tried = true;
     if ((rc = row_patterns(B->col, B->val, B->npad, B->npad, kBatchPatterns, B->num_sms, B->stream, &B->pat))) return rc;
+    if ((rc = batch_boxes(B))) return rc;
   }
   if ((rc = autotune(B))) return rc;
   if (precision != HPCCG_PREC_FP64 && B->spmv_kind != HPCCG_SPMV_STENCIL && !B->pat.count &&

@@ -175,11 +175,19 @@ int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n,
 }
 
 // One thread per pattern: its entries (without the padding slots, offset 0 and value
-// +0.0, at the end) at their places of the 3x3x3 box, in order; *bad where one has none.
-__global__ void k_pat_boxes(const PatEntry64 *t64, int count, int nx, int ny, double *box64, float *box32,
-                            float *box16, int *bad) {
+// +0.0, at the end) at their places of the 3x3x3 box, in order; *bad where one has none.  place (may be null): each
+// pattern's own (nx, ny, box number), nx = 0 for none.
+__global__ void k_pat_boxes(const PatEntry64 *t64, int count, int nx, int ny, const int4 *place, double *box64,
+                            float *box32, float *box16, int *bad) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= count) return;
+  int at = c;
+  if (place) {
+    nx = place[c].x;
+    ny = place[c].y;
+    at = place[c].z;
+    if (nx == 0) return;
+  }
   const PatEntry64 *row = t64 + (size_t)c * kPatW;
   int len = kPatW;
   while (len > 0 && row[len - 1].off == 0 && __double_as_longlong(row[len - 1].v) == 0) --len;
@@ -189,21 +197,32 @@ __global__ void k_pat_boxes(const PatEntry64 *t64, int count, int nx, int ny, do
     const bool have = k < len && row[k].off == off;
     const double v = have ? row[k].v : 0.0;
     k += have;
-    box64[(size_t)c * kPatW + j] = v;
-    box32[(size_t)c * kPatW + j] = (float)v;
-    box16[(size_t)c * kPatW + j] = __bfloat162float(__double2bfloat16(v));
+    box64[(size_t)at * kPatW + j] = v;
+    box32[(size_t)at * kPatW + j] = (float)v;
+    box16[(size_t)at * kPatW + j] = __bfloat162float(__double2bfloat16(v));
   }
   if (k != len) *bad = 1;
 }
+
+static int fill_boxes(RowPatterns *p, int nx, int ny, const int4 *place, cudaStream_t s);
 
 int pattern_boxes(RowPatterns *p, int nx, int ny, cudaStream_t s) {
   p->boxes = false;
   p->box_nx = nx;
   p->box_ny = ny;
   if (!p->count || nx < 3 || ny < 3) return HPCCG_OK;  // narrower: neighbours' offsets coincide
+  return fill_boxes(p, nx, ny, nullptr, s);
+}
+
+int pattern_boxes_placed(RowPatterns *p, const int4 *place, cudaStream_t s) {
+  p->boxes = false;
+  return p->count ? fill_boxes(p, 0, 0, place, s) : HPCCG_OK;
+}
+
+static int fill_boxes(RowPatterns *p, int nx, int ny, const int4 *place, cudaStream_t s) {
   int bad = 1;
   HPCCG_CUDA(cudaMemsetAsync(p->flag, 0, sizeof(int), s));
-  k_pat_boxes<<<(p->count + 31) / 32, 32, 0, s>>>(p->t64, p->count, nx, ny, p->box64, p->box32, p->box16, p->flag);
+  k_pat_boxes<<<(p->count + 31) / 32, 32, 0, s>>>(p->t64, p->count, nx, ny, place, p->box64, p->box32, p->box16, p->flag);
   HPCCG_CUDA(cudaGetLastError());
   HPCCG_CUDA(cudaMemcpyAsync(&bad, p->flag, sizeof(int), cudaMemcpyDeviceToHost, s));
   HPCCG_CUDA(cudaStreamSynchronize(s));

@@ -36,6 +36,9 @@ void free_patterns(RowPatterns *p);
 // (p->box64 and its roundings); p->boxes tells whether every one's entries lie
 // there in order.  Synchronises the stream.
 int pattern_boxes(RowPatterns *p, int nx, int ny, cudaStream_t s);
+// The same for patterns of several grids: place[c] = (nx, ny, box number) of pattern c, on
+// the device; nx = 0: no box.
+int pattern_boxes_placed(RowPatterns *p, const int4 *place, cudaStream_t s);
 
 __device__ __forceinline__ double pat_term(double s, const PatEntry64 &e, const double *__restrict__ x) {
   return __dadd_rn(s, __dmul_rn(e.v, __ldg(x + e.off)));  // the ELL kernels' operations

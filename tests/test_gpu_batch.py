@@ -108,6 +108,30 @@ def test_batch_from_csr_equals_generated(hp, torch):
     assert np.array_equal(out[0], out[1])
 
 
+@pytest.mark.parametrize("sizes", [
+    [(64, 64, 60), (3, 5, 90), (33, 17, 45), (40, 41, 39), (3, 3, 3), (300, 3, 9), (40, 41, 5), (257, 3, 1)],
+    [(31, 31, 31)] * 12 + [(9, 130, 4)],
+    [(128, 96, 40), (2, 7, 5)],
+])
+@pytest.mark.parametrize("prec", [FP64, FP32, BF16])
+def test_batch_box_walks_equal_patterns(hp, torch, sizes, prec):
+    """Generated batches large enough for box walks (the last one has a grid too narrow for
+    them) against the same systems from CSR, whose grids are not known: the same terms in
+    the same order, so the solutions and iterations agree bit for bit."""
+    sysl = _systems(sizes)
+    G = hp.Batch.generated(sizes)
+    C = hp.Batch.from_csr([(A.rowindex, A.colindex, A.values) for A, _, _ in sysl])
+    assert G.stacked_rows >= 2048 * torch.cuda.get_device_properties(0).multi_processor_count
+    db = torch.from_numpy(G.stack([b for _, b, _ in sysl])).cuda()
+    out = []
+    for B in (G, C):
+        dx = torch.zeros_like(db)
+        iters = B.solve(db, dx, prec, 1e-8, 300)[0]
+        out.append((dx.cpu().numpy(), np.asarray(iters)))
+    assert np.array_equal(out[0][1], out[1][1])
+    assert np.array_equal(out[0][0], out[1][0])
+
+
 def test_batch_spmv_bit_exact(hp, torch):
     sysl = _systems(SIZES)
     B = hp.Batch.generated(SIZES)
