@@ -15,12 +15,14 @@
 // graph's order.
 // An iteration, graph of the same pattern rows against this: 32^3 20.0 -> 8.4 us,
 // 64^3 26.5 -> 17.7, 97 x 75 x 61 28.6 -> 21.0, 100^3 40.7 -> 37.4, 128^3 65 -> 73,
-// hence kPersistRows.  At 32^3 it is bound by the two steps' round trips (two hops
+// hence kPersistRows; where the graph walks boxes 72^3 24.1 -> 22.2, 100 x 90 x 51 24.5
+// -> 24.1, 80^3 24.9 -> 26.2, 96^3 26.6 -> 34.8, hence kPersistBoxRows.  At 32^3 it is bound by the two steps' round trips (two hops
 // through L2 of about 1 us each and the sums on the way), above by the gathers.
 #include <algorithm>
 
 #include "hpccg_pattern.cuh"
 #include "hpccg_persist.cuh"
+#include "hpccg_rows.cuh"
 
 namespace hpccg {
 
@@ -254,7 +256,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_cg_persist(const __grid_constant
 }
 
 bool cg_persist_fits(const hpccg_ctx *c) {
-  return c->spmv_kind == kSpmvPattern && c->pat.count > 0 && c->nrow <= kPersistRows;
+  if (c->spmv_kind != kSpmvPattern || !c->pat.count) return false;
+  return c->nrow <= (spmv_args(c).pat_box ? kPersistBoxRows : kPersistRows);
 }
 
 int cg_persist(hpccg_ctx *c) {

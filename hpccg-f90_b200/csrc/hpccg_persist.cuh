@@ -6,6 +6,7 @@ namespace hpccg {
 
 // Rows up to which the one-kernel form runs (it wins at 1.0 million, loses at 2.1).
 constexpr int kPersistRows = 1 << 20;
+constexpr int kPersistBoxRows = 460000;  // where the graph's rows are box walks
 
 // Whether the context's CG runs in one kernel (its row kernel settled as row patterns).
 bool cg_persist_fits(const hpccg_ctx *c);

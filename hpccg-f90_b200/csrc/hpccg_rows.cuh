@@ -414,8 +414,9 @@ inline SpmvArgs spmv_args(const hpccg_ctx *c) {
   a.pat_count = c->pat.count;
   a.geom = StencilGeom{c->gx, c->gy, c->gz};
   a.pm = c->gx ? fp64_map(c->gx, c->gy, c->gz, c->num_sms) : PlaneMap{0, 0, 0, 1, 1, 0};
-  // worth it where the walk's blocks fill the SMs three times over (fewer: gathers)
-  a.pat_box = c->gx && a.pm.plane > 0 && plane_grid(a.pm) >= 3 * c->num_sms && c->pat.boxes ? c->pat.box64 : nullptr;
+  // worth it where every SM has a block of the walk (200 CG iterations, gathers | walk: 72^3
+  // with 135 blocks 4.83 | 4.90 ms, 96^3 with 216 7.19 | 5.32, 112^3 with 392 9.14 | 7.56)
+  a.pat_box = c->gx && a.pm.plane > 0 && plane_grid(a.pm) >= c->num_sms && c->pat.boxes ? c->pat.box64 : nullptr;
   a.tma_ok = a.pm.tiles_x > 0 && c->tmaps_ok;
   if (a.tma_ok) {
     a.tmap[0] = c->tmaps[0];

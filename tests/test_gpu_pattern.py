@@ -90,6 +90,12 @@ def _mixed_rows(rng, n, npat):
     return rowindex, np.concatenate(cols).astype(np.int32), np.concatenate([pats[p][1] for p in which])
 
 
+@pytest.mark.parametrize("nx,ny,nz", [(80, 80, 90), (96, 96, 96), (104, 104, 64), (131, 97, 60)])
+def test_box_walks_equal_ell_one_block_an_sm(env, nx, ny, nz):
+    """Grids whose walk has one block to two per SM, above the one-kernel CG's limit."""
+    test_box_walks_equal_ell(env, nx, ny, nz)
+
+
 @pytest.mark.parametrize("n,npat", [(100, 3), (1000, 32), (5001, 31), (5001, 33), (20000, 400)])
 def test_patterns_of_other_matrices(env, n, npat):
     """Matrices that are no stencil, up to and beyond the number of patterns kept
