@@ -981,7 +981,7 @@ struct hpccg_batch {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int nsys = 0;
   int npad = 0;
-  std::vector<int4> h_dims;         // generated batches: d_dims
+  std::vector<int4> h_dims;         // generated batches: d_dims (as long as the batch lives)
   std::vector<int> n, off, chunk0;  // per system rows, row offset, first chunk (host copies)
   int nchunks = 0;
   int32_t *col = nullptr;
@@ -1002,6 +1002,7 @@ struct hpccg_batch {
   int *d_wtile0 = nullptr, *d_piece0 = nullptr;
   float *p32b = nullptr;
   int nwtiles = 0, npieces = 0, wz = 0;
+  bool tiles_tried = false;
   int spmv_kind = HPCCG_SPMV_ELL;
   RowPatterns pat;         // of the stacked matrix, looked for by the first stored-matrix solve
   bool pat_tried = false;
@@ -1548,7 +1549,8 @@ __global__ void k_batch_to_lp(const double *src, float *f32, __nv_bfloat16 *b16,
 // columns of points), which keep the column walks, nor where the blocks would
 // outnumber the partials.
 static int ensure_tiles(hpccg_batch *B) {
-  if (B->p32b || B->h_dims.empty()) return HPCCG_OK;
+  if (B->tiles_tried || B->h_dims.empty()) return HPCCG_OK;
+  B->tiles_tried = true;
   std::vector<int4> wt, pc;
   std::vector<int> wt0(1, 0), pc0(1, 0);
   int64_t rows = 0, slots = 0;
@@ -1559,10 +1561,7 @@ static int ensure_tiles(hpccg_batch *B) {
   // 16 planes a block (two more are staged), fewer while the blocks do not fill the SMs
   int wz = 16;
   while (wz > 4 && slots / (kBtX * kBtY * wz) < 6 * (int64_t)B->num_sms) wz /= 2;
-  if (slots > 4 * rows) {
-    B->h_dims.clear();
-    return HPCCG_OK;
-  }
+  if (slots > 4 * rows) return HPCCG_OK;
   for (int s = 0; s < B->nsys; ++s) {
     const int4 &d = B->h_dims[s];
     for (int z = 0; z < d.z; z += wz)
@@ -1573,10 +1572,7 @@ static int ensure_tiles(hpccg_batch *B) {
     wt0.push_back((int)wt.size());
     pc0.push_back((int)pc.size());
   }
-  if ((int64_t)wt.size() > B->nchunks || (int64_t)pc.size() > B->nchunks) {
-    B->h_dims.clear();
-    return HPCCG_OK;
-  }
+  if ((int64_t)wt.size() > B->nchunks || (int64_t)pc.size() > B->nchunks) return HPCCG_OK;
   HPCCG_CUDA(cudaMalloc(&B->d_wtiles, sizeof(int4) * wt.size()));
   HPCCG_CUDA(cudaMalloc(&B->d_pieces, sizeof(int4) * pc.size()));
   HPCCG_CUDA(cudaMalloc(&B->d_wtile0, sizeof(int) * wt0.size()));

@@ -175,8 +175,10 @@ int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n,
 }
 
 // One thread per pattern: its entries (without the padding slots, offset 0 and value
-// +0.0, at the end) at their places of the 3x3x3 box, in order; *bad where one has none.  place (may be null): each
-// pattern's own (nx, ny, box number), nx = 0 for none.
+// +0.0, at the end) at their places of the 3x3x3 box, in order; *bad where one has none
+// or the grid is narrower than a box (its neighbours' offsets coincide, so that a place
+// would be found, but not always the right one).  place (may be null): each pattern's
+// own (nx, ny, box number), nx = 0 for none.
 __global__ void k_pat_boxes(const PatEntry64 *t64, int count, int nx, int ny, const int4 *place, double *box64,
                             float *box32, float *box16, int *bad) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -187,6 +189,10 @@ __global__ void k_pat_boxes(const PatEntry64 *t64, int count, int nx, int ny, co
     ny = place[c].y;
     at = place[c].z;
     if (nx == 0) return;
+  }
+  if (nx < 3 || ny < 3) {
+    *bad = 1;
+    return;
   }
   const PatEntry64 *row = t64 + (size_t)c * kPatW;
   int len = kPatW;
@@ -210,7 +216,7 @@ int pattern_boxes(RowPatterns *p, int nx, int ny, cudaStream_t s) {
   p->boxes = false;
   p->box_nx = nx;
   p->box_ny = ny;
-  if (!p->count || nx < 3 || ny < 3) return HPCCG_OK;  // narrower: neighbours' offsets coincide
+  if (!p->count || nx < 3 || ny < 3) return HPCCG_OK;  // k_pat_boxes would refuse it
   return fill_boxes(p, nx, ny, nullptr, s);
 }
 

@@ -132,6 +132,37 @@ def test_batch_box_walks_equal_patterns(hp, torch, sizes, prec):
     assert np.array_equal(out[0][0], out[1][0])
 
 
+@pytest.mark.parametrize("sizes", [
+    [(2, 40, 40)] * 60 + [(40, 2, 40)] * 50,
+    [(1, 40, 40)] * 120 + [(90, 1, 90)] * 20 + [(2, 2, 300)],
+    [(3, 3, 4000)] * 9 + [(3, 40, 9)],
+])
+def test_batch_stored_after_matrix_free(hp, torch, sizes):
+    """Narrow grids whose matrix-free FP32 solve does not suit the tiles, then the stored matrix
+    of the same batch: every precision against the same systems from CSR, bit for bit, and
+    against the oracle's true residual."""
+    sysl = _systems(sizes)
+    G = hp.Batch.generated(sizes)
+    C = hp.Batch.from_csr([(A.rowindex, A.colindex, A.values) for A, _, _ in sysl])
+    assert G.stacked_rows >= 2048 * torch.cuda.get_device_properties(0).multi_processor_count
+    db = torch.from_numpy(G.stack([b for _, b, _ in sysl])).cuda()
+    runs = [(G, hp.SPMV_STENCIL, FP32), (G, hp.SPMV_STENCIL, BF16)]
+    runs += [(B, hp.SPMV_ELL, prec) for prec in (FP64, FP32, BF16) for B in (G, C)]
+    out = []
+    for B, kind, prec in runs:
+        B.set_spmv(kind)
+        dx = torch.zeros_like(db)
+        _, relres, _, st = B.solve(db, dx, prec, 1e-8, 500)
+        assert st == hp.HPCCG_OK
+        x = dx.cpu().numpy()
+        for (A, b, _), xs, rr in zip(sysl, B.unstack(x), relres):
+            true = oracle.true_relres(A, b, xs)
+            assert true <= 1e-8 * (1 + 1e-6) and rr == pytest.approx(true, rel=1e-6)
+        out.append(x)
+    for k in (2, 4, 6):
+        assert np.array_equal(out[k], out[k + 1])
+
+
 def test_batch_spmv_bit_exact(hp, torch):
     sysl = _systems(SIZES)
     B = hp.Batch.generated(SIZES)
