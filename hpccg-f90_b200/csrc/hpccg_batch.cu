@@ -1762,26 +1762,34 @@ static int batch_boxes(hpccg_batch *B) {
           }
           if ((int)tiles.size() >= 5 * B->num_sms) break;
         }
-        B->nbtiles = (int)tiles.size();
+        // the batch takes the tables over once they are complete
         const size_t tb = sizeof(int4) * tiles.size(), gb = sizeof(int2) * B->nsys;
-        e = cudaMalloc(&B->bcode, sizeof(uint16_t) * B->npad);
-        if (e == cudaSuccess) e = cudaMalloc(&B->d_bgroup, gb);
-        if (e == cudaSuccess) e = cudaMalloc(&B->d_btiles, tb);
-        if (e == cudaErrorMemoryAllocation) {  // no room: the patterns serve
-          cudaGetLastError();
-          void *part[] = {B->bcode, B->d_bgroup};
+        uint16_t *bcode = nullptr;
+        int2 *group = nullptr;
+        int4 *btiles = nullptr;
+        e = cudaMalloc(&bcode, sizeof(uint16_t) * B->npad);
+        if (e == cudaSuccess) e = cudaMalloc(&group, gb);
+        if (e == cudaSuccess) e = cudaMalloc(&btiles, tb);
+        if (e == cudaSuccess) {
+          k_batch_box_code<<<B->num_sms * 8, 256, 0, B->stream>>>(B->pat.code, B->npad, place, bcode);
+          e = cudaGetLastError();
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(group, sysgrp.data(), gb, cudaMemcpyHostToDevice, B->stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(btiles, tiles.data(), tb, cudaMemcpyHostToDevice, B->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
+        if (e == cudaSuccess) {
+          B->bcode = bcode;
+          B->d_bgroup = group;
+          B->d_btiles = btiles;
+          B->nbtiles = (int)tiles.size();
+        } else {
+          void *part[] = {bcode, group, btiles};
           for (void *q : part)
             if (q) cudaFree(q);
-          B->bcode = nullptr;
-          B->d_bgroup = nullptr;
-          B->d_btiles = nullptr;
-          e = cudaSuccess;
-        } else if (e == cudaSuccess) {
-          k_batch_box_code<<<B->num_sms * 8, 256, 0, B->stream>>>(B->pat.code, B->npad, place, B->bcode);
-          e = cudaGetLastError();
-          if (e == cudaSuccess) e = cudaMemcpyAsync(B->d_bgroup, sysgrp.data(), gb, cudaMemcpyHostToDevice, B->stream);
-          if (e == cudaSuccess) e = cudaMemcpyAsync(B->d_btiles, tiles.data(), tb, cudaMemcpyHostToDevice, B->stream);
-          if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
+          if (e == cudaErrorMemoryAllocation) {  // no room: the patterns serve
+            cudaGetLastError();
+            e = cudaSuccess;
+          }
         }
       }
     }
