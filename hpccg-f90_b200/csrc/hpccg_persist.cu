@@ -135,6 +135,12 @@ __device__ __forceinline__ bool grid_sum(const PersistArgs &g, double v, unsigne
   return s_ok != 0;
 }
 
+struct StatusWord {
+  int *w;
+  __device__ void set(int v) const { atomicExch(w, v); }
+  __device__ void set_if_ok(int v) const { atomicCAS(w, HPCCG_OK, v); }
+};
+
 // THREADS: of a block, at most (its registers).  ONE: every thread has at most one
 // row, whose r, p, x and Ap stay in registers; only the neighbours' r and p are
 // loaded.
@@ -246,12 +252,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_cg_persist(const __grid_constant
       g.x[i] = pending && ok ? __dadd_rn(xi, __dmul_rn(alpha, ONE ? p1 : pn[i])) : xi;
     }
   }
-  if (!ok) status = HPCCG_ERR_TIMEOUT;
-  if (lead || !ok) {
+  persist_report(StatusWord{&g.st->status}, lead, ok, status);
+  if (lead) {
     g.st->rtrans = rtrans;
     g.st->normr = normr;
     g.st->niters = niters;
-    g.st->status = status;
   }
 }
 
