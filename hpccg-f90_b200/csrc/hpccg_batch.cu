@@ -1712,10 +1712,7 @@ static int batch_boxes(hpccg_batch *B) {
     if (d.x < 3 || d.y < 3) return HPCCG_OK;  // narrower: neighbours' offsets coincide
   void *scratch = nullptr;  // owners, then places; the flag behind them
   const size_t place_bytes = sizeof(int4) * count;
-  if (cudaMalloc(&scratch, place_bytes + sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    return HPCCG_OK;  // without room for the boxes the patterns serve
-  }
+  if (const cudaError_t e = cudaMalloc(&scratch, place_bytes + sizeof(int)); e != cudaSuccess) return optional_table(e);
   unsigned long long *owner = static_cast<unsigned long long *>(scratch);
   int4 *place = static_cast<int4 *>(scratch);
   int *d_bad = reinterpret_cast<int *>(place + count), bad = 1;
@@ -1786,17 +1783,12 @@ static int batch_boxes(hpccg_batch *B) {
           void *part[] = {bcode, group, btiles};
           for (void *q : part)
             if (q) cudaFree(q);
-          if (e == cudaErrorMemoryAllocation) {  // no room: the patterns serve
-            cudaGetLastError();
-            e = cudaSuccess;
-          }
         }
       }
     }
   }
   cudaFree(scratch);
-  HPCCG_CUDA(e);
-  return rc;
+  return rc ? rc : optional_table(e);  // without room for the boxes the patterns serve
 }
 
 // The solve of hpccg_batch_solve; b and x are copied in with `in` and the

@@ -147,6 +147,17 @@ int set_cuda_error(cudaError_t e, const char *what, const char *file, int line);
     if (e_ != cudaSuccess) return ::hpccg::set_cuda_error(e_, #call, __FILE__, __LINE__); \
   } while (0)
 
+// The outcome of setting up a table that a solve can do without: too little memory for
+// it is no error (the caller goes on without the table).
+inline int optional_table(cudaError_t e) {
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return HPCCG_OK;
+  }
+  HPCCG_CUDA(e);
+  return HPCCG_OK;
+}
+
 // ---- deterministic reductions --------------------------------------------
 // Warp butterfly then a fixed-order pass over the warp sums: the result only
 // depends on the block's inputs, not on scheduling.

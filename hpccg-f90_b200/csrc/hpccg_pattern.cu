@@ -121,7 +121,10 @@ int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n,
                at16 = part(sizeof(PatEntry32) * most), b64 = part(sizeof(double) * most),
                b32 = part(sizeof(float) * most), b16 = part(sizeof(float) * most), atf = part(sizeof(int)),
                atc = part(sizeof(uint16_t) * (size_t)npad);
-  HPCCG_CUDA(cudaMalloc(&out->memory, bytes));
+  if (cudaError_t e = cudaMalloc(&out->memory, bytes); e != cudaSuccess) {
+    out->memory = nullptr;
+    return optional_table(e);
+  }
   unsigned char *mem = static_cast<unsigned char *>(out->memory);
   PatTable *t = reinterpret_cast<PatTable *>(mem + at_t);
   out->t64 = reinterpret_cast<PatEntry64 *>(mem + at64);
@@ -170,8 +173,7 @@ int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n,
     if (e == cudaSuccess && !flags[1]) out->count = (int)rows.size();
   }
   if (e != cudaSuccess || !out->count) free_patterns(out);
-  HPCCG_CUDA(e);
-  return HPCCG_OK;
+  return optional_table(e);
 }
 
 // One thread per pattern: its entries (without the padding slots, offset 0 and value
@@ -227,13 +229,16 @@ int pattern_boxes_placed(RowPatterns *p, const int4 *place, cudaStream_t s) {
 
 static int fill_boxes(RowPatterns *p, int nx, int ny, const int4 *place, cudaStream_t s) {
   int bad = 1;
-  HPCCG_CUDA(cudaMemsetAsync(p->flag, 0, sizeof(int), s));
-  k_pat_boxes<<<(p->count + 31) / 32, 32, 0, s>>>(p->t64, p->count, nx, ny, place, p->box64, p->box32, p->box16, p->flag);
-  HPCCG_CUDA(cudaGetLastError());
-  HPCCG_CUDA(cudaMemcpyAsync(&bad, p->flag, sizeof(int), cudaMemcpyDeviceToHost, s));
-  HPCCG_CUDA(cudaStreamSynchronize(s));
-  p->boxes = !bad;
-  return HPCCG_OK;
+  cudaError_t e = cudaMemsetAsync(p->flag, 0, sizeof(int), s);
+  if (e == cudaSuccess) {
+    k_pat_boxes<<<(p->count + 31) / 32, 32, 0, s>>>(p->t64, p->count, nx, ny, place, p->box64, p->box32, p->box16,
+                                                    p->flag);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, p->flag, sizeof(int), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  p->boxes = e == cudaSuccess && !bad;
+  return optional_table(e);
 }
 
 }  // namespace hpccg

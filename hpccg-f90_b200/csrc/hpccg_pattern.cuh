@@ -28,13 +28,13 @@ __device__ __forceinline__ PatEntry32 pat_entry(const PatEntry32 *p) {
 }
 
 // Looks for at most max_count patterns in the rows [0, n) of a 27-slot ELL;
-// out->count = 0 when there are more.  Synchronises the stream.
+// out->count = 0 when there are more, or no memory for the tables.  Synchronises the stream.
 int row_patterns(const int32_t *ell_col, const double *ell_val, int npad, int n, int max_count, int num_sms,
                  cudaStream_t s, RowPatterns *out);
 void free_patterns(RowPatterns *p);
 // For a matrix on a known grid: the patterns as values at the 3x3x3 neighbours
 // (p->box64 and its roundings); p->boxes tells whether every one's entries lie
-// there in order.  Synchronises the stream.
+// there in order (no where memory is short).  Synchronises the stream.
 int pattern_boxes(RowPatterns *p, int nx, int ny, cudaStream_t s);
 // The same for patterns of several grids: place[c] = (nx, ny, box number) of pattern c, on
 // the device; nx = 0: no box.
