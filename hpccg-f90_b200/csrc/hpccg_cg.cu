@@ -364,17 +364,20 @@ static int cg_common(hpccg_ctx *c, int32_t max_iter, double tolerance, int32_t *
     HPCCG_CUDA(cudaEventRecord(c->solve0, c->stream));
     if ((rc = run_cg_eager(c))) return rc;
     HPCCG_CUDA(cudaEventRecord(c->solve1, c->stream));
-  } else if (cg_persist_fits(c)) {
-    HPCCG_CUDA(cudaEventRecord(c->solve0, c->stream));
-    if ((rc = cg_persist(c))) return rc;
-    HPCCG_CUDA(cudaEventRecord(c->solve1, c->stream));
   } else {
-    const SpmvArgs a = spmv_args(c);
-    if (!c->cg_exec || c->cg_graph_kind != a.kind || c->cg_graph_param != a.param ||
-        c->cg_graph_hist_cap != c->hist_cap)
-      if ((rc = build_cg_graph(c))) return rc;
-    HPCCG_CUDA(cudaEventRecord(c->solve0, c->stream));
-    HPCCG_CUDA(cudaGraphLaunch(c->cg_exec, c->stream));
+    bool launched = false;
+    if (cg_persist_fits(c)) {
+      HPCCG_CUDA(cudaEventRecord(c->solve0, c->stream));
+      if ((rc = cg_persist(c, &launched))) return rc;
+    }
+    if (!launched) {
+      const SpmvArgs a = spmv_args(c);
+      if (!c->cg_exec || c->cg_graph_kind != a.kind || c->cg_graph_param != a.param ||
+          c->cg_graph_hist_cap != c->hist_cap)
+        if ((rc = build_cg_graph(c))) return rc;
+      HPCCG_CUDA(cudaEventRecord(c->solve0, c->stream));
+      HPCCG_CUDA(cudaGraphLaunch(c->cg_exec, c->stream));
+    }
     HPCCG_CUDA(cudaEventRecord(c->solve1, c->stream));
   }
   CgState hs;

@@ -103,6 +103,7 @@ struct hpccg_ctx {
   // second p and the barrier slots of the one-kernel CG (allocated on its first solve)
   double *d_p2 = nullptr;
   void *d_slots = nullptr;
+  bool persist_off = false;  // its blocks cannot all be resident
   // scratch
   double *d_partials = nullptr;
   unsigned *d_counter = nullptr;

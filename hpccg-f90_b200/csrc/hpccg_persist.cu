@@ -261,15 +261,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_cg_persist(const __grid_constant
 }
 
 bool cg_persist_fits(const hpccg_ctx *c) {
-  if (c->spmv_kind != kSpmvPattern || !c->pat.count) return false;
+  if (c->persist_off || c->spmv_kind != kSpmvPattern || !c->pat.count) return false;
   return c->nrow <= (spmv_args(c).pat_box ? kPersistBoxRows : kPersistRows);
 }
 
-int cg_persist(hpccg_ctx *c) {
-  if (!c->d_p2) {
-    HPCCG_CUDA(cudaMalloc(&c->d_p2, sizeof(double) * (size_t)c->npad));
-    HPCCG_CUDA(cudaMalloc(&c->d_slots, sizeof(PersistSlot) * 2 * kPersistSlots));
-  }
+int cg_persist(hpccg_ctx *c, bool *launched) {
+  *launched = false;
+  cudaError_t e = cudaSuccess;
+  if (!c->d_slots && (e = cudaMalloc(&c->d_slots, sizeof(PersistSlot) * 2 * kPersistSlots)) != cudaSuccess)
+    c->d_slots = nullptr;
+  if (e == cudaSuccess && !c->d_p2 && (e = cudaMalloc(&c->d_p2, sizeof(double) * (size_t)c->npad)) != cudaSuccess)
+    c->d_p2 = nullptr;
+  if (e != cudaSuccess) return optional_table(e);
   // one row a thread while that fills no more than a block per SM (its rows in
   // registers), in blocks of 256 or 512 threads; else blocks of 1024
   const int sms = std::min(c->num_sms, kPersistBlocks);
@@ -295,8 +298,14 @@ int cg_persist(hpccg_ctx *c) {
   const void *kern = threads == 256   ? (const void *)k_cg_persist<256, true>
                      : threads == 512 ? (const void *)k_cg_persist<512, true>
                                       : (const void *)k_cg_persist<kPersistThreads, false>;
-  HPCCG_CUDA(cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(threads), args, 0, c->stream));
-  return HPCCG_OK;
+  e = cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(threads), args, 0, c->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {  // the process has fewer SMs than the device
+    cudaGetLastError();
+    c->persist_off = true;
+    return HPCCG_OK;
+  }
+  *launched = e == cudaSuccess;
+  return optional_table(e);
 }
 
 }  // namespace hpccg

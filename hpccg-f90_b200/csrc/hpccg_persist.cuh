@@ -22,7 +22,9 @@ __host__ __device__ inline void persist_report(Word &&word, bool lead, bool ok, 
 
 // Whether the context's CG runs in one kernel (its row kernel settled as row patterns).
 bool cg_persist_fits(const hpccg_ctx *c);
-// Launches it on the context's stream: b, x, state and history as the graph's kernels take them.
-int cg_persist(hpccg_ctx *c);
+// Launches it on the context's stream: b, x, state and history as the graph's kernels take
+// them.  *launched = false where its second p finds no memory or its blocks cannot all
+// be resident: nothing has run, and the graph takes the solve.
+int cg_persist(hpccg_ctx *c, bool *launched);
 
 }  // namespace hpccg

@@ -4,6 +4,8 @@ A fixture leaves a few MB of device memory free; each test asks for an optional 
 is larger than that on a system whose solve needs no further memory.  Every kernel of
 the path has run once before, so that none is loaded under pressure.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -22,23 +24,35 @@ def env():
 
 @pytest.fixture
 def leave(env):
-    """leave(n): fills the device but for at most n MB; freed after the test."""
+    """leave(n): fills the device but for at most n MB (driver allocations of 2 MB and more);
+    leave.free() and the end of the test give all of it back."""
     torch, _ = env
+    cu = ctypes.CDLL("libcuda.so.1")
+    cu.cuMemAlloc_v2.argtypes = [ctypes.POINTER(ctypes.c_uint64), ctypes.c_size_t]
+    cu.cuMemFree_v2.argtypes = [ctypes.c_uint64]
     held = []
 
     def fill(mb):
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
-        for _ in range(1000):
-            free = torch.cuda.mem_get_info()[0]
-            if free <= mb * MB:
-                return
-            held.append(torch.empty(max(2 * MB, (free - mb * MB) // (2 * MB) * 2 * MB), dtype=torch.uint8, device="cuda"))
-        raise AssertionError("could not fill the device")
+        size = torch.cuda.mem_get_info()[0]
+        while (over := torch.cuda.mem_get_info()[0] - mb * MB) > 0:
+            size = max(2 * MB, min(size, over) // (2 * MB) * 2 * MB)
+            ptr = ctypes.c_uint64()
+            if cu.cuMemAlloc_v2(ctypes.byref(ptr), size) == 0:
+                held.append(ptr.value)
+            else:
+                assert size > 2 * MB, "could not fill the device"
+                size //= 2
 
+    def free():
+        torch.cuda.synchronize()
+        while held:
+            assert cu.cuMemFree_v2(held.pop()) == 0
+
+    fill.free = free
     yield fill
-    held.clear()
-    torch.cuda.empty_cache()
+    free()
 
 
 def _cg(torch, M, b, n=6):
@@ -86,3 +100,28 @@ def test_batch_row_patterns_are_optional(env, leave):
         out.append((x.cpu().numpy(), iters))
         B.close()
     assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][0], out[1][0])
+
+
+def test_one_kernel_cg_buffers_are_optional(env, leave):
+    """The one-kernel CG's second p takes 8.3 MB here; without it the graph of the same rows
+    runs, whose dot products are associated differently (the bars of test_one_kernel_cg).
+    With memory again the one kernel runs: the same context, the result of a fresh one."""
+    torch, hp = env
+    rows, cols, vals = hp.generate_matrix(101, 101, 102)[:3]
+    big = hp.Matrix.from_csr(*hp.generate_matrix(110, 100, 100)[:3])  # the graph of the pattern rows
+    fresh, M = (hp.Matrix.from_csr(rows, cols, vals) for _ in range(2))
+    b = torch.rand(big.nrow, dtype=torch.float64, device="cuda")
+    _cg(torch, big, b)
+    want = _cg(torch, fresh, b[:M.nrow])
+    y, x = torch.empty_like(want[1]), torch.zeros_like(want[1])
+    M.spmv(want[1], y)  # finds the patterns
+    leave(6)
+    for _ in range(2):  # a second solve finds the buffers missing again
+        x.zero_()
+        it, normr, hist, st = M.cg_device(b[:M.nrow], x, 6, 0.0)
+        assert st == hp.HPCCG_OK and it == 6
+        assert (np.abs(hist - want[0]) <= 1e-12 * want[0]).all()
+        assert np.abs(x.cpu().numpy() - want[1].cpu().numpy()).max() <= 1e-10
+    leave.free()
+    again = _cg(torch, M, b[:M.nrow])
+    assert np.array_equal(again[0], want[0]) and torch.equal(again[1], want[1])
