@@ -1573,21 +1573,30 @@ static int ensure_tiles(hpccg_batch *B) {
     pc0.push_back((int)pc.size());
   }
   if ((int64_t)wt.size() > B->nchunks || (int64_t)pc.size() > B->nchunks) return HPCCG_OK;
-  HPCCG_CUDA(cudaMalloc(&B->d_wtiles, sizeof(int4) * wt.size()));
-  HPCCG_CUDA(cudaMalloc(&B->d_pieces, sizeof(int4) * pc.size()));
-  HPCCG_CUDA(cudaMalloc(&B->d_wtile0, sizeof(int) * wt0.size()));
-  HPCCG_CUDA(cudaMalloc(&B->d_piece0, sizeof(int) * pc0.size()));
-  HPCCG_CUDA(cudaMemcpyAsync(B->d_wtiles, wt.data(), sizeof(int4) * wt.size(), cudaMemcpyHostToDevice, B->stream));
-  HPCCG_CUDA(cudaMemcpyAsync(B->d_pieces, pc.data(), sizeof(int4) * pc.size(), cudaMemcpyHostToDevice, B->stream));
-  HPCCG_CUDA(cudaMemcpyAsync(B->d_wtile0, wt0.data(), sizeof(int) * wt0.size(), cudaMemcpyHostToDevice, B->stream));
-  HPCCG_CUDA(cudaMemcpyAsync(B->d_piece0, pc0.data(), sizeof(int) * pc0.size(), cudaMemcpyHostToDevice, B->stream));
-  HPCCG_CUDA(cudaStreamSynchronize(B->stream));
-  float *p = nullptr;
-  HPCCG_CUDA(cudaMalloc(&p, sizeof(float) * (size_t)B->npad));
+  // the batch takes them over once they are complete; without room the column walks serve
+  void *buf[5] = {};
+  const size_t bytes[5] = {sizeof(int4) * wt.size(), sizeof(int4) * pc.size(), sizeof(int) * wt0.size(),
+                           sizeof(int) * pc0.size(), sizeof(float) * (size_t)B->npad};
+  const void *src[4] = {wt.data(), pc.data(), wt0.data(), pc0.data()};
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < 5 && e == cudaSuccess; ++i) {
+    e = cudaMalloc(&buf[i], bytes[i]);
+    if (e == cudaSuccess && i < 4) e = cudaMemcpyAsync(buf[i], src[i], bytes[i], cudaMemcpyHostToDevice, B->stream);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(B->stream);
+  if (e != cudaSuccess) {
+    for (void *q : buf)
+      if (q) cudaFree(q);
+    return optional_table(e);
+  }
+  B->d_wtiles = static_cast<int4 *>(buf[0]);
+  B->d_pieces = static_cast<int4 *>(buf[1]);
+  B->d_wtile0 = static_cast<int *>(buf[2]);
+  B->d_piece0 = static_cast<int *>(buf[3]);
+  B->p32b = static_cast<float *>(buf[4]);
   B->nwtiles = (int)wt.size();
   B->npieces = (int)pc.size();
   B->wz = wz;
-  B->p32b = p;  // last: the tables are complete
   return HPCCG_OK;
 }
 

@@ -125,3 +125,30 @@ def test_one_kernel_cg_buffers_are_optional(env, leave):
     leave.free()
     again = _cg(torch, M, b[:M.nrow])
     assert np.array_equal(again[0], want[0]) and torch.equal(again[1], want[1])
+
+
+def test_batch_tiles_are_optional(env, leave):
+    """The tiled FP32 iteration's second p takes 105 MB; without it the column walks run, and
+    every system meets the target by a residual formed here in FP64."""
+    torch, hp = env
+    sizes = [(160, 128, 128)] * 10
+    warm = hp.Batch.generated([(1, 1, 300), (2, 1, 50)])  # shapes the tiles do not suit
+    B = hp.Batch.generated(sizes)
+    b = torch.arange(B.stacked_rows, dtype=torch.float64, device="cuda") % 7 - 3
+    x, r = torch.zeros_like(b), torch.zeros_like(b)
+    for W in (warm, B):
+        W.set_spmv(hp.SPMV_STENCIL)
+    warm.solve(b[:warm.stacked_rows], x[:warm.stacked_rows].zero_(), hp.PREC_FP32, 1e-6, 100)
+    x.zero_()
+    leave(40)
+    iters, relres, _, st = B.solve(b, x, hp.PREC_FP32, 1e-6, 200)
+    leave.free()
+    assert st == hp.HPCCG_OK
+    B.spmv(x, r)
+    for s, o in enumerate(B.offsets):
+        v = slice(int(o), int(o + B.nrows[s]))
+        rel = float(torch.linalg.vector_norm(b[v] - r[v]) / torch.linalg.vector_norm(b[v]))
+        assert rel <= 1e-6 * (1 + 1e-6) and relres[s] == pytest.approx(rel, rel=1e-6)
+    want = x.clone()
+    B.solve(b, x.zero_(), hp.PREC_FP32, 1e-6, 200)  # the same form again
+    assert torch.equal(x, want)
