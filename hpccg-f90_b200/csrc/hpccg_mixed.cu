@@ -625,6 +625,20 @@ inline int dispatch_lp(const SpmvArgs &a, int precision, int rpt, F &&f) {
 
 using namespace hpccg;
 
+// What a captured graph's row kernels depend on: their kind, whether they walk the
+// patterns' boxes, and the grid.
+struct RowForm {
+  int kind = 0, gx = 0, gy = 0, gz = 0;
+  bool box = false;
+  bool operator==(const RowForm &o) const {
+    return kind == o.kind && gx == o.gx && gy == o.gy && gz == o.gz && box == o.box;
+  }
+};
+static RowForm row_form(const hpccg_ctx *c) {
+  const SpmvArgs a = spmv_args(c);
+  return RowForm{a.kind, c->gx, c->gy, c->gz, a.pat_box != nullptr};
+}
+
 // Per-context mixed-precision resources, kept beside the context.
 struct MixedRes {
   float *r = nullptr, *p = nullptr, *Ap = nullptr, *d = nullptr, *x32 = nullptr, *y32 = nullptr;
@@ -634,7 +648,7 @@ struct MixedRes {
   MixedState *st = nullptr;
   cudaGraphExec_t exec[3] = {nullptr, nullptr, nullptr};
   int exec_rpt[3] = {0, 0, 0};
-  int exec_kind[3] = {0, 0, 0};
+  RowForm exec_rows[3];
   int rpt[3] = {0, 2, 4};  // rows per thread per precision (index 1 = FP32, 2 = BF16)
   // matrix-free SpMV on p by TMA (when the context uses the stencil and nx % 4 == 0)
   CUtensorMap pmap;
@@ -983,7 +997,7 @@ static int build_mixed_graph(hpccg_ctx *c, MixedRes *m, int precision) {
     return set_cuda_error(e, "build mixed graph", __FILE__, __LINE__);
   }
   m->exec_rpt[precision] = m->rpt[precision];
-  m->exec_kind[precision] = spmv_args(c).kind;
+  m->exec_rows[precision] = row_form(c);
   m->exec_fused[precision] = use_iter(c, m);
   return HPCCG_OK;
 }
@@ -1053,7 +1067,7 @@ static int solve_mixed_common(hpccg_ctx *c, int precision, double rel_tol, int32
     if ((rc = run_mixed_eager(c, m, precision))) return rc;
   } else {
     if (!m->exec[precision] || m->exec_rpt[precision] != m->rpt[precision] ||
-        m->exec_kind[precision] != spmv_args(c).kind || m->exec_fused[precision] != use_iter(c, m))
+        !(m->exec_rows[precision] == row_form(c)) || m->exec_fused[precision] != use_iter(c, m))
       if ((rc = build_mixed_graph(c, m, precision))) return rc;
     HPCCG_CUDA(cudaGraphLaunch(m->exec[precision], c->stream));
   }

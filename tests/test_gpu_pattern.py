@@ -136,3 +136,32 @@ def test_one_kernel_cg(env, nx, ny, nz):
         band = np.where(h1 >= 1e-8 * h1[0], h1, h1[0]) * 1e-12
         assert (np.abs(h0 - h1) <= band).all() and abs(n0 - n1) <= band[-1]
         assert np.abs(x0 - x1).max() <= 1e-10
+
+
+def test_mixed_graph_follows_the_grid(env):
+    """A CSR solved in mixed precision before and after its grid is declared: the second solve
+    runs the box walk (the first one's graph holds the gathers), with the same bits."""
+    torch, hp = env
+    from torch.profiler import ProfilerActivity, profile
+
+    nx, ny, nz = 96, 96, 96
+    M = hp.Matrix.from_csr(*hp.generate_matrix(nx, ny, nz)[:3])
+    b = torch.from_numpy(np.random.default_rng(4).uniform(-1, 1, M.nrow)).cuda()
+    for prec in (hp.PREC_FP32, hp.PREC_BF16):
+        runs = []
+        for grid in (False, True):
+            if grid:
+                M.set_geometry(nx, ny, nz)
+            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+                x = torch.zeros_like(b)
+                info, st = M.solve_mixed_device(b, x, prec, 1e-8)
+                torch.cuda.synchronize()
+            assert st == hp.HPCCG_OK
+            inner = {e.key for e in prof.key_averages() if "k_mp_spmv_dot" in e.key}
+            if not inner:
+                pytest.skip("the profiler reports no kernels here")
+            assert all(("StratLpBox" if grid else "StratLpPattern") in k for k in inner), inner
+            runs.append((info.outer_iters, x))
+        M.close()
+        M = hp.Matrix.from_csr(*hp.generate_matrix(nx, ny, nz)[:3])
+        assert float((runs[0][1] - runs[1][1]).abs().max()) <= 1e-6
