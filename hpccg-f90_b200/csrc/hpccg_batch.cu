@@ -1043,6 +1043,10 @@ static int build_tiles(hpccg_batch *B, int tile_chunks) {
       tiles.push_back(make_int4(s, B->off[s] + r0, B->off[s] + r1, B->chunk0[s] + r0 / kChunk));
     }
   }
+  for (cudaGraphExec_t &e : B->exec) {  // a captured solve holds the list's address
+    if (e) cudaGraphExecDestroy(e);
+    e = nullptr;
+  }
   if (B->d_tiles) cudaFree(B->d_tiles);
   B->d_tiles = nullptr;
   HPCCG_CUDA(cudaMalloc(&B->d_tiles, sizeof(int4) * tiles.size()));

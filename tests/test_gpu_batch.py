@@ -93,6 +93,33 @@ def test_batch_schedule_independent(hp, torch):
     assert np.array_equal(dx.cpu().numpy(), ref[FP64][0])
 
 
+def test_batch_graph_after_another_tile_list(hp, torch):
+    """A captured solve and then other tile lists (a schedule that is set and set back, the
+    matrix-free rows' own tuning) without a solve of that precision in between: the solve is
+    captured anew, with the same bits."""
+    sizes = SIZES + [(40, 36, 33)] * 9
+    B = hp.Batch.generated(sizes)
+    db = torch.from_numpy(B.stack([b for _, b, _ in _systems(sizes)])).cuda()
+
+    def solve(prec):
+        dx = torch.zeros_like(db)
+        assert B.solve(db, dx, prec, 1e-8, 1000)[3] == hp.HPCCG_OK
+        return dx.cpu().numpy()
+
+    B.set_schedule(4, 4)
+    want = [solve(p) for p in (FP64, FP32)]
+    B.set_schedule(1, 8)
+    pad = [torch.empty(1 << k, dtype=torch.uint8, device="cuda") for k in range(9, 24)]
+    B.set_schedule(4, 4)
+    assert np.array_equal(solve(FP64), want[0])
+    B.set_spmv(hp.SPMV_STENCIL)
+    solve(BF16)
+    B.set_spmv(hp.SPMV_ELL)
+    B.set_schedule(4, 4)
+    assert all(np.array_equal(solve(p), w) for p, w in zip((FP64, FP32), want))
+    del pad
+
+
 def test_batch_from_csr_equals_generated(hp, torch):
     sizes = SIZES[:4]
     sysl = _systems(sizes)
