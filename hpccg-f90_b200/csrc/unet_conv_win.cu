@@ -20,8 +20,12 @@
 // issues them (0.77), small grids by one tile's chain of set-up, first slab, ten
 // slabs and drain.  The zero blocks add exact zeros and a voxel's terms keep
 // their order (dy, dz, dx, input group), so the outputs are bit for bit those of
-// the voxels-as-M form (but an infinite or NaN input reaches all eight rows of
-// the tiles that read it: 0 * inf).
+// the voxels-as-M form.  Only an infinite or NaN input breaks this: its zero blocks
+// make NaNs in rows that it does not touch.  So every output that is not finite is
+// formed again from its own taps (win_again), found by 0 * v as it is stored: one
+// instruction a pair of channels, the ReLU being part of the conversion to BF16 (the
+// forward pass at 256^3 2300 us before and 2296 with it, 64^3 batch 4 gradient 1051 and
+// 1055; the rows formed again in line instead of in a function: 2306 and 1055).
 //
 // Columns: a tile spans tc z-planes of one x block (at most 126 voxels); its
 // input rows ("slabs": one y, tc+2 z-planes, x block with a one-voxel halo, both
@@ -114,6 +118,96 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t a) {
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const uint32_t *>(&p);
+}
+
+// The pair, negative numbers as zeros, NaNs as NaNs.
+__device__ __forceinline__ uint32_t pack2_relu(float lo, float hi) {
+  uint32_t d;
+  asm("cvt.rn.relu.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(hi), "f"(lo));
+  return d;
+}
+__device__ __forceinline__ float max_nan(float a, float b) {  // NaN where either is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+// Whether a BF16 pair holds an infinity or a NaN; chk collects 0 * v of several.
+__device__ __forceinline__ uint32_t zero_times(uint32_t v, uint32_t chk) {
+  const __nv_bfloat162 r = __hfma2(*reinterpret_cast<const __nv_bfloat162 *>(&v), __float2bfloat162_rn(0.f),
+                                   *reinterpret_cast<const __nv_bfloat162 *>(&chk));
+  return *reinterpret_cast<const uint32_t *>(&r);
+}
+__device__ __forceinline__ bool not_finite(uint32_t v) { return zero_times(v, 0u) & 0x7fff7fffu; }
+__device__ __forceinline__ bool not_finite(float v) { return !(0.f * v == 0.f); }
+
+// The sum of one voxel and output channel from its own 27 taps, outside ones as zeros.
+template <int NIN>
+__device__ float win_direct(const ConvArgs &a, int b, int z, int y, int x, int co) {
+  const ConvGeom &g = a.g;
+  float s = 0.f;
+  for (int tap = 0; tap < 27; ++tap) {
+    const int zz = z + tap / 9 - 1, yy = y + tap / 3 % 3 - 1, xx = x + tap % 3 - 1;
+    const bool in = (unsigned)zz < (unsigned)g.nz && (unsigned)yy < (unsigned)g.ny && (unsigned)xx < (unsigned)g.nx;
+    const int64_t row = ((int64_t)b * g.nz + zz) * g.ny + yy;
+    for (int k = 0; k < 2 * NIN; ++k) {  // input group, half
+      const uint4 *src = reinterpret_cast<const uint4 *>(NIN > 1 && k >= 2 ? a.in1 : a.in0);
+      const uint4 q = in ? __ldg(src + act_unit(row, k & 1, xx, g.nx)) : make_uint4(0, 0, 0, 0);
+      const uint4 w = __ldg(reinterpret_cast<const uint4 *>(a.wpack) + (((k >> 1) * 27 + tap) * 2 + (k & 1)) * 16 + co);
+      const uint32_t qv[4] = {q.x, q.y, q.z, q.w}, wv[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s = fmaf(__uint_as_float(qv[j] << 16), __uint_as_float(wv[j] << 16), s);
+        s = fmaf(__uint_as_float(qv[j] & 0xffff0000u), __uint_as_float(wv[j] & 0xffff0000u), s);
+      }
+    }
+    if (s != s) break;
+  }
+  return s;
+}
+
+// Forms again the outputs that this lane has just stored and that are not finite:
+// rows r and r + 1, the columns from c0 on of MMA `sub` of unit u, mapped as in the epilogue.
+template <int NIN, int EPI>
+__device__ __noinline__ void win_again(const WinArgs &w, int u, int r, int sub, int c0, int lane) {
+  const ConvArgs &a = w.a;
+  const WinPlan &p = w.p;
+  const ConvGeom &g = a.g;
+  const WinUnit w0 = win_unit(p, u);
+  const int pitch = p.txb + 2, tr = lane >> 2, tc2 = (lane & 3) * 2;
+  constexpr int kCols = EPI == kEpiProject ? 1 : (EPI == kEpiRawF32 ? 8 : 4);
+  for (int i = 0; i < kCols; ++i) {
+    const int c = c0 + (EPI == kEpiProject ? lane & 15 : (EPI == kEpiRawF32 ? 8 * (i >> 1) + tc2 + (i & 1) : 8 * i + tr));
+    const int zi = p.r1 > 1 ? c * p.inv >> 16 : 0, x = w0.x0 + c - zi * pitch, cc = w0.c0 + sub * p.r1 + zi;
+    if (c >= p.nn || zi >= p.r1 || c - zi * pitch >= p.txb || x >= g.nx || cc >= min(p.nc, w0.c0 + p.tc)) continue;
+    for (int k = 0; k < (EPI == kEpiProject ? 1 : 4); ++k) {
+      const int rr = r + (EPI == kEpiProject ? lane >> 4 : k >> 1), h = k & 1;
+      if (rr >= w0.rb) continue;
+      const int64_t row = (int64_t)w0.b * g.nz * g.ny + (int64_t)rr * p.sr + (int64_t)cc * p.sc;
+      auto sum = [&](int co) { return win_direct<NIN>(a, w0.b, p.zrows ? rr : cc, p.zrows ? cc : rr, x, co); };
+      if constexpr (EPI == kEpiProject) {
+        float acc = a.proj[16];
+        for (int co = 0; co < 16; ++co) acc = fmaf(a.proj[co], fmaxf(sum(co) + a.bias[co], 0.f), acc);
+        static_cast<float *>(a.out)[row * g.nx + x] = acc;
+      } else if constexpr (EPI == kEpiRawF32) {
+        float *o = static_cast<float *>(a.out) + act_unit(row, h, x, g.nx) * 8 + tr;
+        if (not_finite(*o)) *o = sum(8 * h + tr);
+      } else {
+        const int64_t at = act_unit(row, h, x, g.nx) * 4 + (lane & 3);
+        uint32_t *o = static_cast<uint32_t *>(a.out) + at;
+        if (!not_finite(*o)) continue;
+        float f[2];
+        for (int j = 0; j < 2; ++j) {
+          const int co = 8 * h + tc2 + j;
+          f[j] = sum(co);
+          if (EPI != kEpiMask && a.bias) f[j] += a.bias[co];
+          if (EPI == kEpiBiasRelu) f[j] = fmaxf(f[j], 0.f);
+        }
+        uint32_t v = pack2(f[0], f[1]);
+        if constexpr (EPI == kEpiMask) v = relu_mask2(v, __ldg(reinterpret_cast<const uint32_t *>(a.act) + at));
+        *o = v;
+      }
+    }
+  }
 }
 
 constexpr int kWinEpiWarps = 8;  // two per TMEM lane quarter
@@ -276,7 +370,7 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
       b0 = a.bias[lane & 15];
 #pragma unroll
       for (int c = 0; c < 17; ++c) proj[c] = a.proj[c];
-      } else if (EPI != kEpiRawF32 && EPI != kEpiMask && a.bias) {
+    } else if (EPI != kEpiRawF32 && EPI != kEpiMask && a.bias) {
       b0 = a.bias[tr];
       b1 = a.bias[tr + 8];
     }
@@ -299,25 +393,28 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
             *ci = sub * p.r1 + zi;
             return zi < p.r1 && x < xe && *ci < ce ? x : -1;
           };
+          // (the loads of the accumulators and the transposes take the whole warp)
           if constexpr (EPI == kEpiProject) {
-            for (int c0 = 16 * part; c0 < p.nn; c0 += 32) {
+            for (int c0 = 16 * part; c0 < p.nn; c0 += 32, __syncwarp()) {
               float v[16];
               tmem_ld16(base + sub * p.nn + c0, v);
               __syncwarp();  // the previous columns' sums have been read
 #pragma unroll
               for (int k = 0; k < 16; ++k)
-                stage[((lane >> 4) * 16 + k) * 17 + (lane & 15)] = fmaxf(v[k] + b0, 0.f);
+                stage[((lane >> 4) * 16 + k) * 17 + (lane & 15)] = max_nan(v[k] + b0, 0.f);
               __syncwarp();
               float acc = proj[16];
 #pragma unroll
               for (int c = 0; c < 16; ++c) acc = fmaf(proj[c], stage[lane * 17 + c], acc);
               int ci;
               const int x = column(c0 + (lane & 15), &ci), gs = lane >> 4;
-              if (x >= 0 && rok[gs])
+              if (x >= 0 && rok[gs]) {
                 static_cast<float *>(a.out)[(row0 + gs * p.sr + (int64_t)ci * p.sc) * g.nx + w0.x0 + x] = acc;
+                if (not_finite(acc)) win_again<NIN, EPI>(w, u, r, sub, c0, lane);
+              }
             }
           } else {
-            for (int c0 = 32 * part; c0 < p.nn; c0 += 64) {
+            for (int c0 = 32 * part; c0 < p.nn; c0 += 64, __syncwarp()) {
               uint32_t act[EPI == kEpiMask ? 4 : 1][2][2];  // all loads of the mask ahead of the sums
               if constexpr (EPI == kEpiMask) {
 #pragma unroll
@@ -333,7 +430,8 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
                       act[i][gs][h] = x >= 0 && rok[gs] ? __ldg(m + ((int64_t)gs * p.sr * 2 + h) * g.nx * 4) : 0;
                 }
               }
-              uint32_t d[2][16];
+              uint32_t d[2][16], chk = 0;  // 0 * what is stored
+              float zero = 0.f;
               tmem_ld_16x256_x4(base + sub * p.nn + c0, d[0]);
               tmem_ld_16x256_x4(base + (16u << 16) + sub * p.nn + c0, d[1]);
               tmem_wait_ld();
@@ -353,8 +451,11 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
                     for (int gs = 0; gs < 2; ++gs)
                       if (rok[gs])
 #pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                          o[((int64_t)gs * p.sr * 2 + h) * g.nx * 8] = __uint_as_float(d[gs][4 * i + 2 * h + e]);
+                        for (int h = 0; h < 2; ++h) {
+                          const float v = __uint_as_float(d[gs][4 * i + 2 * h + e]);
+                          o[((int64_t)gs * p.sr * 2 + h) * g.nx * 8] = v;
+                          zero = fmaf(0.f, v, zero);
+                        }
                   }
                 } else {
                   int ci;
@@ -372,16 +473,17 @@ __global__ void __launch_bounds__(kWinThreads, 1) k_conv3_win(const __grid_const
                         lo += bias;
                         hi += bias;
                       }
-                      if (EPI == kEpiBiasRelu) {
-                        lo = fmaxf(lo, 0.f);
-                        hi = fmaxf(hi, 0.f);
-                      }
-                      uint32_t v = transpose8x8(pack2(lo, hi));  // channels tc2, tc2+1 of half h, voxel tr
+                      // channels tc2, tc2+1 of half h, voxel tr
+                      uint32_t v = transpose8x8(EPI == kEpiBiasRelu ? pack2_relu(lo, hi) : pack2(lo, hi));
                       if constexpr (EPI == kEpiMask) v = relu_mask2(v, act[i][gs][h]);
-                      if (x >= 0 && rok[gs]) o[((int64_t)gs * p.sr * 2 + h) * g.nx * 4] = v;
+                      if (x >= 0 && rok[gs]) {
+                        o[((int64_t)gs * p.sr * 2 + h) * g.nx * 4] = v;
+                        chk = zero_times(v, chk);
+                      }
                     }
                 }
               }
+              if (EPI == kEpiRawF32 ? !(zero == 0.f) : (chk & 0x7fff7fffu) != 0) win_again<NIN, EPI>(w, u, r, sub, c0, lane);
             }
           }
         }

@@ -162,6 +162,46 @@ def test_conv_layer_window_edges(env, nx, ny, nz, nb, nin, epi):
         assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("nx,ny,nz,nb", [(128, 19, 3, 1), (64, 18, 5, 1), (256, 9, 2, 2), (32, 12, 24, 2), (8, 16, 9, 2)])
+@pytest.mark.parametrize("nin", [1, 2])
+@pytest.mark.parametrize("epi", [0, 1, 2, 3])
+def test_conv_layer_non_finite_inputs(env, nx, ny, nz, nb, nin, epi):
+    """Infinite and NaN voxels reach the outputs whose taps read them and no others: the same
+    outputs are not finite as with the brick tiles, with the same values (NaNs that a ReLU
+    follows are 0 in both), and the finite ones keep the bars of test_conv_layer_tc_and_cc."""
+    torch, hp = env
+    rng = np.random.default_rng(nx + 3 * ny + nin)
+    xs = [uo.bf16_round(rng.normal(0, 1, (nb, nz, ny, nx, 16))) for _ in range(nin)]
+    vox = [(0, 0, 0, 0), (nb - 1, nz - 1, ny - 1, nx - 1), (0, nz // 2, min(7, ny - 1), nx // 2), (0, nz - 1, min(8, ny - 1), 3)]
+    for k, v in enumerate(vox):
+        xs[k % nin][v + (5 * k % 16,)] = (np.inf, -np.inf, np.nan, np.inf)[k]
+    W = rng.normal(0, 0.1, (27, 16 * nin, 16)).astype(np.float32)
+    b = rng.normal(0, 0.1, 16).astype(np.float32)
+    proj = rng.normal(0, 0.3, 17).astype(np.float32)
+    dW, db, dp = (torch.from_numpy(v).cuda() for v in (W, b, proj))
+    din = [_bf16_tensor(torch, to_planar(v)) for v in xs] + [None]
+    n = nx * ny * nz * nb
+    dtype, size = {0: (torch.bfloat16, 16 * n), 1: (torch.bfloat16, 16 * n), 2: (torch.float32, n), 3: (torch.float32, 16 * n)}[epi]
+    outs = []
+    for path in (0, 2):
+        out = torch.full((size,), 7.0, dtype=dtype, device="cuda")
+        hp.conv3_layer(din[0], din[1], dW, db, dp, epi, path, out, nx, ny, nz, nb)
+        o = out.float().cpu().numpy()
+        outs.append(o.reshape(nb, nz, ny, nx) if epi == 2 else from_planar(o.reshape(nb, nz, ny, 2, nx, 8)))
+    with np.errstate(invalid="ignore"):
+        pre = uo.conv3(np.concatenate(xs, -1).astype(np.float64), uo.bf16_round(W).astype(np.float64))
+        act = np.nan_to_num(np.maximum(pre + b, 0), nan=0.0, posinf=np.inf)
+        want = {0: act, 1: pre + b, 2: act @ proj[:16].astype(np.float64) + proj[16], 3: pre}[epi]
+    got, brick = outs
+    bad = ~np.isfinite(want)
+    assert bad.any() and not bad.all()
+    assert np.array_equal(got[bad], want[bad], equal_nan=True) and np.array_equal(brick[bad], want[bad], equal_nan=True)
+    fin = ~bad
+    scale = np.abs(want[fin]).max()
+    bar = 1e-3 * scale + (np.abs(want[fin]) * 2.0 ** -8 if epi in (0, 1) else 0)
+    assert (np.abs(got[fin] - want[fin]) <= bar).all() and (np.abs(brick[fin] - want[fin]) <= bar).all()
+
+
 @pytest.mark.parametrize("nx,ny,nz,nb,nin,epi", [(1, 1, 1, 1, 1, 0), (3, 5, 2, 3, 2, 3), (24, 24, 24, 1, 1, 0), (24, 24, 24, 1, 2, 2),
                                                 (40, 37, 40, 1, 2, 0), (41, 69, 70, 1, 1, 3), (40, 67, 64, 1, 2, 2), (72, 1, 2200, 1, 1, 0)])
 def test_conv_layer_cuda_core_splits(env, nx, ny, nz, nb, nin, epi):
