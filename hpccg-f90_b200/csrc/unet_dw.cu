@@ -32,6 +32,10 @@ using namespace tc;
 // added up in registers with rounded FP32 additions (1.6e-7); two accumulator
 // sets let the drain run under the next steps' MMAs.
 //
+// Zeros stand for what lies outside the grid, so an infinity or NaN at a face makes NaNs
+// in the sums of taps that leave the grid there.  A sum that is a NaN at the end is formed
+// again from the terms inside the grid (dw_again); no other sees the difference.
+//
 // A unit is (batch, z, 8 rows of y, up to 112 voxels of x): its ten dY rows
 // (double-buffered) and the X slabs (a ring) arrive by TMA, one box per tensor.
 // Rows outside the grid, the x halo and the padding of dY to whole 16-voxel
@@ -52,7 +56,8 @@ constexpr int kDwChain = 8;  // MMA steps between two drains
 
 struct DwTcArgs {
   ConvGeom g;  // volume and batch only
-  CUtensorMap xmap[2], ymap;  // boxes: pitch units x 3 z x 2 halves; kx units x 2 halves x 10 y
+  const __nv_bfloat16 *x[2], *dy;
+  CUtensorMap xmap[2], ymap;  // of them; boxes: pitch units x 3 z x 2 halves; kx units x 2 halves x 10 y
   float *partial;
   int *err;
   int kx;                    // voxels per unit row, a multiple of 16
@@ -73,13 +78,46 @@ __host__ __device__ constexpr uint32_t idesc_bf16_mn(int M, int N) {
   return idesc_bf16(M, N) | (1u << 15) | (1u << 16);
 }
 
+__device__ __forceinline__ void dw_unit(const DwTcArgs &a, int u, int &b, int &z, int &ya, int &yb, int &x0) {
+  x0 = (u % a.nxb) * a.kx;
+  u /= a.nxb;
+  ya = (u % a.nyb) * kDwRows;
+  yb = min(a.g.ny, ya + kDwRows);
+  u /= a.nyb;
+  z = u % a.g.nz;
+  b = u / a.g.nz;
+}
+
+// The 16 sums at `out` that are NaN, again: this CTA's terms of one tap and input channel
+// ci (ci < 0: of the bias), one after the other.
+__device__ __noinline__ void dw_again(const DwTcArgs &a, int tap, int ci, float *out) {
+  const ConvGeom &g = a.g;
+  const int oz = ci < 0 ? 0 : tap / 9 - 1, oy = ci < 0 ? 0 : tap / 3 % 3 - 1, ox = ci < 0 ? 0 : tap % 3 - 1;
+  float s[16];
+  for (int c = 0; c < 16; ++c) s[c] = 0.f;
+  for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
+    int b, z, ya, yb, x0;
+    dw_unit(a, u, b, z, ya, yb, x0);
+    if ((unsigned)(z + oz) >= (unsigned)g.nz) continue;
+    for (int y = ya; y < yb; ++y) {  // the row of X
+      if ((unsigned)(y - oy) >= (unsigned)g.ny) continue;
+      const int64_t xrow = ((int64_t)b * g.nz + z + oz) * g.ny + y, drow = ((int64_t)b * g.nz + z) * g.ny + y - oy;
+      for (int x = max(x0, -ox); x < min(min(x0 + a.kx, g.nx), g.nx - ox); ++x) {
+        const float v = ci < 0 ? 1.f : __bfloat162float(a.x[ci >> 4][act_elem(xrow, x + ox, ci & 15, g.nx)]);
+        for (int c = 0; c < 16; ++c) s[c] = fmaf(v, __bfloat162float(a.dy[act_elem(drow, x, c, g.nx)]), s[c]);
+      }
+    }
+  }
+  for (int c = 0; c < 16; ++c)
+    if (out[c] != out[c]) out[c] = s[c];
+}
+
 template <int NIN>
 __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__ DwTcArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ uint64_t fullx[kDwSlots], emptyx[kDwSlots], fully[2], emptyy[2], acc_full[2], acc_empty[2], drain;
   __shared__ uint32_t slot;
   constexpr int P = dw_planes(NIN);
-  const ConvGeom &g = a.g;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int ps = dw_plane_bytes(a.kx), slab = P * ps, dyb = dw_dy_bytes(a.kx);
   uint8_t *sY = smem, *sX = smem + 2 * dyb;
@@ -113,15 +151,7 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__
   chain_wait();
   chain_release();  // the TMEM is allocated
   const int ksteps = a.kx / 16, chunk = max(1, kDwChain / ksteps);  // rows between two drains
-  auto unit = [&](int u, int &b, int &z, int &ya, int &yb, int &x0) {
-    x0 = (u % a.nxb) * a.kx;
-    u /= a.nxb;
-    ya = (u % a.nyb) * kDwRows;
-    yb = min(g.ny, ya + kDwRows);
-    u /= a.nyb;
-    z = u % g.nz;
-    b = u / g.nz;
-  };
+  auto unit = [&](int u, int &b, int &z, int &ya, int &yb, int &x0) { dw_unit(a, u, b, z, ya, yb, x0); };
   if (warp == 0) {
     if (lane == 0) {
       uint32_t sc = 0, uc = 0;
@@ -235,6 +265,10 @@ __global__ void __launch_bounds__(kDwThreads, 1) k_dW_tc(const __grid_constant__
           float4 *o = reinterpret_cast<float4 *>(out + (size_t)row * 16);
 #pragma unroll
           for (int k = 0; k < 4; ++k) o[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+          float nan = 0.f;
+#pragma unroll
+          for (int k = 0; k < 16; ++k) nan = fmaf(0.f, v[k], nan);
+          if (!(nan == 0.f)) dw_again(a, dz * 9 + (2 - ii) * 3 + dx, plane < 6 * NIN ? ci : -1, out + (size_t)row * 16);
         }
       }
   }
@@ -263,7 +297,30 @@ constexpr int kDwInRow = kDwInX * 8 + 8;                  // dY: 8 channels a vo
 constexpr int kDwInHalf = kDwInRows * kDwInRow + 4;       // halves 4
 constexpr int kDwInSmem = (2 * kDwInHalf + 3 * (kDwInRows + 2) * kDwInLine) * (int)sizeof(float);
 
-__global__ void __launch_bounds__(kDwInThreads, kDwInPerSm) k_dW_in1(DwArgs a, int xb) {
+// Channel co of tap `tap` (27: the bias) over this block's units, terms inside the grid only.
+__device__ __noinline__ float dw_in1_again(const DwArgs &a, int xb, int tap, int co) {
+  const int nx = a.nx, ny = a.ny, nz = a.nz;
+  const int nxb = (nx + xb - 1) / xb, nyb = (ny + kDwInRows - 1) / kDwInRows;
+  const int64_t nunit = (int64_t)nxb * nyb * nz * a.nb;
+  float s = 0.f;
+  for (int64_t u = blockIdx.x; u < nunit; u += gridDim.x) {
+    const int64_t p = u / nxb, plane = p / nyb;
+    const int x0 = (int)(u - p * nxb) * xb, y0 = (int)(p - plane * nyb) * kDwInRows, z = (int)(plane % nz);
+    for (int y = y0; y < min(ny, y0 + kDwInRows); ++y)
+      for (int x = x0; x < min(nx, x0 + xb); ++x) {
+        const float d = __bfloat162float(a.dy[act_elem(plane * ny + y, x, co, nx)]);
+        const int xx = x + tap % 3 - 1, yy = y + tap / 3 % 3 - 1, dz = tap / 9 - 1;
+        if (tap == 27)
+          s += d;
+        else if ((unsigned)xx < (unsigned)nx && (unsigned)yy < (unsigned)ny && (unsigned)(z + dz) < (unsigned)nz)
+          s = fmaf(a.x_f32[((plane + dz) * ny + yy) * nx + xx], d, s);
+      }
+  }
+  return s;
+}
+
+__global__ void __launch_bounds__(kDwInThreads, kDwInPerSm) k_dW_in1(const __grid_constant__ DwArgs a,
+                                                                   int xb) {
   __shared__ __align__(16) float sm[kDwInSmem / sizeof(float)];
   float *sdy = sm, *sin = sm + 2 * kDwInHalf;
   const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -381,7 +438,11 @@ __global__ void __launch_bounds__(kDwInThreads, kDwInPerSm) k_dW_in1(DwArgs a, i
     }
   }
   __syncthreads();
-  for (int e = t; e < 28 * 16; e += kDwInThreads) a.partial[(size_t)blockIdx.x * 28 * 16 + e] = red[e];
+  for (int e = t; e < 28 * 16; e += kDwInThreads) {
+    float v = red[e];
+    if (v != v) v = dw_in1_again(a, xb, e >> 4, e & 15);  // a NaN may be a zero outside the grid times an infinity
+    a.partial[(size_t)blockIdx.x * 28 * 16 + e] = v;
+  }
 }
 
 // Partials of one layer's gradient (a.partial holds max_blocks of them); *blocks: how many.
@@ -399,6 +460,9 @@ int launch_dW(const DwArgs &a, int max_blocks, int *err, int num_sms, cudaStream
   t.g.ny = a.ny;
   t.g.nz = a.nz;
   t.g.nb = a.nb;
+  t.x[0] = a.x0;
+  t.x[1] = a.x1;
+  t.dy = a.dy;
   t.partial = a.partial;
   t.err = err;
   t.nxb = (a.nx + kDwMaxX - 1) / kDwMaxX;

@@ -163,3 +163,24 @@ def test_every_layers_gradient_sums(env, nx, ny, nz, nb):
         err = np.abs(got - want)
         assert (err <= 50 * 2.0 ** -24 * mag).all(), (l, (err / mag).max())
         assert np.linalg.norm(err) <= 1e-6 * np.linalg.norm(mag), l
+
+
+@pytest.mark.parametrize("nx,ny,nz,nb", SHAPES[:4])
+@pytest.mark.parametrize("last", [False, True])
+@pytest.mark.parametrize("what", ["input", "target"])
+def test_gradients_with_a_non_finite_corner(env, nx, ny, nz, nb, last, what):
+    """An infinite input or target at a corner of a grid reaches the sums that have a term of
+    it: taps that leave the grid there keep their finite sums, the others are what the
+    64-bit sums are."""
+    at = (nb - 1, nz - 1, ny - 1, nx - 1) if last else (0, 0, 0, 0)
+
+    def poke(r, tgt):
+        (r if what == "input" else tgt)[at] = np.inf
+
+    seen = 0
+    for l, got, want, mag in _run(env, nx, ny, nz, nb, nx + nz, poke):
+        bad = ~np.isfinite(want)
+        seen += bad.sum()
+        assert np.array_equal(got[bad], want[bad], equal_nan=True), l
+        assert (np.abs(got[~bad] - want[~bad]) <= 50 * 2.0 ** -24 * mag[~bad]).all(), l
+    assert seen
