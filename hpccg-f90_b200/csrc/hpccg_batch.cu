@@ -4,10 +4,12 @@
 // global column indices); each system's rows start on a 512-row chunk
 // boundary.  A schedule cuts every system into tiles of whole chunks; one
 // persistent kernel per CG phase walks the tiles of all systems that are still
-// active.  Every dot product is reduced per 512-row chunk in a fixed order
-// (each lane's rows in order, then the fixed warp butterfly), and per system over its chunks in
-// index order, so the result does not depend on the schedule: the autotuner
-// may pick any tile size / grid and every iterate stays bit-identical.
+// active.  A phase reduces every dot product per 512-row chunk in a fixed order
+// (each lane's rows in order, then the fixed warp butterfly), and per system over
+// its chunks in a fixed order, so the result does not depend on the schedule: the
+// autotuner may pick any tile size / grid and every iterate stays bit-identical.
+// The tiled FP32 iteration of matrix-free batches (k_batch_tile32) reduces per
+// block of its own fixed lists instead, which no schedule changes.
 //
 // Solvers (all on the device, one CUDA graph with while nodes):
 //   FP64: CG per system (same steps as MPI/src/numerics.F90:108-147, stopping
@@ -513,8 +515,9 @@ __global__ void k_batch_box_code(const uint16_t *code, int n, const int4 *place,
     bcode[i] = (uint16_t)place[code[i]].w;
 }
 
-// The same for the FP32 inner solves, rows as 28 x - (plane box sums), the
-// form of stencil_row_box.
+// ---- the column walk of the FP32 inner solves ----------------------------------------
+// A p of matrix-free rows as 28 x - (plane box sums), the form of stencil_row_box; for
+// the shapes that the tiles (k_batch_tile32) do not suit.
 __device__ __forceinline__ float walk_box32(const float *__restrict__ x, int nx, unsigned mask) {
   float ln[3];
 #pragma unroll

@@ -463,7 +463,8 @@ static int time_current(hpccg_ctx *c, const double *x, double *y, int reps, floa
 }
 
 namespace hpccg {
-// AUTO: time the bit-exact ELL strategies on this matrix and keep the faster.
+// AUTO: row patterns where the matrix has few distinct rows; else time the bit-exact ELL
+// strategies on this matrix and keep the faster.
 int autotune_spmv(hpccg_ctx *c) {
   if (c->spmv_tuned) return HPCCG_OK;
   c->spmv_tuned = true;

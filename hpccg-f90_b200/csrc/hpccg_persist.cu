@@ -13,11 +13,14 @@
 // computing them from the same sums.  Dot products are associated per thread,
 // warp, block and over the blocks in index order: reproducible, but not the
 // graph's order.
-// An iteration, graph of the same pattern rows against this: 32^3 20.0 -> 8.4 us,
-// 64^3 26.5 -> 17.7, 97 x 75 x 61 28.6 -> 21.0, 100^3 40.7 -> 37.4, 128^3 65 -> 73,
-// hence kPersistRows; where the graph walks boxes 72^3 24.1 -> 22.2, 100 x 90 x 51 24.5
-// -> 24.1, 80^3 24.9 -> 26.2, 96^3 26.6 -> 34.8, hence kPersistBoxRows.  At 32^3 it is bound by the two steps' round trips (two hops
-// through L2 of about 1 us each and the sums on the way), above by the gathers.
+// An iteration in us, graph of the same pattern rows | this:
+//   gathers  32^3 20.0 | 8.4, 64^3 26.5 | 17.7, 97 x 75 x 61 28.6 | 21.0,
+//            100^3 40.7 | 37.4, 128^3 65 | 73, hence kPersistRows
+//   boxes    72^3 24.1 | 22.2, 100 x 90 x 51 24.5 | 24.1, 80^3 24.9 | 26.2,
+//            96^3 26.6 | 34.8, hence kPersistBoxRows
+// At 32^3 it is bound by the two steps' round trips (two hops through L2 of about
+// 1 us each and the sums on the way), above by the gathers.
+// Where its buffers find no memory or its blocks cannot all be resident, the graph runs.
 #include <algorithm>
 
 #include "hpccg_pattern.cuh"

@@ -6,19 +6,19 @@
 // half is one 16-byte unit, and a run of consecutive voxels of one row and
 // half is one contiguous span, which is exactly the layout the tensor cores
 // read (no-swizzle K-major core matrices: 8 rows x 16 bytes; the two halves
-// are the two K chunks).  So every operand tile arrives by 1D bulk copies
-// (cp.async.bulk) of whole row spans, with zero fill at the grid faces.
+// are the two K chunks).  So operand tiles are fetched as they lie: boxes of a
+// 5D tensor map (act_tmap) or whole row spans, with zero fill at the grid faces.
 //
 // A conv is an implicit GEMM on tcgen05 over the 27 taps and each 16-channel
 // input group, accumulated in FP32 in TMEM:
-//  * window tiles (unet_conv_win.cu): voxels are the MMA's N, eight output rows x
-//    16 channels its M;
+//  * window tiles (unet_conv_win.cu, with its roles and copies): the network's
+//    form; voxels are the MMA's N, eight output rows x 16 channels its M;
 //  * brick tiles (unet_conv.cu): 128 voxels of a bx*by*bz brick are M, the 16
 //    channels N, each tap's shifted brick fetched on its own.  Kept as the
 //    independent form that hpccg_unet_conv3_layer offers beside the other two.
-// Roles (192 threads): warp 0 fetches (its lanes issue the row spans in
-// parallel), warp 1 allocates TMEM and lane 0 issues the MMAs, warps 2-5 (one per
-// TMEM lane quarter) run the epilogue.
+//    192 threads: warp 0 fetches (its lanes issue 1D bulk copies of the row spans in
+//    parallel), warp 1 allocates TMEM and lane 0 issues the MMAs, warps 2-5 (one
+//    per TMEM lane quarter) run the epilogue.
 #pragma once
 #include "hpccg_internal.cuh"
 #include "unet_tc.cuh"

@@ -81,7 +81,8 @@ int hpccg_gpu_download_csr(const hpccg_ctx *ctx, int32_t *rowindex, int32_t *col
  * kernel on the stored matrix on first use (never the matrix-free stencil,
  * which is opt-in): the ELL as row patterns where the matrix has few distinct
  * rows (get_spmv then reports HPCCG_SPMV_ELL), else an ELL kernel; the others
- * force one kernel. */
+ * force one kernel.  Row patterns need 2 bytes a row of device memory more and are left
+ * out where it is short. */
 #define HPCCG_SPMV_AUTO 0
 #define HPCCG_SPMV_ELL 1        /* thread per row, column-major ELL (param: resident blocks/SM hint 2,3,4,8) */
 #define HPCCG_SPMV_ELL2 2       /* two rows per thread, 16-byte loads (same param)  */
@@ -95,7 +96,8 @@ int hpccg_gpu_set_spmv(hpccg_ctx *ctx, int32_t kind, int32_t param);
  * diagonal, -1.0 elsewhere).  On success the matrix-free SpMV
  * HPCCG_SPMV_STENCIL may be selected: it forms every row sum from x alone, in
  * the CSR's term order, so y, fused dots and CG histories are bit-identical
- * to the ELL kernels' while A is never read.  Returns HPCCG_ERR_UNSUPPORTED
+ * to those of HPCCG_SPMV_ELL while A is never read (AUTO's rows have the same
+ * bits, its CG of small systems other roundings of the dots: see hpccg_gpu_cg).  Returns HPCCG_ERR_UNSUPPORTED
  * when the matrix differs (the geometry is then cleared) and
  * HPCCG_ERR_INVALID_ARG when nx*ny*nz is not the row count.  Contexts from
  * hpccg_gpu_create_generated are checked and have the geometry already. */
@@ -111,7 +113,11 @@ int hpccg_gpu_get_spmv(const hpccg_ctx *ctx, int32_t *kind, int32_t *param);
  * `normr < tolerance` runs at the top of each iteration).  resid_hist
  * (nullable, length >= max_iter+1) receives [0] = Initial Residual and
  * [k] = the normr of iteration k, k = 1..niters.  The whole loop runs on the
- * device inside one CUDA graph with a device-side while condition. */
+ * device: inside one CUDA graph with a device-side while condition, or, under
+ * HPCCG_SPMV_AUTO and up to 2^20 rows of few distinct kinds, in one cooperative
+ * kernel.  The two associate the dot products differently, each always in
+ * the same way, so their histories agree to rounding; select HPCCG_SPMV_ELL for
+ * the graph's at every size. */
 int hpccg_gpu_cg(hpccg_ctx *ctx, const double *b, double *x, int32_t max_iter,
                  double tolerance, int32_t *niters, double *normr, double *resid_hist);
 

@@ -152,7 +152,7 @@ def test_mixed_graph_follows_the_grid(env):
         for grid in (False, True):
             if grid:
                 M.set_geometry(nx, ny, nz)
-            with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
                 x = torch.zeros_like(b)
                 info, st = M.solve_mixed_device(b, x, prec, 1e-8)
                 torch.cuda.synchronize()
