@@ -24,8 +24,9 @@
 // make NaNs in rows that it does not touch.  So every output that is not finite is
 // formed again from its own taps (win_again), found by 0 * v as it is stored: one
 // instruction a pair of channels, the ReLU being part of the conversion to BF16 (the
-// forward pass at 256^3 2300 us before and 2296 with it, 64^3 batch 4 gradient 1051 and
-// 1055; the rows formed again in line instead of in a function: 2306 and 1055).
+// forward pass at 256^3 2288 us before and 2277 with it, 64^3 batch 4 gradient 1061
+// and 1024; the rows formed again in line instead of in a function: 2306 and 1055).  A
+// forward pass at 128^3 with two infinite inputs takes 4.4 ms instead of 0.44.
 //
 // Columns: a tile spans tc z-planes of one x block (at most 126 voxels); its
 // input rows ("slabs": one y, tc+2 z-planes, x block with a one-voxel halo, both
@@ -140,29 +141,44 @@ __device__ __forceinline__ uint32_t zero_times(uint32_t v, uint32_t chk) {
 __device__ __forceinline__ bool not_finite(uint32_t v) { return zero_times(v, 0u) & 0x7fff7fffu; }
 __device__ __forceinline__ bool not_finite(float v) { return !(0.f * v == 0.f); }
 
-// The sum of one voxel and output channel from its own 27 taps, outside ones as zeros.
+// The sums of one voxel for the output channels co and co + 1 (co even) from its own 27
+// taps, outside ones as zeros; the loads of three taps at a time.
 template <int NIN>
-__device__ float win_direct(const ConvArgs &a, int b, int z, int y, int x, int co) {
+__device__ __forceinline__ float2 win_direct(const ConvArgs &a, int b, int z, int y, int x, int co) {
   const ConvGeom &g = a.g;
-  float s = 0.f;
-  for (int tap = 0; tap < 27; ++tap) {
-    const int zz = z + tap / 9 - 1, yy = y + tap / 3 % 3 - 1, xx = x + tap % 3 - 1;
-    const bool in = (unsigned)zz < (unsigned)g.nz && (unsigned)yy < (unsigned)g.ny && (unsigned)xx < (unsigned)g.nx;
+  float s0 = 0.f, s1 = 0.f;
+  for (int t = 0; t < 9; ++t) {
+    const int zz = z + t / 3 - 1, yy = y + t % 3 - 1;
+    const bool line = (unsigned)zz < (unsigned)g.nz && (unsigned)yy < (unsigned)g.ny;
     const int64_t row = ((int64_t)b * g.nz + zz) * g.ny + yy;
-    for (int k = 0; k < 2 * NIN; ++k) {  // input group, half
-      const uint4 *src = reinterpret_cast<const uint4 *>(NIN > 1 && k >= 2 ? a.in1 : a.in0);
-      const uint4 q = in ? __ldg(src + act_unit(row, k & 1, xx, g.nx)) : make_uint4(0, 0, 0, 0);
-      const uint4 w = __ldg(reinterpret_cast<const uint4 *>(a.wpack) + (((k >> 1) * 27 + tap) * 2 + (k & 1)) * 16 + co);
-      const uint32_t qv[4] = {q.x, q.y, q.z, q.w}, wv[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        s = fmaf(__uint_as_float(qv[j] << 16), __uint_as_float(wv[j] << 16), s);
-        s = fmaf(__uint_as_float(qv[j] & 0xffff0000u), __uint_as_float(wv[j] & 0xffff0000u), s);
+    for (int k = 0; k < 2 * NIN; ++k) {  // input group, half
+      const uint4 *src = reinterpret_cast<const uint4 *>(k >= 2 ? a.in1 : a.in0);
+      const uint4 *wp = reinterpret_cast<const uint4 *>(a.wpack) + (((k >> 1) * 27 + 3 * t) * 2 + (k & 1)) * 16 + co;
+      uint4 q[3], w[3][2];
+#pragma unroll
+      for (int dx = 0; dx < 3; ++dx) {
+        const int xx = x + dx - 1;
+        q[dx] = line && (unsigned)xx < (unsigned)g.nx ? __ldg(src + act_unit(row, k & 1, xx, g.nx)) : make_uint4(0, 0, 0, 0);
+        w[dx][0] = __ldg(wp + 32 * dx);
+        w[dx][1] = __ldg(wp + 32 * dx + 1);
+      }
+#pragma unroll
+      for (int dx = 0; dx < 3; ++dx) {
+        const uint32_t qv[4] = {q[dx].x, q[dx].y, q[dx].z, q[dx].w};
+        const uint32_t w0[4] = {w[dx][0].x, w[dx][0].y, w[dx][0].z, w[dx][0].w};
+        const uint32_t w1[4] = {w[dx][1].x, w[dx][1].y, w[dx][1].z, w[dx][1].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float lo = __uint_as_float(qv[j] << 16), hi = __uint_as_float(qv[j] & 0xffff0000u);
+          s0 = fmaf(hi, __uint_as_float(w0[j] & 0xffff0000u), fmaf(lo, __uint_as_float(w0[j] << 16), s0));
+          s1 = fmaf(hi, __uint_as_float(w1[j] & 0xffff0000u), fmaf(lo, __uint_as_float(w1[j] << 16), s1));
+        }
       }
     }
-    if (s != s) break;
+    if (s0 != s0 && s1 != s1) break;
   }
-  return s;
+  return make_float2(s0, s1);
 }
 
 // Forms again the outputs that this lane has just stored and that are not finite:
@@ -186,23 +202,29 @@ __device__ __noinline__ void win_again(const WinArgs &w, int u, int r, int sub, 
       auto sum = [&](int co) { return win_direct<NIN>(a, w0.b, p.zrows ? rr : cc, p.zrows ? cc : rr, x, co); };
       if constexpr (EPI == kEpiProject) {
         float acc = a.proj[16];
-        for (int co = 0; co < 16; ++co) acc = fmaf(a.proj[co], fmaxf(sum(co) + a.bias[co], 0.f), acc);
+        for (int co = 0; co < 16; co += 2) {
+          const float2 f = sum(co);
+          acc = fmaf(a.proj[co], fmaxf(f.x + a.bias[co], 0.f), acc);
+          acc = fmaf(a.proj[co + 1], fmaxf(f.y + a.bias[co + 1], 0.f), acc);
+        }
         static_cast<float *>(a.out)[row * g.nx + x] = acc;
       } else if constexpr (EPI == kEpiRawF32) {
         float *o = static_cast<float *>(a.out) + act_unit(row, h, x, g.nx) * 8 + tr;
-        if (not_finite(*o)) *o = sum(8 * h + tr);
+        if (!not_finite(*o)) continue;
+        const float2 f = sum(8 * h + (tr & ~1));
+        *o = tr & 1 ? f.y : f.x;
       } else {
         const int64_t at = act_unit(row, h, x, g.nx) * 4 + (lane & 3);
         uint32_t *o = static_cast<uint32_t *>(a.out) + at;
         if (!not_finite(*o)) continue;
-        float f[2];
-        for (int j = 0; j < 2; ++j) {
-          const int co = 8 * h + tc2 + j;
-          f[j] = sum(co);
-          if (EPI != kEpiMask && a.bias) f[j] += a.bias[co];
-          if (EPI == kEpiBiasRelu) f[j] = fmaxf(f[j], 0.f);
+        const int co = 8 * h + tc2;
+        float2 f = sum(co);
+        if (EPI != kEpiMask && a.bias) {
+          f.x += a.bias[co];
+          f.y += a.bias[co + 1];
         }
-        uint32_t v = pack2(f[0], f[1]);
+        if (EPI == kEpiBiasRelu) f = make_float2(fmaxf(f.x, 0.f), fmaxf(f.y, 0.f));
+        uint32_t v = pack2(f.x, f.y);
         if constexpr (EPI == kEpiMask) v = relu_mask2(v, __ldg(reinterpret_cast<const uint32_t *>(a.act) + at));
         *o = v;
       }

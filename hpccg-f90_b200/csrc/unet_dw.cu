@@ -34,7 +34,7 @@ using namespace tc;
 //
 // Zeros stand for what lies outside the grid, so an infinity or NaN at a face makes NaNs
 // in the sums of taps that leave the grid there.  A sum that is a NaN at the end is formed
-// again from the terms inside the grid (dw_again); no other sees the difference.
+// again from the terms inside the grid (dw_again), until it is a NaN for good.
 //
 // A unit is (batch, z, 8 rows of y, up to 112 voxels of x): its ten dY rows
 // (double-buffered) and the X slabs (a ring) arrive by TMA, one box per tensor.
@@ -94,6 +94,7 @@ __device__ __noinline__ void dw_again(const DwTcArgs &a, int tap, int ci, float 
   const ConvGeom &g = a.g;
   const int oz = ci < 0 ? 0 : tap / 9 - 1, oy = ci < 0 ? 0 : tap / 3 % 3 - 1, ox = ci < 0 ? 0 : tap % 3 - 1;
   float s[16];
+#pragma unroll
   for (int c = 0; c < 16; ++c) s[c] = 0.f;
   for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
     int b, z, ya, yb, x0;
@@ -102,12 +103,21 @@ __device__ __noinline__ void dw_again(const DwTcArgs &a, int tap, int ci, float 
     for (int y = ya; y < yb; ++y) {  // the row of X
       if ((unsigned)(y - oy) >= (unsigned)g.ny) continue;
       const int64_t xrow = ((int64_t)b * g.nz + z + oz) * g.ny + y, drow = ((int64_t)b * g.nz + z) * g.ny + y - oy;
+#pragma unroll 2
       for (int x = max(x0, -ox); x < min(min(x0 + a.kx, g.nx), g.nx - ox); ++x) {
         const float v = ci < 0 ? 1.f : __bfloat162float(a.x[ci >> 4][act_elem(xrow, x + ox, ci & 15, g.nx)]);
-        for (int c = 0; c < 16; ++c) s[c] = fmaf(v, __bfloat162float(a.dy[act_elem(drow, x, c, g.nx)]), s[c]);
+        float d[16];
+        load_voxel(a.dy, act_unit(drow, 0, x, g.nx), g.nx, d);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) s[c] = fmaf(v, d[c], s[c]);
       }
+      bool left = false;  // a sum that may still be a number
+#pragma unroll
+      for (int c = 0; c < 16; ++c) left |= out[c] != out[c] && s[c] == s[c];
+      if (!left) return;
     }
   }
+#pragma unroll
   for (int c = 0; c < 16; ++c)
     if (out[c] != out[c]) out[c] = s[c];
 }
@@ -314,6 +324,7 @@ __device__ __noinline__ float dw_in1_again(const DwArgs &a, int xb, int tap, int
           s += d;
         else if ((unsigned)xx < (unsigned)nx && (unsigned)yy < (unsigned)ny && (unsigned)(z + dz) < (unsigned)nz)
           s = fmaf(a.x_f32[((plane + dz) * ny + yy) * nx + xx], d, s);
+        if (s != s) return s;
       }
   }
   return s;

@@ -483,20 +483,6 @@ __global__ void __launch_bounds__(256) k_reduce_partials(const float *partial, i
   }
 }
 
-// The 16 channels of a voxel as floats.
-__device__ __forceinline__ void load_voxel(const __nv_bfloat16 *act, int64_t unit0, int nx, float *f) {
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(act) + unit0 + (int64_t)h * nx);
-    const __nv_bfloat162 *p2 = reinterpret_cast<const __nv_bfloat162 *>(&q);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const float2 t = __bfloat1622float2(p2[c]);
-      f[8 * h + 2 * c] = t.x;
-      f[8 * h + 2 * c + 1] = t.y;
-    }
-  }
-}
 // Voxel index -> unit of its first half.
 __device__ __forceinline__ int64_t voxel_unit(int64_t v, int nx) {
   const int64_t row = (uint64_t)v <= 0xFFFFFFFFull ? (int64_t)((uint32_t)v / (uint32_t)nx) : v / nx;

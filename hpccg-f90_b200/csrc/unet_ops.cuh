@@ -25,6 +25,20 @@ struct DwArgs {
   float *partial;                    // [gridDim.x][27*cin + 1][16]
 };
 
+// The 16 channels of a voxel as floats.
+__device__ __forceinline__ void load_voxel(const __nv_bfloat16 *act, int64_t unit0, int nx, float *f) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(act) + unit0 + (int64_t)h * nx);
+    const __nv_bfloat162 *p2 = reinterpret_cast<const __nv_bfloat162 *>(&q);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float2 t = __bfloat1622float2(p2[c]);
+      f[8 * h + 2 * c] = t.x;
+      f[8 * h + 2 * c + 1] = t.y;
+    }
+  }
+}
 // Two FP32 numbers in a register pair, and their fused multiply-add.
 __device__ __forceinline__ unsigned long long pack_f32x2(float lo, float hi) {
   unsigned long long r;
